@@ -66,21 +66,23 @@ MJ_DEV float box_entry(const RayInv& ri, float lx, float ly, float lz, float hx,
   return (tmax >= entry && entry < max_t) ? entry : -1.0f;
 }
 
-// MuJoCo's ray_quad: roots of a x^2 + 2 b x + c = 0 in x0 <= x1; returns the smaller
-// non-negative one or -1.
-MJ_HD float ray_quad(float a, float b, float c, float* x0, float* x1) {
+// MuJoCo's ray_quad: roots of a x^2 + 2 b x + c = 0 (a > 0) in x0 <= x1; returns the smaller
+// non-negative one or -1. The roots' signs are their numerators', so only the root asked for is
+// divided.
+MJ_HD bool quad_numerators(float a, float b, float c, float* n0, float* n1) {
   float det = b * b - a * c;
-  if (det < kMinVal) {
-    *x0 = -1.0f;
-    *x1 = -1.0f;
-    return -1.0f;
-  }
+  if (det < kMinVal) return false;
   det = sqrtf(det);
-  *x0 = (-b - det) / a;
-  *x1 = (-b + det) / a;
-  if (*x0 >= 0.0f) return *x0;
-  if (*x1 >= 0.0f) return *x1;
-  return -1.0f;
+  *n0 = -b - det;
+  *n1 = -b + det;
+  return true;
+}
+
+MJ_HD float ray_quad(float a, float b, float c) {
+  float n0, n1;
+  if (!quad_numerators(a, b, c, &n0, &n1)) return -1.0f;
+  const float n = n0 >= 0.0f ? n0 : n1;
+  return n >= 0.0f ? n / a : -1.0f;
 }
 
 // Geom frame of a world-block geom record.
@@ -117,8 +119,7 @@ MJ_HD float ray_sphere(const GeomFrame& g, const Ray& r, V3* n) {
   float a = dot(r.d, r.d);
   float b = dot(r.d, dif);
   float c = dot(dif, dif) - g.size.x * g.size.x;
-  float x0, x1;
-  float x = ray_quad(a, b, c, &x0, &x1);
+  float x = ray_quad(a, b, c);
   if (x < 0.0f) return -1.0f;
   *n = normalize(dif + r.d * x);
   return x;
@@ -133,8 +134,7 @@ MJ_HD float ray_ellipsoid(const GeomFrame& g, const Ray& r, V3* n) {
   float a = dot(sd, sd);
   float b = dot(sd, so);
   float c = dot(so, so) - 1.0f;
-  float x0, x1;
-  float x = ray_quad(a, b, c, &x0, &x1);
+  float x = ray_quad(a, b, c);
   if (x < 0.0f) return -1.0f;
   V3 p = lo + ld * x;
   V3 ln = normalize(cmul(p, cmul(s, s)));
@@ -152,25 +152,28 @@ MJ_HD float ray_capsule(const GeomFrame& g, const Ray& r, V3* n) {
   float a = ld.x * ld.x + ld.y * ld.y;
   float b = ld.x * lo.x + ld.y * lo.y;
   float c = lo.x * lo.x + lo.y * lo.y - rad * rad;
-  float x0, x1;
-  float sol = ray_quad(a, b, c, &x0, &x1);
+  float sol = ray_quad(a, b, c);
   if (sol >= 0.0f && fabsf(lo.z + sol * ld.z) <= h) {
     x = sol;
     part = 0;
   }
   float aa = dot(ld, ld);
   for (int cap = 0; cap < 2; ++cap) {
+    // a ray that starts short of a cap and does not run towards it never reaches its half space
+    if (cap == 0 ? (lo.z < h && ld.z <= 0.0f) : (lo.z > -h && ld.z >= 0.0f)) continue;
     float zc = cap == 0 ? h : -h;
     V3 dif = V3{lo.x, lo.y, lo.z - zc};
     float bb = dot(ld, dif);
     float cc = dot(dif, dif) - rad * rad;
-    ray_quad(aa, bb, cc, &x0, &x1);
-    float xs[2] = {x0, x1};
+    float xn[2];
+    if (!quad_numerators(aa, bb, cc, &xn[0], &xn[1])) continue;
     for (int i = 0; i < 2; ++i) {
-      float z = lo.z + xs[i] * ld.z;
+      if (!(xn[i] >= 0.0f)) continue;
+      float xs = xn[i] / aa;
+      float z = lo.z + xs * ld.z;
       bool side_ok = cap == 0 ? (z >= h) : (z <= -h);
-      if (xs[i] >= 0.0f && side_ok && (x < 0.0f || xs[i] < x)) {
-        x = xs[i];
+      if (side_ok && (x < 0.0f || xs < x)) {
+        x = xs;
         part = 1 + cap;
       }
     }
@@ -212,8 +215,7 @@ MJ_HD float ray_cylinder(const GeomFrame& g, const Ray& r, V3* n) {
   float a = ld.x * ld.x + ld.y * ld.y;
   float b = ld.x * lo.x + ld.y * lo.y;
   float c = lo.x * lo.x + lo.y * lo.y - rad * rad;
-  float x0, x1;
-  float sol = ray_quad(a, b, c, &x0, &x1);
+  float sol = ray_quad(a, b, c);
   if (sol >= 0.0f && fabsf(lo.z + sol * ld.z) <= h && (x < 0.0f || sol < x)) {
     x = sol;
     part = 0;
@@ -230,34 +232,92 @@ MJ_HD float ray_cylinder(const GeomFrame& g, const Ray& r, V3* n) {
   return x;
 }
 
-MJ_HD float ray_box(const GeomFrame& g, const Ray& r, V3* n) {
-  V3 lo, ld;
-  map_local(g, r, &lo, &ld);
+// Approximate reciprocal (a few ulp), for estimates that are checked or padded.
+MJ_HD float approx_rcp(float x) {
+#ifdef __CUDA_ARCH__
+  return __fdividef(1.0f, x);
+#else
+  return 1.0f / x;
+#endif
+}
+
+// MuJoCo's ray_box: the nearest of the face crossings that lie within their face.
+MJ_HD float ray_box_faces(V3 lo, V3 ld, V3 size, int* axis, float* dir) {
   float lp[3] = {lo.x, lo.y, lo.z};
   float lv[3] = {ld.x, ld.y, ld.z};
-  float sz[3] = {g.size.x, g.size.y, g.size.z};
+  float sz[3] = {size.x, size.y, size.z};
   float x = -1.0f;
-  int face_axis = -1;
-  float face_side = 0.0f;
+#pragma unroll
   for (int i = 0; i < 3; ++i) {
     if (fabsf(lv[i]) > kMinVal) {
+#pragma unroll
       for (int side = -1; side <= 1; side += 2) {
         float sol = ((float)side * sz[i] - lp[i]) / lv[i];
         if (sol >= 0.0f) {
-          int j = i == 0 ? 1 : 0;
-          int k = i == 2 ? 1 : 2;
+          const int j = i == 0 ? 1 : 0;
+          const int k = i == 2 ? 1 : 2;
           if (fabsf(lp[j] + sol * lv[j]) <= sz[j] && fabsf(lp[k] + sol * lv[k]) <= sz[k] && (x < 0.0f || sol < x)) {
             x = sol;
-            face_axis = i;
-            face_side = (float)side;
+            *axis = i;
+            *dir = (float)side;
           }
         }
       }
     }
   }
+  return x;
+}
+
+// One box axis of the ray in the box frame: estimated crossings of its two faces, and what their
+// estimate and a face test at them can be off by (positions to 2e-6 of the coordinates).
+MJ_HD void box_axis(float lp, float lv, float sz, float* tn, float* tf, float* e) {
+  const float r = approx_rcp(lv);
+  const float c = -lp * r, d = sz * fabsf(r);
+  *tn = c - d;
+  *tf = c + d;
+  *e = 4.0e-6f * (fabsf(lp) * fabsf(r) + d);
+}
+
+// The six face crossings of ray_box_faces cost a division and two face tests each, and nearly every
+// ray misses the box or enters it well inside one face: the estimated crossings of the three slabs
+// decide those by a margin, and only the entered face is computed, as ray_box_faces does. Rays
+// within the margin of an edge, from inside or along an axis take ray_box_faces.
+MJ_HD float ray_box_local(V3 lo, V3 ld, V3 size, int* axis, float* dir) {
+  if (fminf(fminf(fabsf(ld.x), fabsf(ld.y)), fabsf(ld.z)) > 1.0e-10f) {
+    float nx, ny, nz, fx, fy, fz, ex, ey, ez;
+    box_axis(lo.x, ld.x, size.x, &nx, &fx, &ex);
+    box_axis(lo.y, ld.y, size.y, &ny, &fy, &ey);
+    box_axis(lo.z, ld.z, size.z, &nz, &fz, &ez);
+    const float far_hi = fminf(fminf(fx + ex, fy + ey), fz + ez);
+    const float near_lo = fmaxf(fmaxf(nx - ex, ny - ey), nz - ez);
+    if (near_lo > far_hi || far_hi < 0.0f) return -1.0f;
+    const float far_lo = fminf(fminf(fx - ex, fy - ey), fz - ez);
+    // the axis entered last, by a margin over the others, before any is left
+    float t = -1.0f, p = 0.0f, v = 0.0f, s = 0.0f;
+    int i = -1;
+    if (nx - ex > fmaxf(ny + ey, nz + ez) && nx + ex < far_lo) t = nx - ex, p = lo.x, v = ld.x, s = size.x, i = 0;
+    if (ny - ey > fmaxf(nx + ex, nz + ez) && ny + ey < far_lo) t = ny - ey, p = lo.y, v = ld.y, s = size.y, i = 1;
+    if (nz - ez > fmaxf(nx + ex, ny + ey) && nz + ez < far_lo) t = nz - ez, p = lo.z, v = ld.z, s = size.z, i = 2;
+    if (t > 0.0f) {
+      *axis = i;
+      *dir = v > 0.0f ? -1.0f : 1.0f;
+      return (*dir * s - p) / v;
+    }
+  }
+  return ray_box_faces(lo, ld, size, axis, dir);
+}
+
+MJ_HD float ray_box(const GeomFrame& g, const Ray& r, V3* n) {
+  V3 lo, ld;
+  map_local(g, r, &lo, &ld);
+  int face_axis = -1;
+  float face_side = 0.0f;
+  const float x = ray_box_local(lo, ld, g.size, &face_axis, &face_side);
   if (x < 0.0f) return -1.0f;
   // column face_axis of the frame, times the side
-  *n = V3{g.mat.m[face_axis] * face_side, g.mat.m[3 + face_axis] * face_side, g.mat.m[6 + face_axis] * face_side};
+  const V3 col = face_axis == 0 ? V3{g.mat.m[0], g.mat.m[3], g.mat.m[6]}
+                                : (face_axis == 1 ? V3{g.mat.m[1], g.mat.m[4], g.mat.m[7]} : V3{g.mat.m[2], g.mat.m[5], g.mat.m[8]});
+  *n = col * face_side;
   return x;
 }
 
