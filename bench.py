@@ -630,8 +630,11 @@ def frame_chunks(m, d, rc) -> int:
 def render_launches(rc, chunks: int, nlight: int) -> int:
   """Kernels one render call launches: the wavefront's stages per chunk of worlds (primary, and
   with RGB cameras surface + resolve, mirror + mirror surface with reflections, shadow with
-  shadowing lights), else the single megakernel / path kernel."""
+  shadowing lights), else the single fused kernel (scenes of up to 32 geoms without meshes) /
+  megakernel / path kernel."""
   if not (rc.tier == 0 and rc.schedule == 2 and not rc.has_transparency):
+    return 1
+  if rc.enabled_geom_ids.shape[0] <= 32 and not rc.mesh_nface and not rc.nhfield and nlight <= 16:
     return 1
   rgb = any(rc.base.render_rgb)
   per = 1 + (2 if rgb else 0) + (2 if rgb and rc.has_reflection else 0)

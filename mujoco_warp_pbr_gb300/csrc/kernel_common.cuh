@@ -61,14 +61,29 @@ MJ_DEV void camera_frame_ray(const Pixel& p, int32_t n, int32_t sx, int32_t sy, 
 // Bundle rays x0, x1 and weight t of sample i of n along an axis of nb bundle rays: the sample
 // sits at bundle coordinate (i + 0.5) nb / n - 0.5 = num / den, in integers so that t is exactly 0
 // on a bundle pixel centre.
-MJ_DEV void bundle_axis(int32_t i, int32_t n, int32_t nb, int32_t* x0, int32_t* x1, float* t) {
+// With 32-bit integers where the products fit (every usual size: the 64-bit division is a hundred
+// instructions, twice per ray), else out of line with 64.
+static __device__ __noinline__ int32_t bundle_floor64(int32_t i, int32_t n, int32_t nb, float* t) {
   const int64_t num = (int64_t)(2 * i + 1) * nb - n;
   const int64_t den = 2 * (int64_t)n;
   int32_t a = (int32_t)((num + den) / den) - 1;  // num + den > 0
   a = min(max(a, 0), max(nb - 2, 0));
+  *t = (float)(num - (int64_t)a * den) / (float)den;
+  return a;
+}
+
+MJ_DEV void bundle_axis(int32_t i, int32_t n, int32_t nb, int32_t* x0, int32_t* x1, float* t) {
+  int32_t a;
+  if (n < (1 << 15) && nb < (1 << 15)) {
+    const int32_t num = (2 * i + 1) * nb - n, den = 2 * n;
+    a = (int32_t)((uint32_t)(num + den) / (uint32_t)den) - 1;
+    a = min(max(a, 0), max(nb - 2, 0));
+    *t = (float)(num - a * den) / (float)den;
+  } else {
+    a = bundle_floor64(i, n, nb, t);
+  }
   *x0 = a;
   *x1 = min(a + 1, nb - 1);
-  *t = (float)(num - (int64_t)a * den) / (float)den;
 }
 
 MJ_DEV V3 ray_vec(const float* a, int64_t i) { return V3{a[i * 3], a[i * 3 + 1], a[i * 3 + 2]}; }

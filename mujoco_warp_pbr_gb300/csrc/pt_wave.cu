@@ -29,12 +29,14 @@
 // one shadow entry (32 B) per slot.
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 #include "abi_internal.h"
 #include <cooperative_groups.h>
 
 #include "pt_bounce.cuh"
 #include "refill.cuh"
+#include "scan.cuh"
 
 namespace mjpbr {
 namespace {
@@ -358,10 +360,59 @@ __global__ void __launch_bounds__(kThreads) ptw_geometry_kernel(const __grid_con
 #ifndef MJPBR_PTW_REFILL_STEPS
 #define MJPBR_PTW_REFILL_STEPS 32
 #endif
+// Idle lanes before a warp of the scanned stages with meshes fetches again.
+#ifndef MJPBR_SCAN_MIN_IDLE
+#define MJPBR_SCAN_MIN_IDLE 8
+#endif
 
-// Closest hit of every live path, lanes refilled from the queue (refill.cuh); the pending
-// next-event terms of the path's last bounce are added first.
-template <bool kMesh>
+// Closest hits of `items` rays: start(item, &max_dist) gives a ray (and sets the lane's world block
+// blk), finish(hit) stores its hit.
+template <bool kMesh, bool kScan, class Start, class Finish>
+MJ_DEV void closest_queue(const MjpbrScene& s, const Stack& st, const BlockLayout& L, bool cull, int64_t items,
+                          unsigned long long* fetched, const float*& blk, const Start& start, const Finish& finish, int32_t* err) {
+  float max_dist;
+  if constexpr (kScan && !kMesh) {
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < items; i += (int64_t)gridDim.x * kThreads) {
+      const Ray r = start(i, &max_dist);
+      finish(scan_trace<false>(NodeBoxes{blk, &L}, s, st, blk, L, r, max_dist, cull, err));
+    }
+  } else if constexpr (kScan) {
+    ClosestWalk q;
+    auto done = [&](ClosestWalk& qq) {
+      if (qq.tie) qq.h = trace_ray<true>(s, st, blk, L, qq.m.r, max_dist, cull, false, err);
+      finish(qq.h);
+    };
+    refill_loop<MJPBR_PTW_REFILL_STEPS, MJPBR_SCAN_MIN_IDLE>(
+        items, fetched, q,
+        [&](int64_t item, ClosestWalk& qq) {
+          qq.m.r = start(item, &max_dist);
+          qq.m.meshes = scan_closest<true>(qq.h, qq.tie, NodeBoxes{blk, &L}, blk, L, qq.m.r, max_dist, cull);
+          qq.m.slot = -1;
+          qq.m.sp = 0;
+          if (qq.m.meshes) return true;
+          done(qq);
+          return false;
+        },
+        [&](ClosestWalk& qq) { return walk_closest_step(qq, s, st, blk, L, cull, err); }, [&](ClosestWalk& qq, int32_t) { done(qq); }, err);
+  } else {
+    ClosestQuery q;
+    refill_loop<MJPBR_PTW_REFILL_STEPS>(
+        items, fetched, q,
+        [&](int64_t item, ClosestQuery& qq) {
+          const Ray r = start(item, &max_dist);
+          closest_begin(qq, st, r, max_dist, err);
+          return true;
+        },
+        [&](ClosestQuery& qq) { return closest_step<kMesh>(qq, s, st, blk, L, cull, err); },
+        [&](ClosestQuery& qq, int32_t) { finish(qq.h); }, err);
+  }
+}
+
+// Closest hit of every live path; the pending next-event terms of the path's last bounce are added
+// first. Scenes of up to kScanGeoms geoms are scanned (scan.cuh): without meshes the lanes stride over
+// the queue, with them the meshes are traced resumably, lanes refilled from the queue (refill.cuh);
+// larger scenes walk the scene BVH resumably.
+template <bool kMesh, bool kScan>
 __global__ void __launch_bounds__(kThreads, 3) ptw_extend_kernel(const __grid_constant__ MjpbrScene s,
                                                                  const __grid_constant__ PtWaveMap wm, int32_t cur, bool pending_nee) {
   extern __shared__ __align__(16) float smem[];
@@ -369,47 +420,43 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_extend_kernel(const __grid_co
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
   const bool cull = s.settings.cull_backfaces != 0;
   const int64_t items = min((int64_t)wm.counters[cur], wm.path_cap);
+  unsigned long long* fetched = reinterpret_cast<unsigned long long*>(wm.counters + 4);
   int32_t err = 0;
-  ClosestQuery q;
   const float* blk = nullptr;
   int32_t path = -1;
-  refill_loop<MJPBR_PTW_REFILL_STEPS>(
-      items, reinterpret_cast<unsigned long long*>(wm.counters + 4), q,
-      [&](int64_t item, ClosestQuery& qq) {
-        path = wm.queue[cur][item];
-        PathRec& r = wm.path[path];
-        if (pending_nee) apply_nee(wm, path, r);
-        const float4 o = r.o, d = r.d;
-        blk = world_block(s, wm.w0 + (path / wm.nsample) / wm.pixels);
-        closest_begin(qq, st, Ray{V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}}, o.w, &err);
-        return true;
-      },
-      [&](ClosestQuery& qq) { return closest_step<kMesh>(qq, s, st, blk, L, cull, &err); },
-      [&](ClosestQuery& qq, int32_t) {
-        const Hit& hit = qq.h;
-        wm.hit[path] = pack_hit(hit);
-        PathRec& r = wm.path[path];
-        const int4 meta = r.meta;
-        const int32_t sample = meta.z;
-        const int32_t passes = meta.y;
-        const bool camera_ray = (meta.w & 1) != 0;
-        if (camera_ray && passes == 0 && sample == 0) {
-          int32_t ww, smp;
-          Pixel p;
-          path_pixel(s, wm, path, &ww, &p, &smp);
-          const float dcam_z = r.beta.w;
-          write_geometry(s, ww, p, hit, dcam_z);
-          if (hit.geom != -1) r.rad.w = hit.dist * -dcam_z;
-        }
-      },
-      &err);
+  auto start = [&](int64_t item, float* max_dist) {
+    path = wm.queue[cur][item];
+    PathRec& r = wm.path[path];
+    if (pending_nee) apply_nee(wm, path, r);
+    const float4 o = r.o, d = r.d;
+    blk = world_block(s, wm.w0 + (path / wm.nsample) / wm.pixels);
+    *max_dist = o.w;
+    return Ray{V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}};
+  };
+  auto finish = [&](const Hit& hit) {
+    wm.hit[path] = pack_hit(hit);
+    PathRec& r = wm.path[path];
+    const int4 meta = r.meta;
+    const int32_t sample = meta.z;
+    const int32_t passes = meta.y;
+    const bool camera_ray = (meta.w & 1) != 0;
+    if (camera_ray && passes == 0 && sample == 0) {
+      int32_t ww, smp;
+      Pixel p;
+      path_pixel(s, wm, path, &ww, &p, &smp);
+      const float dcam_z = r.beta.w;
+      write_geometry(s, ww, p, hit, dcam_z);
+      if (hit.geom != -1) r.rad.w = hit.dist * -dcam_z;
+    }
+  };
+  closest_queue<kMesh, kScan>(s, st, L, cull, items, fetched, blk, start, finish, &err);
   if (err && s.error_word) atomicOr(s.error_word, err);
 }
 
 // The first bounce's extend, with the start folded in: each path's camera ray is generated where
 // it is traced (start_sample, pt_bounce.cuh) and the path record written once, after the hit; the
 // path queue of the shade stage is the identity.
-template <bool kMesh>
+template <bool kMesh, bool kScan>
 __global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
                                                                        const __grid_constant__ PtWaveMap wm) {
   extern __shared__ __align__(16) float smem[];
@@ -417,47 +464,43 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __g
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
   const bool cull = s.settings.cull_backfaces != 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) wm.counters[0] = wm.npath;  // the shade stage's queue
+  unsigned long long* fetched = reinterpret_cast<unsigned long long*>(wm.counters + 4);
   int32_t err = 0;
-  ClosestQuery q;
   const float* blk = nullptr;
   int32_t path = -1;
   // the path's start state (the same for the ray and for the record stored after the hit)
-  auto start = [&](int32_t i, PathState& ps, Pixel& p, int32_t& w, int32_t& sample) {
+  auto start_state = [&](int32_t i, PathState& ps, Pixel& p, int32_t& w, int32_t& sample) {
     path_pixel(s, wm, i, &w, &p, &sample);
     p.rec = world_block(s, w) + L.cam_off + p.cam * kCamFloats;
     const M3 R = cam_mat(p.rec);
     const V3 cpos{p.rec[0], p.rec[1], p.rec[2]};
     start_sample(ps, s, p, pixel_seed_of(s, seed, w, p), R, cpos, sample);
   };
-  refill_loop<MJPBR_PTW_REFILL_STEPS>(
-      wm.npath, reinterpret_cast<unsigned long long*>(wm.counters + 4), q,
-      [&](int64_t item, ClosestQuery& qq) {
-        path = (int32_t)item;
-        wm.queue[0][path] = path;
-        PathState ps;
-        Pixel p;
-        int32_t w, sample;
-        start(path, ps, p, w, sample);
-        blk = world_block(s, w);
-        closest_begin(qq, st, Ray{ps.o, ps.d}, ps.max_dist, &err);
-        return true;
-      },
-      [&](ClosestQuery& qq) { return closest_step<kMesh>(qq, s, st, blk, L, cull, &err); },
-      [&](ClosestQuery& qq, int32_t) {
-        const Hit& hit = qq.h;
-        wm.hit[path] = pack_hit(hit);
-        PathState ps;
-        Pixel p;
-        int32_t w, sample;
-        start(path, ps, p, w, sample);
-        float first_depth = 0.0f;
-        if (sample == 0) {
-          write_geometry(s, w, p, hit, ps.dcam_z);
-          if (hit.geom != -1) first_depth = hit.dist * -ps.dcam_z;
-        }
-        store_path(wm.path[path], ps, first_depth);
-      },
-      &err);
+  auto start = [&](int64_t item, float* max_dist) {
+    path = (int32_t)item;
+    wm.queue[0][path] = path;
+    PathState ps;
+    Pixel p;
+    int32_t w, sample;
+    start_state(path, ps, p, w, sample);
+    blk = world_block(s, w);
+    *max_dist = ps.max_dist;
+    return Ray{ps.o, ps.d};
+  };
+  auto finish = [&](const Hit& hit) {
+    wm.hit[path] = pack_hit(hit);
+    PathState ps;
+    Pixel p;
+    int32_t w, sample;
+    start_state(path, ps, p, w, sample);
+    float first_depth = 0.0f;
+    if (sample == 0) {
+      write_geometry(s, w, p, hit, ps.dcam_z);
+      if (hit.geom != -1) first_depth = hit.dist * -ps.dcam_z;
+    }
+    store_path(wm.path[path], ps, first_depth);
+  };
+  closest_queue<kMesh, kScan>(s, st, L, cull, wm.npath, fetched, blk, start, finish, &err);
   if (err && s.error_word) atomicOr(s.error_word, err);
 }
 
@@ -510,31 +553,62 @@ __global__ void __launch_bounds__(kThreads, MJPBR_PTW_SHADE_CTAS) ptw_shade_kern
 }
 
 // ---------------------------------------------------------------- shadow rays
-// Any hit of every recorded shadow ray, lanes refilled from the queue (refill.cuh).
-template <bool kMesh>
+// Any hit of every recorded shadow ray: scanned (scan.cuh; without meshes the lanes stride over the
+// queue) or, past kScanGeoms geoms, by the scene BVH, lanes refilled from the queue (refill.cuh).
+template <bool kMesh, bool kScan>
 __global__ void __launch_bounds__(kThreads, 3) ptw_shadow_kernel(const __grid_constant__ MjpbrScene s,
                                                                  const __grid_constant__ PtWaveMap wm) {
   extern __shared__ __align__(16) float smem[];
-  const Stack st = wave_stack(s, smem);
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
   const bool cull = s.settings.cull_backfaces != 0;
   const int64_t items = min((int64_t)wm.counters[2], wm.shadow_cap);
+  unsigned long long* fetched = reinterpret_cast<unsigned long long*>(wm.counters + 6);
   int32_t err = 0;
-  AnyQuery q;
   const float* blk = nullptr;
   int32_t target = -1;
-  refill_loop<MJPBR_PTW_REFILL_STEPS>(
-      items, reinterpret_cast<unsigned long long*>(wm.counters + 6), q,
-      [&](int64_t item, AnyQuery& qq) {
-        const ShadowEntry e = wm.shadow[item];
-        target = __float_as_int(e.d.w);
-        const int32_t path = target / wm.nslot;
-        blk = world_block(s, wm.w0 + (path / wm.nsample) / wm.pixels);
-        any_begin(qq, st, Ray{V3{e.o.x, e.o.y, e.o.z}, V3{e.d.x, e.d.y, e.d.z}}, e.o.w, &err);
-        return true;
-      },
-      [&](AnyQuery& qq) { return any_step<kMesh>(qq, s, st, blk, L, cull, &err); },
-      [&](AnyQuery&, int32_t res) { wm.vis[target] = res == kAnyClear ? 1 : 0; }, &err);
+  auto start = [&](int64_t item, float* max_dist) {
+    const ShadowEntry e = wm.shadow[item];
+    target = __float_as_int(e.d.w);
+    const int32_t path = target / wm.nslot;
+    blk = world_block(s, wm.w0 + (path / wm.nsample) / wm.pixels);
+    *max_dist = e.o.w;
+    return Ray{V3{e.o.x, e.o.y, e.o.z}, V3{e.d.x, e.d.y, e.d.z}};
+  };
+  float max_dist;
+  if constexpr (kScan && !kMesh) {
+    uint32_t meshes;
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < items; i += (int64_t)gridDim.x * kThreads) {
+      const Ray r = start(i, &max_dist);
+      wm.vis[target] = scan_any<false>(blk, L, r, max_dist, cull, &meshes) ? 0 : 1;
+    }
+  } else if constexpr (kScan) {
+    const Stack st = wave_stack(s, smem);
+    MeshWalk q;
+    refill_loop<MJPBR_PTW_REFILL_STEPS, MJPBR_SCAN_MIN_IDLE>(
+        items, fetched, q,
+        [&](int64_t item, MeshWalk& qq) {
+          qq.r = start(item, &qq.cut);
+          qq.sp = 0;
+          const bool hit = scan_any<true>(blk, L, qq.r, qq.cut, cull, &qq.meshes);
+          if (!hit && qq.meshes) return true;
+          wm.vis[target] = hit ? 0 : 1;
+          return false;
+        },
+        [&](MeshWalk& qq) { return walk_any_step(qq, s, st, blk, L, &err); },
+        [&](MeshWalk&, int32_t res) { wm.vis[target] = res == kAnyClear ? 1 : 0; }, &err);
+  } else {
+    const Stack st = wave_stack(s, smem);
+    AnyQuery q;
+    refill_loop<MJPBR_PTW_REFILL_STEPS>(
+        items, fetched, q,
+        [&](int64_t item, AnyQuery& qq) {
+          const Ray r = start(item, &max_dist);
+          any_begin(qq, st, r, max_dist, &err);
+          return true;
+        },
+        [&](AnyQuery& qq) { return any_step<kMesh>(qq, s, st, blk, L, cull, &err); },
+        [&](AnyQuery&, int32_t res) { wm.vis[target] = res == kAnyClear ? 1 : 0; }, &err);
+  }
   if (err && s.error_word) atomicOr(s.error_word, err);
 }
 
@@ -624,14 +698,14 @@ int set_smem(K kern, size_t smem, const char* what) {
   return ensure_smem(reinterpret_cast<const void*>(kern), smem, what);
 }
 
-template <bool kMesh, bool kTex>
+template <bool kMesh, bool kTex, bool kScan>
 int launch_pt_wave(const MjpbrScene& s, uint32_t seed, cudaStream_t stream, int32_t chunk, int64_t pixels) {
   const size_t stack = (size_t)kThreads * stack_entries(s.settings.stack_depth) * 8;
   auto k_geometry = ptw_geometry_kernel<kMesh>;
-  auto k_extend = ptw_extend_kernel<kMesh>;
-  auto k_first = ptw_first_extend_kernel<kMesh>;
+  auto k_extend = ptw_extend_kernel<kMesh, kScan>;
+  auto k_first = ptw_first_extend_kernel<kMesh, kScan>;
   auto k_shade = ptw_shade_kernel<kMesh, kTex>;
-  auto k_shadow = ptw_shadow_kernel<kMesh>;
+  auto k_shadow = ptw_shadow_kernel<kMesh, kScan>;
   auto k_resolve = ptw_resolve_kernel<kTex>;
   int rc = set_smem(k_geometry, stack, "path wavefront geometry");
   if (!rc) rc = set_smem(k_extend, stack, "path wavefront extend");
@@ -740,10 +814,15 @@ int render_pt_wave_launch(const MjpbrScene& s, uint32_t seed, cudaStream_t strea
   }
   const bool mesh = s.nmesh + s.nhfield > 0 && s.blas_root != nullptr;
   const bool tex = s.settings.textures || s.settings.has_env || s.settings.env_background;
-  if (mesh && tex) return launch_pt_wave<true, true>(s, seed, stream, chunk, pixels);
-  if (mesh) return launch_pt_wave<true, false>(s, seed, stream, chunk, pixels);
-  if (tex) return launch_pt_wave<false, true>(s, seed, stream, chunk, pixels);
-  return launch_pt_wave<false, false>(s, seed, stream, chunk, pixels);
+  auto launch = [&](auto m, auto t) {
+    constexpr bool kMesh = decltype(m)::value, kTex = decltype(t)::value;
+    return s.nbvh_geom <= kScanGeoms ? launch_pt_wave<kMesh, kTex, true>(s, seed, stream, chunk, pixels)
+                                     : launch_pt_wave<kMesh, kTex, false>(s, seed, stream, chunk, pixels);
+  };
+  if (mesh && tex) return launch(std::true_type{}, std::true_type{});
+  if (mesh) return launch(std::true_type{}, std::false_type{});
+  if (tex) return launch(std::false_type{}, std::true_type{});
+  return launch(std::false_type{}, std::false_type{});
 }
 
 }  // namespace mjpbr

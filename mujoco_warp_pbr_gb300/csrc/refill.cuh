@@ -27,8 +27,10 @@ MJ_DEV uint64_t global_ns() {
 // query's result (result kAnyAbort after kMaxRaySteps steps, with kErrWorkQueue in *err).
 // `counter` (64-bit, zero before the launch) hands the items out. Every trip takes new items or
 // advances a ray, so the loop ends; a launch still running after kRefillTimeLimitNs sets
-// kErrWorkQueue and returns instead of spinning.
-template <int32_t kSteps, class Query, class Fetch, class Step, class Finish>
+// kErrWorkQueue and returns instead of spinning. kMinIdle: idle lanes it takes for the warp to fetch
+// (with fewer, the busy lanes go on), and the warp fetches again while that many are idle: for fetches
+// that do much of a ray's work, and often all of it.
+template <int32_t kSteps, int32_t kMinIdle = 1, class Query, class Fetch, class Step, class Finish>
 MJ_DEV void refill_loop(int64_t items, unsigned long long* counter, Query& q, const Fetch& fetch, const Step& step, const Finish& finish,
                         int32_t* err) {
   const unsigned full = 0xffffffffu;
@@ -43,7 +45,7 @@ MJ_DEV void refill_loop(int64_t items, unsigned long long* counter, Query& q, co
     }
     const bool need = !busy && !exhausted;
     const unsigned m = __ballot_sync(full, need);
-    if (m) {
+    if (m && (kMinIdle <= 1 || __popc(m) >= kMinIdle || __ballot_sync(full, busy) == 0)) {
       const int leader = __ffs(m) - 1;
       unsigned long long base = 0;
       if (lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(m));
@@ -57,6 +59,7 @@ MJ_DEV void refill_loop(int64_t items, unsigned long long* counter, Query& q, co
           steps = 0;
         }
       }
+      if (kMinIdle > 1 && __popc(__ballot_sync(full, !busy && !exhausted)) >= kMinIdle) continue;
     }
     if (__ballot_sync(full, busy) == 0) {
       if (__all_sync(full, exhausted)) return;

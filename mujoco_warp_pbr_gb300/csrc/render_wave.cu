@@ -31,11 +31,13 @@
 // two shadow entries (64 B); the library renders as many worlds per chunk as the scratch holds.
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 #include <vector>
 
 #include "abi_internal.h"
 #include "refill.cuh"
 #include "rt_shade.cuh"
+#include "scan.cuh"
 
 namespace mjpbr {
 namespace {
@@ -254,15 +256,21 @@ MJ_DEV void emit_shadows(const MjpbrScene& s, const WaveMap& wm, const float* bl
 }
 
 // ---------------------------------------------------------------- 1. primary rays
-template <bool kMesh, bool kStaged>
+template <bool kMesh, bool kStaged, bool kScan>
 __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_TRACE_CTAS) wave_primary_kernel(const __grid_constant__ MjpbrScene s,
                                                                 const __grid_constant__ WaveMap wm) {
   extern __shared__ __align__(16) float smem[];
   const int32_t w = wm.w0 + blockIdx.y;
   const float* blk = world_block_of<kStaged>(s, w, smem, kThreads);
-  __syncthreads();
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
   const Stack st = wave_stack(s, smem + (kStaged ? s.world_block_floats : 0));
+  __shared__ __align__(16) float boxes[kScan ? kSlotBoxFloats : 4];
+  if (kScan && threadIdx.x == 0) boxes[kSlotBoxFloats - 4] = 0.0f;
+  __syncthreads();
+  if constexpr (kScan) {
+    stage_boxes(blk, L, boxes, kThreads);
+    __syncthreads();
+  }
   int32_t cam, tx, ty;
   tile_of(wm.geo, blockIdx.x, &cam, &tx, &ty);
   Pixel p;
@@ -289,7 +297,12 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_TRACE_CTAS) wave_primary_
     float max_dist, depth_z;
     primary_ray(s, p, n, smp % n, smp / n, &dcam, &ocam, &max_dist, &depth_z);
     const Ray ray{cpos + mul(R, ocam), mul(R, dcam)};
-    const Hit hit = trace_ray<kMesh>(s, st, blk, L, ray, max_dist, cull, false, &err);
+    Hit hit;
+    if constexpr (kScan) {
+      hit = scan_trace<kMesh>(staged_boxes(boxes), s, st, blk, L, ray, max_dist, cull, &err);
+    } else {
+      hit = trace_ray<kMesh>(s, st, blk, L, ray, max_dist, cull, false, &err);
+    }
     if (smp == 0) write_geometry(s, w, p, hit, depth_z);
     if (rgb) out[(int64_t)p.pixelid * nn + smp] = pack_hit(hit);
   }
@@ -375,6 +388,10 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_SHADE_CTAS) wave_surface_
 #ifndef MJPBR_WAVE_REFILL_STEPS
 #define MJPBR_WAVE_REFILL_STEPS 32
 #endif
+// Idle lanes before a warp of the scanned stages fetches again.
+#ifndef MJPBR_SCAN_MIN_IDLE
+#define MJPBR_SCAN_MIN_IDLE 8
+#endif
 
 // Closest hit of every queued mirror ray, lanes refilled from the queue (refill.cuh).
 template <bool kMesh>
@@ -400,6 +417,41 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_
       },
       [&](ClosestQuery& qq) { return closest_step<kMesh>(qq, s, st, blk, L, cull, &err); },
       [&](ClosestQuery& qq, int32_t) { wm.hit[1][sample] = pack_hit(qq.h); }, &err);
+  if (err && s.error_word) atomicOr(s.error_word, err);
+}
+
+// The mirror stage of scanned scenes (scan.cuh): the primitives when a ray is fetched, its meshes
+// resumably.
+__global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_scan_kernel(const __grid_constant__ MjpbrScene s,
+                                                                                            const __grid_constant__ WaveMap wm) {
+  extern __shared__ __align__(16) float smem[];
+  const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
+  const Stack st = wave_stack(s, smem);
+  const bool cull = s.settings.cull_backfaces != 0;
+  const int64_t items = min((int64_t)wm.counters[0], wm.mirror_cap);
+  int32_t err = 0;
+  ClosestWalk q;
+  const float* blk = nullptr;
+  int32_t sample = -1;
+  auto done = [&](ClosestWalk& qq) {
+    if (qq.tie) qq.h = trace_ray<true>(s, st, blk, L, qq.m.r, kMaxVal, cull, false, &err);
+    wm.hit[1][sample] = pack_hit(qq.h);
+  };
+  refill_loop<MJPBR_WAVE_REFILL_STEPS, MJPBR_SCAN_MIN_IDLE>(
+      items, reinterpret_cast<unsigned long long*>(wm.counters + 4), q,
+      [&](int64_t item, ClosestWalk& qq) {
+        const MirrorEntry e = wm.mirror[item];
+        sample = e.index.x;
+        blk = s.world_blocks + (int64_t)(wm.w0 + sample / wm.per_world) * s.world_block_floats;
+        qq.m.r = Ray{V3{e.o.x, e.o.y, e.o.z}, V3{e.d.x, e.d.y, e.d.z}};
+        qq.m.meshes = scan_closest<true>(qq.h, qq.tie, NodeBoxes{blk, &L}, blk, L, qq.m.r, kMaxVal, cull);
+        qq.m.slot = -1;
+        qq.m.sp = 0;
+        if (qq.m.meshes) return true;
+        done(qq);
+        return false;
+      },
+      [&](ClosestWalk& qq) { return walk_closest_step(qq, s, st, blk, L, cull, &err); }, [&](ClosestWalk& qq, int32_t) { done(qq); }, &err);
   if (err && s.error_word) atomicOr(s.error_word, err);
 }
 
@@ -444,6 +496,25 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_SHADE_CTAS) wave_mirror_s
 }
 
 // ---------------------------------------------------------------- 5. shadow rays (persistent)
+// Ray k of a shadow entry, its world block and its count's index; false when its light takes fewer.
+MJ_DEV bool entry_ray(const MjpbrScene& s, const WaveMap& wm, const BlockLayout& L, const ShadowEntry& e, int32_t k, int32_t ns, uint32_t seed,
+                      const float** blk, int32_t* target, Ray* r, float* max_dist) {
+  const int32_t tgt = __float_as_int(e.l.w);
+  const int32_t li = tgt % wm.nl;
+  const int32_t sample = tgt / (2 * wm.nl);
+  const int32_t seg = (tgt / wm.nl) & 1;
+  int32_t w, cam, pixelid, smp;
+  sample_pixel(s, wm, sample, &w, &cam, &pixelid, &smp);
+  *blk = s.world_blocks + (int64_t)w * s.world_block_floats;
+  *target = tgt;
+  const Light light = load_light(*blk + L.light_off + li * kLightFloats);
+  if (k >= shadow_ray_count(light, ns)) return false;
+  r->o = V3{e.o.x, e.o.y, e.o.z};
+  shadow_ray(light, ns, r->o, V3{e.l.x, e.l.y, e.l.z}, e.o.w, pixel_seed_of(s, seed, w, cam, pixelid), 2 * smp + seg, L.nlight, li, k, &r->d,
+             max_dist);
+  return true;
+}
+
 // Work items: (entry, ray k < shadow_samples), traced as any-hit queries with lanes refilled from
 // the queue (refill.cuh); each unoccluded ray adds one to its entry's count (an integer sum, so
 // the counts do not depend on the order).
@@ -464,27 +535,51 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_TRACE_CTAS) wave_shadow_k
       items, reinterpret_cast<unsigned long long*>(wm.counters + 2), q,
       [&](int64_t item, AnyQuery& qq) {
         const int32_t ei = (int32_t)(item / ns), k = (int32_t)(item - (int64_t)ei * ns);
-        const ShadowEntry e = wm.shadow[ei];
-        const int32_t tgt = __float_as_int(e.l.w);
-        const int32_t li = tgt % wm.nl;
-        const int32_t sample = tgt / (2 * wm.nl);
-        const int32_t seg = (tgt / wm.nl) & 1;
-        int32_t w, cam, pixelid, smp;
-        sample_pixel(s, wm, sample, &w, &cam, &pixelid, &smp);
-        blk = s.world_blocks + (int64_t)w * s.world_block_floats;
-        const Light light = load_light(blk + L.light_off + li * kLightFloats);
-        if (k >= shadow_ray_count(light, ns)) return false;
         Ray r;
         float max_dist;
-        r.o = V3{e.o.x, e.o.y, e.o.z};
-        shadow_ray(light, ns, r.o, V3{e.l.x, e.l.y, e.l.z}, e.o.w, pixel_seed_of(s, seed, w, cam, pixelid), 2 * smp + seg, L.nlight, li, k,
-                   &r.d, &max_dist);
+        if (!entry_ray(s, wm, L, wm.shadow[ei], k, ns, seed, &blk, &target, &r, &max_dist)) return false;
         any_begin(qq, st, r, max_dist, &err);
-        target = tgt;
         return true;
       },
       [&](AnyQuery& qq) { return any_step<kMesh>(qq, s, st, blk, L, cull, &err); },
       [&](AnyQuery&, int32_t res) {
+        if (res == kAnyClear) atomicAdd(&wm.vis[target], 1);
+      },
+      &err);
+  if (err && s.error_word) atomicOr(s.error_word, err);
+}
+
+// The shadow stage of scanned scenes (scan.cuh): the primitives when a ray is fetched, its meshes
+// resumably.
+__global__ void __launch_bounds__(kThreads, MJPBR_WAVE_TRACE_CTAS) wave_shadow_scan_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
+                                                                                           const __grid_constant__ WaveMap wm) {
+  extern __shared__ __align__(16) float smem[];
+  const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
+  const Stack st = wave_stack(s, smem);
+  const bool cull = s.settings.cull_backfaces != 0;
+  const int32_t ns = max(s.settings.shadow_samples, 1);
+  const int64_t items = min((int64_t)wm.counters[1], wm.shadow_cap) * ns;
+  int32_t err = 0;
+  MeshWalk q;
+  const float* blk = nullptr;
+  int32_t target = -1;
+  refill_loop<MJPBR_WAVE_REFILL_STEPS, MJPBR_SCAN_MIN_IDLE>(
+      items, reinterpret_cast<unsigned long long*>(wm.counters + 2), q,
+      [&](int64_t item, MeshWalk& qq) {
+        const int32_t ei = (int32_t)(item / ns), k = (int32_t)(item - (int64_t)ei * ns);
+        Ray r;
+        float max_dist;
+        if (!entry_ray(s, wm, L, wm.shadow[ei], k, ns, seed, &blk, &target, &r, &max_dist)) return false;
+        qq.r = r;
+        qq.cut = max_dist;
+        qq.sp = 0;
+        if (scan_any<true>(blk, L, r, max_dist, cull, &qq.meshes)) return false;
+        if (qq.meshes) return true;
+        atomicAdd(&wm.vis[target], 1);
+        return false;
+      },
+      [&](MeshWalk& qq) { return walk_any_step(qq, s, st, blk, L, &err); },
+      [&](MeshWalk&, int32_t res) {
         if (res == kAnyClear) atomicAdd(&wm.vis[target], 1);
       },
       &err);
@@ -711,16 +806,22 @@ int set_smem(K kern, size_t smem, const char* what) {
   return ensure_smem(reinterpret_cast<const void*>(kern), smem, what);
 }
 
-template <bool kMesh, bool kTex, bool kStaged>
+template <bool kMesh, bool kTex, bool kStaged, bool kScan>
 int launch_wave(const MjpbrScene& s, uint32_t seed, cudaStream_t stream, int32_t chunk, int32_t per_world) {
   const size_t stack = (size_t)kThreads * stack_entries(s.settings.stack_depth) * 8;
   // world blocks staged in shared memory, or read in place when they do not fit
   const size_t blk_bytes = kStaged ? (size_t)s.world_block_floats * sizeof(float) : 0;
-  auto k_primary = wave_primary_kernel<kMesh, kStaged>;
+  auto k_primary = wave_primary_kernel<kMesh, kStaged, kScan>;
   auto k_surface = wave_surface_kernel<kMesh, kTex, kStaged>;
-  auto k_mirror = wave_mirror_kernel<kMesh>;
+  auto k_mirror = [] {
+    if constexpr (kScan) return &wave_mirror_scan_kernel;
+    else return &wave_mirror_kernel<kMesh>;
+  }();
   auto k_msurface = wave_mirror_surface_kernel<kMesh, kTex>;
-  auto k_shadow = wave_shadow_kernel<kMesh>;
+  auto k_shadow = [] {
+    if constexpr (kScan) return &wave_shadow_scan_kernel;
+    else return &wave_shadow_kernel<kMesh>;
+  }();
   auto k_resolve = wave_resolve_kernel<kTex, kStaged>;
   int rc = set_smem(k_primary, blk_bytes + stack, "wavefront primary");
   if (!rc) rc = set_smem(k_surface, blk_bytes, "wavefront surface");
@@ -837,17 +938,31 @@ int render_wave_launch(const MjpbrScene& s, uint32_t seed, cudaStream_t stream) 
   }
   const bool mesh = s.nmesh + s.nhfield > 0 && s.blas_root != nullptr;
   const bool tex = s.settings.textures || s.settings.has_env || s.settings.env_background;
-  const size_t stack = (size_t)kThreads * stack_entries(s.settings.stack_depth) * 8;
-  if (world_block_staged(s.world_block_floats, stack)) {
-    if (mesh && tex) return launch_wave<true, true, true>(s, seed, stream, chunk, per_world);
-    if (mesh) return launch_wave<true, false, true>(s, seed, stream, chunk, per_world);
-    if (tex) return launch_wave<false, true, true>(s, seed, stream, chunk, per_world);
-    return launch_wave<false, false, true>(s, seed, stream, chunk, per_world);
+  if (fused_supported(s)) {
+    // the whole frame is one kernel: the profile's first stage
+    stage_mark(stream);
+    const int rc = render_fused_launch(s, seed, stream);
+    for (int k = 0; k < kStages; ++k) stage_mark(stream);
+    return rc;
   }
-  if (mesh && tex) return launch_wave<true, true, false>(s, seed, stream, chunk, per_world);
-  if (mesh) return launch_wave<true, false, false>(s, seed, stream, chunk, per_world);
-  if (tex) return launch_wave<false, true, false>(s, seed, stream, chunk, per_world);
-  return launch_wave<false, false, false>(s, seed, stream, chunk, per_world);
+  const size_t stack = (size_t)kThreads * stack_entries(s.settings.stack_depth) * 8;
+  const bool staged = world_block_staged(s.world_block_floats, stack);
+  auto launch = [&](auto m, auto t, auto b, auto scan) {
+    return launch_wave<decltype(m)::value, decltype(t)::value, decltype(b)::value, decltype(scan)::value>(s, seed, stream, chunk, per_world);
+  };
+  using std::bool_constant;
+  auto pick = [&](auto b) {
+    if (mesh && tex) return launch(bool_constant<true>{}, bool_constant<true>{}, b, bool_constant<false>{});
+    if (mesh) return launch(bool_constant<true>{}, bool_constant<false>{}, b, bool_constant<false>{});
+    if (tex) return launch(bool_constant<false>{}, bool_constant<true>{}, b, bool_constant<false>{});
+    return launch(bool_constant<false>{}, bool_constant<false>{}, b, bool_constant<false>{});
+  };
+  if (!staged) return pick(bool_constant<false>{});
+  if (mesh && s.nbvh_geom <= kScanGeoms) {
+    if (tex) return launch(bool_constant<true>{}, bool_constant<true>{}, bool_constant<true>{}, bool_constant<true>{});
+    return launch(bool_constant<true>{}, bool_constant<false>{}, bool_constant<true>{}, bool_constant<true>{});
+  }
+  return pick(bool_constant<true>{});
 }
 
 }  // namespace mjpbr

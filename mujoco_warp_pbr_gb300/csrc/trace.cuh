@@ -136,52 +136,69 @@ MJ_DEV float mesh_query(const MjpbrScene& sc, const Stack& st, int sp0, int32_t 
   return best;
 }
 
+// Primitive geom g (plane, sphere, ellipsoid, capsule, cylinder, box) against the ray: distance (or
+// -1) in w, world normal in x, y, z; -1 for the geoms traced through a triangle BVH. One copy in the
+// binary for every query of a kernel: a kernel's hot code has to stay in the instruction cache.
+#ifndef MJPBR_PRIM_INLINE
+#define MJPBR_PRIM_INLINE __noinline__
+#endif
+static __device__ MJPBR_PRIM_INLINE float4 primitive_hit(const float* g, V3 o, V3 d) {
+  const Ray r{o, d};
+  const GeomFrame f = geom_frame(g);
+  V3 n = v3(0.0f);
+  float t = -1.0f;
+  switch (__float_as_int(g[3])) {
+    case MJPBR_GEOM_PLANE:
+      MJPBR_COUNT(kOpPlane);
+      t = ray_plane(f, r, &n);
+      break;
+    case MJPBR_GEOM_SPHERE:
+      MJPBR_COUNT(kOpSphere);
+      t = ray_sphere(f, r, &n);
+      break;
+    case MJPBR_GEOM_ELLIPSOID:
+      MJPBR_COUNT(kOpEllipsoid);
+      t = ray_ellipsoid(f, r, &n);
+      break;
+    case MJPBR_GEOM_CAPSULE:
+      MJPBR_COUNT(kOpCapsule);
+      t = ray_capsule(f, r, &n);
+      break;
+    case MJPBR_GEOM_CYLINDER:
+      MJPBR_COUNT(kOpCylinder);
+      t = ray_cylinder(f, r, &n);
+      break;
+    case MJPBR_GEOM_BOX:
+      MJPBR_COUNT(kOpBoxPrim);
+      t = ray_box(f, r, &n);
+      break;
+    default:
+      break;
+  }
+  return make_float4(n.x, n.y, n.z, t);
+}
+
+MJ_DEV float intersect_primitive(const float* g, const Ray& r, V3* n) {
+  const float4 h = primitive_hit(g, r.o, r.d);
+  *n = V3{h.x, h.y, h.z};
+  return h.w;
+}
+
 // One geom against the ray: distance (or -1), world normal, mesh hit details. Height fields are
 // traced as meshes (the reference's traverse.py:161-164 queries MuJoCo Warp's height-field mesh BVH).
 template <bool kMesh>
 MJ_DEV float intersect_geom(const MjpbrScene& sc, const Stack& st, int sp, const float* g, const Ray& r, float max_t,
                             bool cull, bool any, V3* n, float* u, float* v, int32_t* face, int32_t* mesh, int32_t* err) {
   const int32_t type = __float_as_int(g[3]);
+  if (!kMesh || (type != MJPBR_GEOM_MESH && type != MJPBR_GEOM_SDF && type != MJPBR_GEOM_HFIELD)) return intersect_primitive(g, r, n);
+  const int32_t mid = __float_as_int(g[17]);  // triangle BVH (a height field's follows the meshes')
+  if (mid < 0) return -1.0f;
   const GeomFrame f = geom_frame(g);
-  float d = -1.0f;
-  switch (type) {
-    case MJPBR_GEOM_PLANE:
-      MJPBR_COUNT(kOpPlane);
-      d = ray_plane(f, r, n);
-      break;
-    case MJPBR_GEOM_SPHERE:
-      MJPBR_COUNT(kOpSphere);
-      d = ray_sphere(f, r, n);
-      break;
-    case MJPBR_GEOM_ELLIPSOID:
-      MJPBR_COUNT(kOpEllipsoid);
-      d = ray_ellipsoid(f, r, n);
-      break;
-    case MJPBR_GEOM_CAPSULE:
-      MJPBR_COUNT(kOpCapsule);
-      d = ray_capsule(f, r, n);
-      break;
-    case MJPBR_GEOM_CYLINDER:
-      MJPBR_COUNT(kOpCylinder);
-      d = ray_cylinder(f, r, n);
-      break;
-    case MJPBR_GEOM_BOX:
-      MJPBR_COUNT(kOpBoxPrim);
-      d = ray_box(f, r, n);
-      break;
-    default:
-      if (kMesh && (type == MJPBR_GEOM_MESH || type == MJPBR_GEOM_SDF || type == MJPBR_GEOM_HFIELD)) {
-        const int32_t mid = __float_as_int(g[17]);  // triangle BVH (a height field's follows the meshes')
-        if (mid >= 0) {
-          V3 lo, ld, nl = v3(0.0f);
-          map_local(f, r, &lo, &ld);
-          d = mesh_query(sc, st, sp, mid, lo, ld, max_t, cull, any, &nl, u, v, face, err);
-          *n = any ? v3(0.0f) : mul(f.mat, nl);
-          *mesh = mid;
-        }
-      }
-      break;
-  }
+  V3 lo, ld, nl = v3(0.0f);
+  map_local(f, r, &lo, &ld);
+  const float d = mesh_query(sc, st, sp, mid, lo, ld, max_t, cull, any, &nl, u, v, face, err);
+  *n = any ? v3(0.0f) : mul(f.mat, nl);
+  *mesh = mid;
   return d;
 }
 
@@ -253,34 +270,6 @@ __device__ __noinline__ Hit trace_ray(const MjpbrScene& sc, const Stack& st, con
     }
   }
   return h;
-}
-
-// Primitive geom g (plane, sphere, ellipsoid, capsule, cylinder, box) against the ray: distance or -1,
-// world normal in *n; -1 for the geoms traced through a triangle BVH.
-MJ_DEV float intersect_primitive(const float* g, const Ray& r, V3* n) {
-  const GeomFrame f = geom_frame(g);
-  switch (__float_as_int(g[3])) {
-    case MJPBR_GEOM_PLANE:
-      MJPBR_COUNT(kOpPlane);
-      return ray_plane(f, r, n);
-    case MJPBR_GEOM_SPHERE:
-      MJPBR_COUNT(kOpSphere);
-      return ray_sphere(f, r, n);
-    case MJPBR_GEOM_ELLIPSOID:
-      MJPBR_COUNT(kOpEllipsoid);
-      return ray_ellipsoid(f, r, n);
-    case MJPBR_GEOM_CAPSULE:
-      MJPBR_COUNT(kOpCapsule);
-      return ray_capsule(f, r, n);
-    case MJPBR_GEOM_CYLINDER:
-      MJPBR_COUNT(kOpCylinder);
-      return ray_cylinder(f, r, n);
-    case MJPBR_GEOM_BOX:
-      MJPBR_COUNT(kOpBoxPrim);
-      return ray_box(f, r, n);
-    default:
-      return -1.0f;
-  }
 }
 
 // Triangle BVH of geom g (a mesh's, an SDF's mesh or a height field's), -1 for none.
