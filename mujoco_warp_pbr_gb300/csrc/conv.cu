@@ -1023,34 +1023,44 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const uint16_t* __restri
 
 
 // ---- weight gradients, warp-specialised: per tap, D_tap (c_out x cin, FP32 in tensor memory) +=
-// grad_out (c_out x pixels) * input shifted by the tap (cin x pixels)^T, K = the tile's 128
-// pixels, 16 per MMA. Both operands are MN-major (channels contiguous, as NHWC stores them), so
-// they are the TMA boxes as they land: grad_out as channel-group planes of 128 pixels x 16 bytes,
-// the input as the forward kernel stages it (halo rows, one copy with halo columns for one-row
-// tiles, three dx-shifted copies otherwise). MN-major descriptors: leading byte offset = stride
-// between 8-pixel groups (128 B), stride byte offset = stride between 8-channel groups (a plane).
+// grad_out (c_out x pixels) * input shifted by the tap (cin x pixels)^T, K = the tile's pixels, 16
+// per MMA. Both operands are MN-major (channels contiguous, as NHWC stores them), so they are the
+// TMA boxes as they land: grad_out as channel-group planes of the tile's pixels x 16 bytes, the
+// input as its rows with a halo row above and below and a halo column left and right, each row as
+// channel-group planes. The 16 pixels of an MMA lie in one image row (a row is 16 pixels or more),
+// so a tap's view of them is an offset of the descriptor, whatever the row's length. MN-major
+// descriptors: leading byte offset = stride between 8-pixel groups (128 B), stride byte offset =
+// stride between 8-channel groups (a plane). With rows outside channel groups, the groups of the row
+// below follow a row's own at the same stride: one MMA takes the taps of several dy (N = their
+// number times the channels, at most 256), three times fewer and larger MMAs than tap by tap.
 // M = c_out padded to 64 or 128 (zero planes); an M = 64 accumulator holds row r in tensor-memory
-// lane 32 (r / 16) + r % 16. Warp 4 loads, warps 5-7 issue the MMAs of taps j, j + 3, j + 6, and
-// after the CTA's tiles warps 0-3 add the accumulators to grad_weight with atomics. A launch
-// covers the taps whose accumulators fit the 512 tensor-memory columns (ntap x cin); the launcher
-// loops over tap ranges.
+// lane 32 (r / 16) + r % 16. Warp 4 loads, warps 5-7 issue the MMAs of dx = 0, 1, 2; warps 0-3
+// meanwhile sum the bias gradient from the staged grad_out, and after the CTA's tiles add the
+// accumulators to grad_weight, four channels per reduction (a lane's 16 accumulators are 64
+// consecutive bytes of it). A launch covers the taps (in the order dx, dy) whose accumulators fit
+// the 512 tensor-memory columns; the launcher loops over tap ranges.
 constexpr int kWgThreads = 256;
-constexpr int kWgIssuers = 3;
 constexpr int kWgMaxStages = 6;
+#ifndef MJPBR_WG_ROWS
+#define MJPBR_WG_ROWS 2
+#endif
 
 struct WgGeom {
-  ConvGeom g;
+  ConvGeom g;          // a tile: rows x pitch pixels, a multiple of 128
   int32_t ntiles;
-  int32_t single, spitch;
+  int32_t ksteps;      // MMAs along a tile's pixels
+  int32_t spitch;      // staged pixels per row: pitch + 2
   int32_t mpad;        // MMA M: 64 or 128
-  int32_t plane;       // bytes of one input channel-group plane: (rows + 2) x spitch x 16
-  int32_t in_copy;     // bytes of one input copy: (c_in / 8) planes
-  int32_t in2_copy;    // bytes of one in2 copy: (c_in2 / 8) planes
-  int32_t a_bytes;     // grad_out planes per stage: mpad / 8 x 2 KB
+  int32_t gplane;      // bytes of a grad_out channel-group plane
+  int32_t rowplane;    // bytes of an input row's channel-group plane: spitch x 16
+  int32_t in_bytes;    // (rows + 2) rows of (c_in / 8) planes
+  int32_t in2_bytes;   // (rows + 2) rows of (c_in2 / 8) planes
+  int32_t a_bytes;     // grad_out planes per stage: mpad / 8
   int32_t in_off, in2_off, stage_bytes;
   int32_t nstage;
-  int32_t tap0, ntap;  // taps of this launch
+  int32_t tap0, ntap;  // taps of this launch, tap = dx * 3 + dy
   int32_t tmem_cols;
+  int32_t vector;      // grad_weight is 16-byte aligned
 };
 
 __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const __grid_constant__ MjpbrConvGrad p, const __grid_constant__ WgGeom wg,
@@ -1060,15 +1070,17 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
   __shared__ uint64_t full[kWgMaxStages], empty[kWgMaxStages], done;
   __shared__ uint32_t tmem_slot;
   __shared__ int32_t abort_flag;
+  __shared__ float part[128 * 9];  // bias gradient, per thread of warps 0-3
   const ConvGeom& g = wg.g;
   const int32_t cout = p.c_out, cin = g.cin;
   const int32_t nst = wg.nstage;
-  const int32_t issuers = min(kWgIssuers, wg.ntap);
+  const int32_t dx0 = wg.tap0 / 3, issuers = (wg.tap0 + wg.ntap - 1) / 3 - dx0 + 1;
+  const bool bias = p.grad_bias && wg.tap0 == 0;  // warps 0-3 read grad_out too
   const uint32_t s0 = umma::smem_addr(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // zero planes of the padded M rows (never written by the TMA)
   for (int32_t st = 0; st < nst; ++st) {
-    for (int32_t i = (cout / 8) * 128 + tid; i < wg.a_bytes / 16; i += kWgThreads) {
+    for (int32_t i = (cout / 8) * (wg.gplane / 16) + tid; i < wg.a_bytes / 16; i += kWgThreads) {
       *reinterpret_cast<uint4*>(smem + st * wg.stage_bytes + i * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
   }
@@ -1077,7 +1089,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
   if (tid == 128) {
     for (int i = 0; i < nst; ++i) {
       umma::mbar_init(&full[i], 1);
-      umma::mbar_init(&empty[i], issuers);
+      umma::mbar_init(&empty[i], issuers + (bias ? 4 : 0));
     }
     umma::mbar_init(&done, issuers);
     abort_flag = 0;
@@ -1089,10 +1101,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
   const uint32_t tmem = tmem_slot;
   volatile int32_t* abort_v = &abort_flag;
   bool ok = true;
-  const int32_t copies = wg.single ? 1 : 3;
   if (warp == 4) {
     if (lane == 0) {
-      const uint32_t bytes = (uint32_t)(16 * kTilePx * (cout / 8) + copies * (wg.in_copy + wg.in2_copy));
+      const uint32_t bytes = (uint32_t)(wg.gplane * (cout / 8) + wg.in_bytes + wg.in2_bytes);
       int32_t k = 0, issued = 0;
       for (int32_t tile = blockIdx.x; tile < wg.ntiles && ok; tile += gridDim.x, ++k) {
         int32_t img, y0, x0;
@@ -1103,11 +1114,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
         const uint32_t base = s0 + buf * wg.stage_bytes;
         umma::mbar_arrive_expect_tx(&full[buf], bytes);
         umma::tma_load_5d(base, &tm_go, &full[buf], 0, x0, y0, 0, img);
-        for (int32_t dx = 0; dx < copies; ++dx) {
-          const int32_t xs = wg.single ? x0 - 1 : dx - 1;
-          umma::tma_load_5d(base + wg.in_off + dx * wg.in_copy, &tm_in, &full[buf], 0, xs, y0 - 1, 0, img);
-          if (p.c_in2 > 0) umma::tma_load_5d(base + wg.in2_off + dx * wg.in2_copy, &tm_in2, &full[buf], 0, xs, y0 - 1, 0, img);
-        }
+        umma::tma_load_5d(base + wg.in_off, &tm_in, &full[buf], 0, x0 - 1, 0, y0 - 1, img);
+        if (p.c_in2 > 0) umma::tma_load_5d(base + wg.in2_off, &tm_in2, &full[buf], 0, x0 - 1, 0, y0 - 1, img);
         issued = k + 1;
       }
       if (!ok) {
@@ -1117,9 +1125,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
     }
   } else if (warp >= 5 && warp < 5 + issuers) {
     if (lane == 0) {
-      const int32_t j = warp - 5;
-      const uint32_t id_in = umma::make_idesc_bf16((uint32_t)wg.mpad, (uint32_t)p.c_in) | (1u << 15) | (1u << 16);
-      const uint32_t id_in2 = p.c_in2 > 0 ? umma::make_idesc_bf16((uint32_t)wg.mpad, (uint32_t)p.c_in2) | (1u << 15) | (1u << 16) : 0u;
+      const int32_t dx = dx0 + warp - 5;
+      const int32_t dy0 = max(wg.tap0 - dx * 3, 0), dy1 = min(wg.tap0 + wg.ntap - dx * 3, 3);
+      const uint32_t id = umma::make_idesc_bf16((uint32_t)wg.mpad, 0) | (1u << 15) | (1u << 16);
       int32_t k = 0;
       bool issued = false;
       for (int32_t tile = blockIdx.x; tile < wg.ntiles && ok; tile += gridDim.x, ++k) {
@@ -1128,20 +1136,22 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
         if (!ok) break;
         umma::fence_after_sync();
         const uint32_t base = s0 + buf * wg.stage_bytes;
-        const uint64_t a0 = umma::make_desc(base, 128, 2048);
-        const uint64_t b_in = umma::make_desc(base + wg.in_off, 128, wg.plane);
-        const uint64_t b_in2 = umma::make_desc(base + wg.in2_off, 128, wg.plane);
-        for (int32_t t = j; t < wg.ntap; t += kWgIssuers) {
-          const int32_t tap = wg.tap0 + t, dy = tap / 3, dx = tap % 3;
-          // start of the tap's view of the staged input, in 16-byte units
-          const uint32_t sh = wg.single ? (uint32_t)(dy * wg.spitch + dx) : (uint32_t)(dx * wg.in_copy + dy * g.pitch * 16) >> 4;
-          const uint32_t sh2 = wg.single ? sh : (uint32_t)(dx * wg.in2_copy + dy * g.pitch * 16) >> 4;
-          const uint32_t d = tmem + (uint32_t)(t * cin);
+        const uint64_t a0 = umma::make_desc(base, 128, wg.gplane);
+        for (int32_t src = 0; src < (p.c_in2 > 0 ? 2 : 1); ++src) {
+          const int32_t c = src ? p.c_in2 : p.c_in;
+          const int32_t most = min(3, 256 / c);  // dy of one MMA
+          const uint64_t b0 = umma::make_desc(base + (src ? wg.in2_off : wg.in_off), 128, wg.rowplane);
+          const uint32_t row16 = (uint32_t)(c / 8 * wg.rowplane) >> 4;
+          for (int32_t dy = dy0; dy < dy1; dy += most) {
+            const int32_t n = min(most, dy1 - dy) * c;
+            const uint32_t idesc = id | ((uint32_t)n >> 3) << 17;
+            const uint32_t d = tmem + (uint32_t)((src ? wg.ntap * p.c_in : 0) + (dx * 3 + dy - wg.tap0) * c);
 #pragma unroll 1
-          for (int32_t ks = 0; ks < kTilePx / 16; ++ks) {
-            const bool acc = k > 0 || ks > 0;
-            umma::mma_bf16(d, a0 + ks * 16, b_in + sh + ks * 16, id_in, acc);
-            if (p.c_in2 > 0) umma::mma_bf16(d + (uint32_t)p.c_in, a0 + ks * 16, b_in2 + sh2 + ks * 16, id_in2, acc);
+            for (int32_t ks = 0; ks < wg.ksteps; ++ks) {
+              const int32_t row = ks * 16 / g.pitch;
+              const uint32_t at = (uint32_t)(row + dy) * row16 + (uint32_t)(ks * 16 - row * g.pitch + dx);
+              umma::mma_bf16(d, a0 + ks * 16, b0 + at, idesc, k > 0 || ks > 0);
+            }
           }
         }
         umma::commit(&empty[buf]);
@@ -1152,20 +1162,56 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
       if (!ok && issued) umma::mbar_wait(&done, 0);
     }
   } else if (warp < 4) {
+    // ---- bias gradient: 128 / (c_out / 8) threads per channel group, each its pixels of every tile ----
+    if (bias) {
+      const int32_t groups = cout / 8, share = 128 / groups;
+      const int32_t cg = tid / share, p0 = tid - cg * share;
+      float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      int32_t k = 0;
+      for (int32_t tile = blockIdx.x; tile < wg.ntiles && ok; tile += gridDim.x, ++k) {
+        const int32_t buf = k % nst;
+        ok = __all_sync(0xFFFFFFFFu, ws_wait(&full[buf], (k / nst) & 1, abort_v, kEpilogueBackoffNs));
+        if (!ok) break;
+        if (cg < groups) {
+          const uint8_t* plane = smem + buf * wg.stage_bytes + cg * wg.gplane;
+          for (int32_t px = p0; px < wg.ksteps * 16; px += share) {
+            const uint4 v = *reinterpret_cast<const uint4*>(plane + px * 16);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              acc[2 * i] += __uint_as_float(w[i] << 16);
+              acc[2 * i + 1] += __uint_as_float(w[i] & 0xFFFF0000u);
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) umma::mbar_arrive(&empty[buf]);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) part[tid * 9 + i] = acc[i];
+    }
     // ---- epilogue: accumulator rows -> grad_weight ----
-    ok = ws_wait(&done, 0, abort_v, kEpilogueBackoffNs);
+    ok = ok && ws_wait(&done, 0, abort_v, kEpilogueBackoffNs);
     if (__all_sync(0xFFFFFFFFu, ok)) {
       umma::fence_after_sync();
       const int32_t row = wg.mpad == 128 ? tid : (lane < 16 ? warp * 16 + lane : -1);
       for (int32_t t = 0; t < wg.ntap; ++t) {
-        const int32_t tap = wg.tap0 + t;
+        const int32_t tap = wg.tap0 + t, dx = tap / 3, dy = tap - dx * 3;
         for (int32_t c0 = 0; c0 < cin; c0 += 16) {
+          const int32_t col = c0 < p.c_in ? t * p.c_in + c0 : wg.ntap * p.c_in + t * p.c_in2 + c0 - p.c_in;
           float v[16];
-          umma::tmem_load16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * cin + c0), v);
+          umma::tmem_load16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)col, v);
           if (row >= 0 && row < cout) {
-            float* gw = p.grad_weight + ((int64_t)row * 9 + tap) * cin + c0;
+            float* gw = p.grad_weight + ((int64_t)row * 9 + dy * 3 + dx) * cin + c0;
+            if (wg.vector) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) atomicAdd(gw + i, v[i]);
+              for (int i = 0; i < 16; i += 4) {
+                atomicAdd(reinterpret_cast<float4*>(gw + i), make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) atomicAdd(gw + i, v[i]);
+            }
           }
         }
       }
@@ -1176,49 +1222,69 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
   if (!ok && tid % 32 == 0 && p.error_word) atomicOr(p.error_word, kErrWaitTimeout);
   umma::fence_before_sync();
   __syncthreads();
+  if (bias && tid < cout && !*abort_v) {
+    const int32_t share = 128 / (cout / 8);
+    float sum = 0.0f;
+    for (int32_t i = 0; i < share; ++i) sum += part[((tid >> 3) * share + i) * 9 + (tid & 7)];
+    atomicAdd(p.grad_bias + tid, sum);
+  }
   if (warp == 0) umma::tmem_free(tmem, (uint32_t)wg.tmem_cols);
 }
 
+// Tensor map of a BF16 NHWC activation as 5-D (8 channels, pixel, channel group, row, image): a box
+// lands as rows of channel-group planes.
+int make_row_map(CUtensorMap* m, const void* base, int32_t ch, int32_t w, int32_t h, int32_t n, int32_t bw, int32_t bh) {
+  const cuuint64_t dims[5] = {8, (cuuint64_t)w, (cuuint64_t)(ch / 8), (cuuint64_t)h, (cuuint64_t)n};
+  const cuuint64_t strides[4] = {(cuuint64_t)ch * 2, 16, (cuuint64_t)w * ch * 2, (cuuint64_t)h * w * ch * 2};
+  const cuuint32_t box[5] = {8, (cuuint32_t)bw, (cuuint32_t)(ch / 8), (cuuint32_t)bh, 1};
+  return encode(m, base, 5, dims, strides, box);
+}
 
 constexpr int kWgradWsUnsuitable = -1000;
 
 // Plans and launches conv3x3_wgrad_ws_kernel over the tap ranges that fit tensor memory;
 // kWgradWsUnsuitable when two stages do not fit shared memory (the caller falls back).
 int wgrad_ws_launch(const MjpbrConvGrad& c, const WgradGeom& gg, cudaStream_t stream) {
+  if (c.c_out > 128 || c.c_in > 256 || c.c_in2 > 256) return kWgradWsUnsuitable;  // M and N of an MMA
   WgGeom wg;
   wg.g.pitch = gg.pitch;
-  wg.g.rows = gg.rows;
   wg.g.tiles_per_row = gg.tiles_per_row;
-  wg.g.tiles_per_img = gg.tiles_per_img;
   wg.g.cin = gg.cin;
-  wg.ntiles = gg.total;
-  wg.single = gg.rows == 1;
-  wg.spitch = wg.single ? gg.pitch + 2 : gg.pitch;
+  wg.spitch = gg.pitch + 2;
   wg.mpad = c.c_out <= 64 ? 64 : 128;
-  if (c.c_out > 128) return kWgradWsUnsuitable;
-  const int32_t copies = wg.single ? 1 : 3;
+  wg.rowplane = wg.spitch * 16;
+  wg.vector = aligned16(c.grad_weight);
+  // image rows per tile: 128 pixels' worth, doubled while the image divides and two stages fit (a tile
+  // loads two halo rows beside its own)
   auto round128 = [](int64_t v) { return (int32_t)((v + 127) / 128 * 128); };
-  wg.plane = (gg.rows + 2) * wg.spitch * 16;
-  wg.in_copy = (c.c_in / 8) * wg.plane;
-  wg.in2_copy = (c.c_in2 / 8) * wg.plane;
-  wg.a_bytes = wg.mpad / 8 * 2048;
-  wg.in_off = wg.a_bytes;
-  wg.in2_off = round128((int64_t)wg.in_off + (int64_t)copies * wg.in_copy);
-  wg.stage_bytes = round128((int64_t)wg.in2_off + (int64_t)copies * wg.in2_copy);
-  // TMA destinations are 128-byte aligned: the dx copies must be too
-  if (!wg.single && ((wg.in_copy % 128) || (wg.in2_copy % 128))) return kWgradWsUnsuitable;
-  wg.nstage = std::min<int64_t>(kWgMaxStages, (int64_t)kPipeSmemMax / wg.stage_bytes);
-  if (wg.nstage < 2) return kWgradWsUnsuitable;
+  auto plan = [&](int32_t rows) {
+    wg.g.rows = rows;
+    wg.ksteps = rows * gg.pitch / 16;
+    wg.gplane = rows * gg.pitch * 16;
+    wg.a_bytes = wg.mpad / 8 * wg.gplane;
+    wg.in_bytes = (rows + 2) * (c.c_in / 8) * wg.rowplane;
+    wg.in2_bytes = (rows + 2) * (c.c_in2 / 8) * wg.rowplane;
+    wg.in_off = wg.a_bytes;
+    wg.in2_off = round128((int64_t)wg.in_off + wg.in_bytes);  // TMA destinations are 128-byte aligned
+    wg.stage_bytes = round128((int64_t)wg.in2_off + wg.in2_bytes);
+    wg.nstage = std::min<int64_t>(kWgMaxStages, (int64_t)kPipeSmemMax / wg.stage_bytes);
+    return wg.nstage;
+  };
+  int32_t rows = gg.rows;
+  while (rows < MJPBR_WG_ROWS * gg.rows && c.height % (2 * rows) == 0 && plan(2 * rows) >= 2) rows *= 2;
+  if (plan(rows) < 2) return kWgradWsUnsuitable;
+  wg.g.tiles_per_img = (c.height / rows) * gg.tiles_per_row;
+  wg.ntiles = c.nimg * wg.g.tiles_per_img;
   const size_t smem = (size_t)wg.nstage * wg.stage_bytes;
   if (int rc = ensure_smem(reinterpret_cast<const void*>(conv3x3_wgrad_ws_kernel), kPipeSmemMax, "conv3x3 wgrad")) return rc;
   CUtensorMap tm_go, tm_in, tm_in2;
   memset(&tm_in2, 0, sizeof(tm_in2));
-  if (make_act_map(&tm_go, c.grad_out, c.c_out, c.width, c.height, c.nimg, gg.pitch, gg.rows, c.c_out / 8) != 0) return MJPBR_ERR_CUDA;
-  if (make_act_map(&tm_in, c.in, c.c_in, c.width, c.height, c.nimg, wg.spitch, gg.rows + 2, c.c_in / 8) != 0) return MJPBR_ERR_CUDA;
-  if (c.c_in2 > 0 && make_act_map(&tm_in2, c.in2, c.c_in2, c.width, c.height, c.nimg, wg.spitch, gg.rows + 2, c.c_in2 / 8) != 0) return MJPBR_ERR_CUDA;
+  if (make_act_map(&tm_go, c.grad_out, c.c_out, c.width, c.height, c.nimg, gg.pitch, rows, c.c_out / 8) != 0) return MJPBR_ERR_CUDA;
+  if (make_row_map(&tm_in, c.in, c.c_in, c.width, c.height, c.nimg, wg.spitch, rows + 2) != 0) return MJPBR_ERR_CUDA;
+  if (c.c_in2 > 0 && make_row_map(&tm_in2, c.in2, c.c_in2, c.width, c.height, c.nimg, wg.spitch, rows + 2) != 0) return MJPBR_ERR_CUDA;
   const int32_t per_pass = std::min(9, 512 / gg.cin);
   if (per_pass < 1) return kWgradWsUnsuitable;
-  const int64_t grid = std::min<int64_t>(gg.total, conv_sm_count());
+  const int64_t grid = std::min<int64_t>(wg.ntiles, conv_sm_count());
   for (int32_t t0 = 0; t0 < 9; t0 += per_pass) {
     wg.tap0 = t0;
     wg.ntap = std::min(per_pass, 9 - t0);
@@ -1260,13 +1326,7 @@ int conv3x3_wgrad_launch(const MjpbrConvGrad& c, cudaStream_t stream) {
   if (conv_pipeline_enabled() && (c.c_in2 == 0 || c.in2_full) && (int64_t)c.nimg * c.height * c.width <= INT32_MAX) {
     const int rc = wgrad_ws_launch(c, g, stream);
     if (rc != kWgradWsUnsuitable) {
-      if (rc != MJPBR_OK) return rc;
-      if (c.grad_bias) {
-        const int64_t npix = (int64_t)c.nimg * c.height * c.width;
-        bias_grad_kernel<<<(unsigned)((npix + kBiasPix - 1) / kBiasPix), 256, 0, stream>>>(c.grad_out, npix, c.c_out, c.grad_bias);
-        return check_launch("bias_grad_kernel");
-      }
-      return MJPBR_OK;
+      return rc;
     }
   }
   const int32_t mblocks = (9 * g.cin + 127) / 128;

@@ -174,6 +174,54 @@ def test_conv3x3_wgrad_matches_cpu(nimg, h, w, c1, c2, cout, per_cta, full):
   np.testing.assert_allclose(gb.cpu().numpy(), ref_b + 0.25, rtol=1e-4, atol=1e-4 * scale)
 
 
+# the edges of the weight gradient's plan: heights that hold one, two or an odd number of rows per tile,
+# taps over several launches, one to three rows of taps per MMA, both accumulator heights, channels past
+# an MMA's, and an output that is not 16-byte aligned
+WGRAD_EDGES = [
+  # nimg, h, w, c1, c2, cout, offset of the output in floats
+  (2, 6, 128, 32, 0, 32, 0),
+  (1, 5, 128, 48, 0, 48, 0),
+  (2, 24, 16, 96, 0, 96, 0),
+  (1, 8, 32, 64, 96, 64, 0),
+  (1, 2, 256, 144, 0, 128, 0),
+  (1, 8, 16, 272, 0, 16, 0),
+  (1, 4, 64, 16, 16, 16, 1),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("nimg,h,w,c1,c2,cout,offset", WGRAD_EDGES)
+def test_conv3x3_wgrad_edges_match_cpu(nimg, h, w, c1, c2, cout, offset):
+  from mujoco_warp_pbr_gb300 import _lib
+
+  g = torch.Generator().manual_seed(h * 1000 + w + c1 + c2 + cout)
+  x = (torch.rand((nimg, h, w, c1), generator=g) * 2 - 1).to(torch.bfloat16)
+  x2 = (torch.rand((nimg, h, w, c2), generator=g) * 2 - 1).to(torch.bfloat16) if c2 else None
+  dy = (torch.rand((nimg, h, w, cout), generator=g) * 2 - 1).to(torch.bfloat16)
+  ref_w, ref_b = wgrad_ref(
+    x.float().numpy().astype(np.float64), dy.float().numpy().astype(np.float64), None if x2 is None else x2.float().numpy().astype(np.float64)
+  )
+  n = cout * 9 * (c1 + c2)
+  gw = torch.zeros(n + offset, dtype=torch.float32, device="cuda")[offset:]
+  gb = torch.zeros(cout, dtype=torch.float32, device="cuda")
+  err = torch.zeros(1, dtype=torch.int32, device="cuda")
+  dx, dx2, ddy = x.cuda(), (x2.cuda() if x2 is not None else None), dy.cuda()
+  c = _lib.ConvGrad(
+    in_=dx.data_ptr(), in2=dx2.data_ptr() if dx2 is not None else None, grad_out=ddy.data_ptr(), grad_weight=gw.data_ptr(),
+    grad_bias=gb.data_ptr(), error_word=err.data_ptr(), nimg=nimg, height=h, width=w, c_in=c1, c_in2=c2, c_out=cout, tiles_per_cta=0, in2_full=1,
+  )
+  _lib.call("mjpbr_conv3x3_wgrad_bf16", ctypes.byref(c), torch.cuda.current_stream().cuda_stream)
+  torch.cuda.synchronize()
+  assert int(err.item()) == 0
+  # sums of nimg * h * w products below 1 (exact in FP32), accumulated in FP32: partial sums stay below
+  # 4 sqrt(n), and each of n additions rounds by 2^-24 of them
+  k = nimg * h * w
+  atol = k * 2.0**-24 * 4.0 * np.sqrt(k)
+  np.testing.assert_allclose(gw.cpu().numpy().reshape(ref_w.shape), ref_w, rtol=0, atol=atol)
+  np.testing.assert_allclose(gb.cpu().numpy(), ref_b, rtol=0, atol=atol)
+
+
 @pytest.mark.gpu
 @pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
 def test_upsample2_is_nearest():
