@@ -469,6 +469,15 @@ int mjpbr_unpool_add_grad(const float* dskip, const float* dpool, const uint16_t
  * (c_in, 9, c_out) tap-reversed copy of a convolution weight. */
 int mjpbr_adam(float* param, float* grad, float* m, float* v, uint16_t* copy, uint16_t* flip, int64_t n, int32_t cout, int32_t cin,
                float lr, float beta1, float beta2, float eps, int32_t step, void* stream);
+/* mjpbr_adam of count parameter arrays in one launch per MJPBR_ADAM_BATCH of them. */
+#define MJPBR_ADAM_BATCH 32
+typedef struct MjpbrAdamParam {
+  float *param, *grad, *m, *v;
+  uint16_t *copy, *flip;
+  int64_t n;
+  int32_t cout, cin;
+} MjpbrAdamParam;
+int mjpbr_adam_many(const MjpbrAdamParam* params, int32_t count, float lr, float beta1, float beta2, float eps, int32_t step, void* stream);
 
 /* mjpbr_refit_bvh + mjpbr_render in one call that allocates nothing and takes no scratch from the
  * caller: the per-world blocks and the path tracer's work counter live in static device memory of

@@ -49,6 +49,12 @@ class KpcnWeights(ctypes.Structure):
   _fields_ = [("weight", c_vp * KPCN_LAYERS), ("bias", c_vp * KPCN_LAYERS)]
 
 
+class AdamParam(ctypes.Structure):
+  """MjpbrAdamParam."""
+
+  _fields_ = [("param", c_vp), ("grad", c_vp), ("m", c_vp), ("v", c_vp), ("copy", c_vp), ("flip", c_vp), ("n", ctypes.c_int64), ("cout", c_i32), ("cin", c_i32)]
+
+
 class Texture(ctypes.Structure):
   """MjpbrTexture."""
 
@@ -332,6 +338,7 @@ _SIGNATURES = {
   "mjpbr_kpcn_apply_grad": (ctypes.c_int, [c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_vp]),
   "mjpbr_split_concat_grad": (ctypes.c_int, [c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_i32, c_i32, c_vp]),
   "mjpbr_unpool_add_grad": (ctypes.c_int, [c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_i32, c_vp]),
+  "mjpbr_adam_many": (ctypes.c_int, [ctypes.POINTER(AdamParam), c_i32, ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float, c_i32, c_vp]),
   "mjpbr_adam": (
     ctypes.c_int,
     [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, ctypes.c_int64, c_i32, c_i32, ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float, c_i32, c_vp],

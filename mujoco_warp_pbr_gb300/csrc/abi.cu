@@ -381,6 +381,10 @@ int mjpbr_unpool_add_grad(const float* dskip, const float* dpool, const uint16_t
   return unpool_add_grad_launch(dskip, dpool, act, dact, nimg, h, w, c, static_cast<cudaStream_t>(stream));
 }
 
+int mjpbr_adam_many(const MjpbrAdamParam* params, int32_t count, float lr, float beta1, float beta2, float eps, int32_t step, void* stream) {
+  return adam_many_launch(params, count, lr, beta1, beta2, eps, step, static_cast<cudaStream_t>(stream));
+}
+
 int mjpbr_adam(float* param, float* grad, float* m, float* v, uint16_t* copy, uint16_t* flip, int64_t n, int32_t cout, int32_t cin,
                float lr, float beta1, float beta2, float eps, int32_t step, void* stream) {
   return adam_launch(param, grad, m, v, copy, flip, n, cout, cin, lr, beta1, beta2, eps, step, static_cast<cudaStream_t>(stream));

@@ -70,6 +70,7 @@ int split_concat_grad_launch(const float* dcat, const uint16_t* low, float* dski
                              int32_t c1, int32_t c2, cudaStream_t st);
 int unpool_add_grad_launch(const float* dskip, const float* dpool, const uint16_t* act, uint16_t* dact, int32_t nimg, int32_t h,
                            int32_t w, int32_t c, cudaStream_t st);
+int adam_many_launch(const MjpbrAdamParam* params, int32_t count, float lr, float beta1, float beta2, float eps, int32_t step, cudaStream_t st);
 int adam_launch(float* param, float* grad, float* m, float* v, uint16_t* copy, uint16_t* flip, int64_t n, int32_t cout, int32_t cin,
                 float lr, float beta1, float beta2, float eps, int32_t step, cudaStream_t st);
 int newton_sync_poses_launch(const float* body_q, int32_t nbody, const int32_t* shape_body, const float* shape_transform,

@@ -11,6 +11,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "abi_internal.h"
 #include "denoise_common.cuh"
@@ -363,25 +364,34 @@ __global__ void unpool_add_grad_kernel(const float* __restrict__ dskip, const fl
 
 // Adam on FP32 master parameters; refreshes the BF16 copy (c_out, 9, c_in) and, when flip is
 // given, the input-gradient copy (c_in, 9, c_out) with the taps reversed; zeroes the gradient.
-__global__ void adam_kernel(float* __restrict__ param, float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
-                            uint16_t* __restrict__ copy, uint16_t* __restrict__ flip, int64_t n, int32_t cout, int32_t cin, float lr,
-                            float beta1, float beta2, float eps, float bc1, float bc2) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float g = grad[i];
-  const float mi = beta1 * m[i] + (1.0f - beta1) * g;
-  const float vi = beta2 * v[i] + (1.0f - beta2) * g * g;
-  m[i] = mi;
-  v[i] = vi;
-  const float p = param[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-  param[i] = p;
-  grad[i] = 0.0f;
-  if (copy) copy[i] = bf16_bits(p);
-  if (flip) {
-    const int32_t ci = (int32_t)(i % cin);
-    const int32_t tap = (int32_t)((i / cin) % 9);
-    const int32_t co = (int32_t)(i / ((int64_t)cin * 9));
-    flip[((int64_t)ci * 9 + (8 - tap)) * cout + co] = bf16_bits(p);
+// The parameter arrays of a network (a weight and a bias per layer, most of them smaller than a
+// wave) share one launch: `first` gives each array its run of CTAs.
+struct AdamBatch {
+  int32_t count;
+  int32_t first[MJPBR_ADAM_BATCH + 1];
+  MjpbrAdamParam p[MJPBR_ADAM_BATCH];
+};
+
+__global__ void adam_kernel(const __grid_constant__ AdamBatch b, float lr, float beta1, float beta2, float eps, float bc1, float bc2) {
+  int32_t k = 0;
+  while (k + 1 < b.count && (int32_t)blockIdx.x >= b.first[k + 1]) ++k;
+  const MjpbrAdamParam& a = b.p[k];
+  const int64_t i = (int64_t)((int32_t)blockIdx.x - b.first[k]) * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  const float g = a.grad[i];
+  const float mi = beta1 * a.m[i] + (1.0f - beta1) * g;
+  const float vi = beta2 * a.v[i] + (1.0f - beta2) * g * g;
+  a.m[i] = mi;
+  a.v[i] = vi;
+  const float p = a.param[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+  a.param[i] = p;
+  a.grad[i] = 0.0f;
+  if (a.copy) a.copy[i] = bf16_bits(p);
+  if (a.flip) {
+    const int32_t ci = (int32_t)(i % a.cin);
+    const int32_t tap = (int32_t)((i / a.cin) % 9);
+    const int32_t co = (int32_t)(i / ((int64_t)a.cin * 9));
+    a.flip[((int64_t)ci * 9 + (8 - tap)) * a.cout + co] = bf16_bits(p);
   }
 }
 
@@ -512,13 +522,34 @@ int unpool_add_grad_launch(const float* dskip, const float* dpool, const uint16_
   return check_launch("unpool_add_grad_kernel");
 }
 
+int adam_many_launch(const MjpbrAdamParam* params, int32_t count, float lr, float beta1, float beta2, float eps, int32_t step, cudaStream_t st) {
+  if (!params || count < 1 || step < 1) return set_error(MJPBR_ERR_ARG, "adam: bad arguments");
+  for (int32_t k = 0; k < count; ++k) {
+    const MjpbrAdamParam& a = params[k];
+    if (!a.param || !a.grad || !a.m || !a.v || a.n <= 0) return set_error(MJPBR_ERR_ARG, "adam: bad arguments");
+    if (a.flip && (a.cout < 1 || a.cin < 1 || (int64_t)a.cout * 9 * a.cin != a.n)) return set_error(MJPBR_ERR_ARG, "adam: flip needs n = c_out * 9 * c_in");
+  }
+  const float bc1 = 1.0f - powf(beta1, (float)step), bc2 = 1.0f - powf(beta2, (float)step);
+  for (int32_t k0 = 0; k0 < count; k0 += MJPBR_ADAM_BATCH) {
+    AdamBatch b = {};
+    b.count = std::min(count - k0, MJPBR_ADAM_BATCH);
+    int64_t total = 0;
+    for (int32_t k = 0; k < b.count; ++k) {
+      b.p[k] = params[k0 + k];
+      total += (b.p[k].n + 255) / 256;
+      if (total > INT32_MAX) return set_error(MJPBR_ERR_ARG, "adam: too many parameters for one launch");
+      b.first[k + 1] = (int32_t)total;
+    }
+    adam_kernel<<<(unsigned)total, 256, 0, st>>>(b, lr, beta1, beta2, eps, bc1, bc2);
+    if (int rc = check_launch("adam_kernel")) return rc;
+  }
+  return MJPBR_OK;
+}
+
 int adam_launch(float* param, float* grad, float* m, float* v, uint16_t* copy, uint16_t* flip, int64_t n, int32_t cout, int32_t cin,
                 float lr, float beta1, float beta2, float eps, int32_t step, cudaStream_t st) {
-  if (!param || !grad || !m || !v || n <= 0 || step < 1) return set_error(MJPBR_ERR_ARG, "adam: bad arguments");
-  if (flip && (cout < 1 || cin < 1 || (int64_t)cout * 9 * cin != n)) return set_error(MJPBR_ERR_ARG, "adam: flip needs n = c_out * 9 * c_in");
-  const float bc1 = 1.0f - powf(beta1, (float)step), bc2 = 1.0f - powf(beta2, (float)step);
-  adam_kernel<<<blocks(n, 256), 256, 0, st>>>(param, grad, m, v, copy, flip, n, cout, cin, lr, beta1, beta2, eps, bc1, bc2);
-  return check_launch("adam_kernel");
+  const MjpbrAdamParam one = {param, grad, m, v, copy, flip, n, cout, cin};
+  return adam_many_launch(&one, 1, lr, beta1, beta2, eps, step, st);
 }
 
 }  // namespace mjpbr

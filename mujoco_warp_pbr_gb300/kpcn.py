@@ -327,12 +327,13 @@ class KPCN:
 
   def adam(self, lr: float, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1.0e-8) -> None:
     self.step_count += 1
-    st = self._stream()
+    params = []
     for l in self.layers.values():
       s = l.spec
-      cin = s.c_in + s.c_in2
-      _lib.call("mjpbr_adam", _ptr(l.w), _ptr(l.gw), _ptr(l.mw), _ptr(l.vw), _ptr(l.w16), _ptr(l.flip16), l.w.numel(), s.c_out, cin, lr, beta1, beta2, eps, self.step_count, st)
-      _lib.call("mjpbr_adam", _ptr(l.b), _ptr(l.gb), _ptr(l.mb), _ptr(l.vb), None, None, l.b.numel(), 0, 0, lr, beta1, beta2, eps, self.step_count, st)
+      params.append((_ptr(l.w), _ptr(l.gw), _ptr(l.mw), _ptr(l.vw), _ptr(l.w16), _ptr(l.flip16), l.w.numel(), s.c_out, s.c_in + s.c_in2))
+      params.append((_ptr(l.b), _ptr(l.gb), _ptr(l.mb), _ptr(l.vb), None, None, l.b.numel(), 0, 0))
+    table = (_lib.AdamParam * len(params))(*params)
+    _lib.call("mjpbr_adam_many", table, len(params), lr, beta1, beta2, eps, self.step_count, self._stream())
 
   def train_step(self, x0: torch.Tensor, radiance: torch.Tensor, target: torch.Tensor, lr: float, scale: torch.Tensor | None = None, offset: torch.Tensor | None = None) -> torch.Tensor:
     self.forward(x0, radiance, train=True)
