@@ -7,10 +7,10 @@
 // K-major core-matrix layout (8 pixels x 16 bytes), so that the A operand of tap (dy, dx) is one
 // descriptor with a uniform 16-byte row stride.
 //
-// conv3x3_ws_kernel (the default, further below) is a persistent warp-specialised kernel whose
-// operands arrive by TMA. conv3x3_kernel, directly below, is the first version: one CTA per tile
-// staging three dx-shifted copies of its rows with plain loads (MJPBR_CONV_PIPELINE=0 selects it,
-// as do batches of more than 2^31 pixels).
+// conv3x3_flat_kernel (the default, further below) and conv3x3_ws_kernel (half-resolution skips) are
+// persistent warp-specialised kernels whose operands arrive by TMA. conv3x3_kernel, directly below, is
+// the first version: one CTA per tile staging three dx-shifted copies of its rows with plain loads
+// (MJPBR_CONV_PIPELINE=0 selects it, as do batches of more than 2^31 pixels).
 //
 // The U-Net's skip concatenation is read in place: channels past c_in come from in2, either at
 // the output resolution (in2_full) or at half of it, upsampled x2 (nearest) while staging.
@@ -206,7 +206,6 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_kernel(const __grid_c
 
 constexpr int kWsThreads = 192;
 constexpr int kMaxStages = 4;
-constexpr int kMaxSlots = 8;  // row-ring slots
 
 struct WsGeom {
   ConvGeom g;
@@ -224,38 +223,7 @@ struct WsGeom {
   int32_t s2_off, b_off;
   int32_t nstage;
   int32_t acc_cols;  // tensor-memory columns of one accumulator
-  // row ring (tiles of one image row, resident weights): each CTA takes a contiguous range of
-  // tiles ordered down the image columns and loads every input row once into a ring of nslot
-  // slots of 2 x (c_in + c_in2) / 16 planes of (pitch + 2) pixels
-  int32_t ring;
-  int32_t nslot;
-  int32_t slot_bytes;
-  int32_t rowplane;  // bytes of one row plane: (pitch + 2) x 16
-  int32_t in2_off;   // offset of the in2 planes in a slot (a multiple of 128)
 };
-
-// The i-th tile of this CTA: strided over the grid, or (ring) the i-th of a contiguous range in
-// column-major order (image, tile column, row). False past the CTA's last tile.
-__device__ __forceinline__ bool cta_tile(const WsGeom& wg, int32_t i, int32_t& img, int32_t& y0, int32_t& x0) {
-  const ConvGeom& g = wg.g;
-  if (wg.ring) {
-    const int32_t t = (int32_t)((int64_t)blockIdx.x * wg.ntiles / gridDim.x) + i;
-    if (t >= (int32_t)((int64_t)(blockIdx.x + 1) * wg.ntiles / gridDim.x)) return false;
-    const int32_t h = g.tiles_per_img / g.tiles_per_row;  // image rows
-    const int32_t col = t / h;
-    y0 = t - col * h;
-    img = col / g.tiles_per_row;
-    x0 = (col - img * g.tiles_per_row) * g.pitch;
-    return true;
-  }
-  const int32_t tile = blockIdx.x + i * gridDim.x;
-  if (tile >= wg.ntiles) return false;
-  img = tile / g.tiles_per_img;
-  const int32_t t = tile - img * g.tiles_per_img;
-  y0 = (t / g.tiles_per_row) * g.rows;
-  x0 = (t % g.tiles_per_row) * g.pitch;
-  return true;
-}
 
 struct StageInfo {
   int32_t in2;  // chunks of in2 (else of in)
@@ -335,7 +303,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
                                                                    const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_in2,
                                                                    const __grid_constant__ CUtensorMap tm_w) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ uint64_t full[kMaxSlots], ready[kMaxSlots], empty[kMaxSlots];
+  __shared__ uint64_t full[kMaxStages], ready[kMaxStages], empty[kMaxStages];
   __shared__ uint64_t acc_full[2], acc_empty[2], wbar, drain;
   __shared__ uint32_t tmem_slot;
   __shared__ int32_t abort_flag;
@@ -351,7 +319,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
   const uint32_t ncols = 2u * (uint32_t)wg.acc_cols;
   if (warp == 0) umma::tmem_alloc(&tmem_slot, ncols);
   if (tid == 128) {
-    for (int i = 0; i < (wg.ring ? wg.nslot : nst); ++i) {
+    for (int i = 0; i < nst; ++i) {
       umma::mbar_init(&full[i], 1);
       umma::mbar_init(&ready[i], 1);
       umma::mbar_init(&empty[i], 1);
@@ -384,28 +352,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
       umma::tma_load_4d(s0 + wg.b_off, &tm_w, &wbar, 0, 0, 0, 0);
     }
     int32_t k = 0, issued = 0, prev_in2 = 0, prev_nc = 0, prev_y0 = 0;
-    if (wg.ring) {
-      // one load per input row: the rows of a run of tiles down one tile column plus the
-      // halo rows above and below (outside the image the TMA reads zeros)
-      const uint32_t row_bytes = (uint32_t)(16 * wg.spitch * 2 * nchunk);
-      int32_t i = 0, img, y0, x0;
-      while (lane == 0 && ok && cta_tile(wg, i, img, y0, x0)) {
-        int32_t n = 1, img2, y2, x2;
-        while (cta_tile(wg, i + n, img2, y2, x2) && img2 == img && x2 == x0) ++n;
-        for (int32_t r = y0 - 1; r <= y0 + n && ok; ++r, ++k) {
-          const int32_t slot = k % wg.nslot;
-          if (k >= wg.nslot) ok = ws_wait(&empty[slot], ((k / wg.nslot) + 1) & 1, abort_v, kLoaderBackoffNs);
-          if (!ok) break;
-          const uint32_t sa = s0 + slot * wg.slot_bytes;
-          umma::mbar_arrive_expect_tx(&full[slot], row_bytes);
-          umma::tma_load_5d(sa, &tm_in, &full[slot], 0, x0 - 1, r, 0, img);
-          if (p.c_in2 > 0) umma::tma_load_5d(sa + wg.in2_off, &tm_in2, &full[slot], 0, x0 - 1, r, 0, img);
-          issued = k + 1;
-        }
-        i += n;
-      }
-    }
-    for (int32_t tile = wg.ring ? wg.ntiles : blockIdx.x; tile < wg.ntiles && ok; tile += gridDim.x) {
+    for (int32_t tile = blockIdx.x; tile < wg.ntiles && ok; tile += gridDim.x) {
       int32_t img, y0, x0;
       tile_origin(g, tile, img, y0, x0);
       for (int32_t sidx = 0; sidx < nsp && ok; ++sidx, ++k) {
@@ -463,8 +410,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
     }
     if (!ok && lane == 0) {
       // the copies in flight land before the CTA's shared memory is released
-      const int32_t nb = wg.ring ? wg.nslot : nst;
-      for (int32_t kk = max(0, issued - nb); kk < issued; ++kk) umma::mbar_wait(&full[kk % nb], (kk / nb) & 1);
+      for (int32_t kk = max(0, issued - nst); kk < issued; ++kk) umma::mbar_wait(&full[kk % nst], (kk / nst) & 1);
     }
   } else if (warp == 5) {
     // ---- MMA issuer ----
@@ -477,52 +423,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
       const uint32_t bchunk16 = (uint32_t)(2 * cout);
       if (wg.resident) ok = ws_wait(&wbar, 0, abort_v);
       int32_t k = 0, i = 0, last = -1;
-      if (wg.ring) {
-        // tile row y of a run uses the ring rows y - 1, y, y + 1 (loads base + j, j = y - y_run
-        // + dy); a row is released after its last tile: row y - 1 after tile y, and the run's last
-        // two rows after its last tile
-        const uint64_t b_all = umma::make_desc(s0 + wg.b_off, cout * 16, 128);
-        const uint32_t plane16 = (uint32_t)wg.rowplane >> 4;
-        int32_t base = 0, waited = 0, img, y0, x0;
-        while (ok && cta_tile(wg, i, img, y0, x0)) {
-          int32_t n = 1, img2, y2, x2;
-          while (cta_tile(wg, i + n, img2, y2, x2) && img2 == img && x2 == x0) ++n;
-          for (int32_t j = 0; j < n && ok; ++j, ++i) {
-            const int32_t b = i & 1;
-            if (i >= 2) ok = ws_wait(&acc_empty[b], ((i >> 1) + 1) & 1, abort_v);
-            while (ok && waited <= base + j + 2) {
-              ok = ws_wait(&full[waited % wg.nslot], (waited / wg.nslot) & 1, abort_v);
-              ++waited;
-            }
-            if (!ok) break;
-            umma::fence_after_sync();
-            const uint32_t acc = tmem + (uint32_t)(b * wg.acc_cols);
-            for (int32_t dy = 0; dy < 3; ++dy) {
-              const uint32_t slot_addr = s0 + ((base + j + dy) % wg.nslot) * wg.slot_bytes;
-              const uint64_t a_row = umma::make_desc(slot_addr, wg.rowplane, 128);
-              const uint64_t a_in2 = umma::make_desc(slot_addr + wg.in2_off, wg.rowplane, 128);
-              for (int32_t cc = 0; cc < nchunk; ++cc) {
-                const uint64_t ad = cc < nci ? a_row + 2 * cc * plane16 : a_in2 + 2 * (cc - nci) * plane16;
-                const uint64_t bd = b_all + cc * bchunk16;
-#pragma unroll
-                for (int32_t dx = 0; dx < 3; ++dx) {
-                  umma::mma_bf16(acc, ad + dx, bd + (dy * 3 + dx) * btap16, idesc, dy > 0 || cc > 0 || dx > 0);
-                }
-              }
-            }
-            umma::commit(&empty[(base + j) % wg.nslot]);
-            last = (base + j) % wg.nslot;
-            if (j == n - 1) {
-              umma::commit(&empty[(base + j + 1) % wg.nslot]);
-              umma::commit(&empty[(base + j + 2) % wg.nslot]);
-            }
-            umma::commit(&acc_full[b]);
-          }
-          base += n + 2;
-        }
-        k = waited;
-      }
-      for (int32_t tile = wg.ring ? wg.ntiles : blockIdx.x; tile < wg.ntiles && ok; tile += gridDim.x, ++i) {
+      for (int32_t tile = blockIdx.x; tile < wg.ntiles && ok; tile += gridDim.x, ++i) {
         const int32_t b = i & 1;
         if (i >= 2) ok = ws_wait(&acc_empty[b], ((i >> 1) + 1) & 1, abort_v);
         if (!ok) break;
@@ -562,7 +463,9 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
     // ---- epilogue: warp w reads accumulator rows (pixels) 32 w .. 32 w + 31 ----
     const int32_t m = tid;
     int32_t img, y0, x0;
-    for (int32_t i = 0; cta_tile(wg, i, img, y0, x0); ++i) {
+    int32_t i = 0;
+    for (int32_t tile = blockIdx.x; tile < wg.ntiles; tile += gridDim.x, ++i) {
+      tile_origin(g, tile, img, y0, x0);
       const int32_t b = i & 1;
       ok = ws_wait(&acc_full[b], (i >> 1) & 1, abort_v, kEpilogueBackoffNs);
       // tcgen05.ld is warp-collective
@@ -620,6 +523,316 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
   if (warp == 0) umma::tmem_free(tmem, ncols);
 }
 
+// ---- blocks of padded rows: the kernel of every layer whose operands fit (conv3x3_ws_kernel takes the
+// rest: half-resolution skips and very wide layers).
+//
+// A block is T x 128 consecutive positions of an image strip's rows laid end to end, each row with its
+// two halo columns (pitch + 2 positions): in that order the input of tap (dy, dx) lies dy rows and dx
+// positions further, for every position, so one staged copy serves all taps of images of any width.
+// The two positions per row that are halo columns compute garbage that is not stored (1.5 % of the
+// work at 128 pixels a row, 3 % at 64, 6 % at 32, 11 % at 16), where tiles of whole short rows needed
+// three shifted copies of every row. A block stages its rows and two halo rows once for T
+// accumulators: 11 rows for 7.9 at 128 pixels and T = 8, where single tiles staged 3 rows for 1.
+//
+// One CTA per SM. Warp 8 loads stages (all channels of a block, or G 16-channel chunks at a time); warps
+// 9 and 10 issue the MMAs of the even and odd accumulators of a block (one thread issues an MMA every
+// 65 clk at best, the tensor pipe takes one every 40 at N = 32); warps 0-7 run the epilogue, warps 0-3
+// the even, 4-7 the odd accumulators, while the next block's MMAs fill the other half of tensor
+// memory. Barriers: full / empty per stage, acc_full / acc_empty per half.
+//
+// The sum's order: chunk by chunk with the nine taps inside, or (`by_row`, the layers whose weights fit
+// beside four rows of input) row by row of taps with the chunks inside.
+//
+// Bound by MMA issue and the operands' shared-memory reads (45 MMAs of N = 32 a tile in the widest
+// layer, 52 clocks each against the 40 that reading 5 KB takes), by HBM in the first layer. 1024 images
+// of 128 x 128 and their lower levels, us: the network's 15 layers 10,500 -> 5,090; its decoder's first
+// layer (32 + 48 -> 32) 2,375 -> 1,096, one level down (48 + 64 -> 48) 1,488 -> 480, 32 -> 32 channels
+// 937 -> 509. T at most 6: at 8 a stage of all channels leaves room for two stages only (541), at 4 the
+// halo rows are 7 for 4 (565).
+constexpr int kFlatThreads = 352;
+constexpr int kFlatMaxStages = 6;
+constexpr size_t kFlatSmem = 208 * 1024;
+#ifndef MJPBR_FLAT_TILES
+#define MJPBR_FLAT_TILES 6
+#endif
+
+struct FlatGeom {
+  int32_t pitch, prow;     // pixels of a strip's row; with its halo columns
+  int32_t strips;          // strips of an image (width / pitch)
+  int32_t tiles;           // 128-position tiles of a strip
+  int32_t blocks, nblock;  // blocks of a strip; of the batch
+  int32_t T;               // tiles of a block
+  int32_t nrow;            // staged rows of a block
+  int32_t plane;           // bytes of a channel-group plane of a stage: nrow x prow x 16
+  int32_t group;           // chunks of a stage; 0: all chunks of both inputs
+  int32_t by_row;
+  int32_t resident;        // weights resident, else per stage
+  int32_t in2_off, b_off;  // offsets in a stage of in2's planes (group 0) and of its weights
+  int32_t stage_bytes, nstage;
+  int32_t tmem_cols;
+  int32_t wide;            // 32-byte aligned outputs
+  uint32_t row_magic;      // position / prow = its product with row_magic, high word (positions below 2^24; else 0)
+};
+
+// The image strip and first position of a block.
+__device__ __forceinline__ void flat_block(const FlatGeom& fg, int32_t b, int32_t& img, int32_t& x0, int32_t& t0) {
+  const int32_t strip = b / fg.blocks;
+  t0 = (b - strip * fg.blocks) * fg.T;
+  img = strip / fg.strips;
+  x0 = (strip - img * fg.strips) * fg.pitch;
+}
+
+__device__ __forceinline__ void store_bf16x16(uint16_t* o, const float* v, bool wide) {
+  uint32_t w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) w[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+                 "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+  } else {
+    reinterpret_cast<uint4*>(o)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    reinterpret_cast<uint4*>(o)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
+
+__device__ __forceinline__ void store_f32x16(float* o, const float* v, bool wide) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 8) {
+    if (wide) {
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + i), "f"(v[i]), "f"(v[i + 1]), "f"(v[i + 2]), "f"(v[i + 3]),
+                   "f"(v[i + 4]), "f"(v[i + 5]), "f"(v[i + 6]), "f"(v[i + 7])
+                   : "memory");
+    } else {
+      reinterpret_cast<float4*>(o + i)[0] = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+      reinterpret_cast<float4*>(o + i)[1] = make_float4(v[i + 4], v[i + 5], v[i + 6], v[i + 7]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kFlatThreads, 1) conv3x3_flat_kernel(const __grid_constant__ MjpbrConv p, const __grid_constant__ FlatGeom fg,
+                                                                       const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_in2,
+                                                                       const __grid_constant__ CUtensorMap tm_w) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ uint64_t full[kFlatMaxStages], empty[kFlatMaxStages], acc_full[2], acc_empty[2], wbar, drain[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int32_t abort_flag;
+  __shared__ __align__(16) float sbias[256];
+  const int32_t cout = p.c_out;
+  const int32_t nci = p.c_in / 16, nchunk = nci + p.c_in2 / 16;
+  const int32_t G = fg.group;
+  const int32_t nsp = G ? (nci + G - 1) / G + (nchunk - nci + G - 1) / G : 1;  // stages of a block
+  const int32_t nst = fg.nstage;
+  const uint32_t s0 = umma::smem_addr(smem);
+  const uint32_t stages0 = s0 + (fg.resident ? (uint32_t)(9 * 2 * nchunk * cout * 16 + 255) / 256 * 256 : 0u);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+  if (warp == 0) umma::tmem_alloc(&tmem_slot, (uint32_t)fg.tmem_cols);
+  for (int32_t i = tid; i < cout; i += kFlatThreads) sbias[i] = p.bias ? __ldg(p.bias + i) : 0.0f;
+  if (tid == 256) {
+    for (int i = 0; i < nst; ++i) {
+      umma::mbar_init(&full[i], 1);
+      umma::mbar_init(&empty[i], 2);
+    }
+    for (int i = 0; i < 2; ++i) {
+      umma::mbar_init(&acc_full[i], 2);
+      umma::mbar_init(&acc_empty[i], 8);
+      umma::mbar_init(&drain[i], 1);
+    }
+    umma::mbar_init(&wbar, 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tmem = tmem_slot;
+  volatile int32_t* abort_v = &abort_flag;
+  bool ok = true;
+
+  if (warp == 8) {
+    if (lane == 0) {
+      if (fg.resident) {
+        umma::mbar_arrive_expect_tx(&wbar, (uint32_t)(9 * 2 * nchunk * cout * 16));
+        umma::tma_load_4d(s0, &tm_w, &wbar, 0, 0, 0, 0);
+      }
+      int32_t k = 0, issued = 0;
+      for (int32_t b = blockIdx.x; b < fg.nblock && ok; b += gridDim.x) {
+        int32_t img, x0, t0;
+        flat_block(fg, b, img, x0, t0);
+        const int32_t y = t0 * 128 / fg.prow - 1;
+        for (int32_t sidx = 0; sidx < nsp && ok; ++sidx, ++k) {
+          const int32_t buf = k % nst;
+          if (k >= nst) ok = ws_wait(&empty[buf], ((k / nst) + 1) & 1, abort_v, 64);
+          if (!ok) break;
+          const uint32_t base = stages0 + buf * fg.stage_bytes;
+          if (!G) {
+            umma::mbar_arrive_expect_tx(&full[buf], (uint32_t)(2 * nchunk * fg.plane));
+            umma::tma_load_5d(base, &tm_in, &full[buf], 0, x0 - 1, y, 0, img);
+            if (p.c_in2 > 0) umma::tma_load_5d(base + fg.in2_off, &tm_in2, &full[buf], 0, x0 - 1, y, 0, img);
+          } else {
+            const StageInfo st = stage_info(sidx, nci, nchunk, G);
+            umma::mbar_arrive_expect_tx(&full[buf], (uint32_t)(2 * G * fg.plane) + (fg.resident ? 0u : (uint32_t)(9 * 2 * G * cout * 16)));
+            umma::tma_load_5d(base, st.in2 ? &tm_in2 : &tm_in, &full[buf], 0, x0 - 1, y, st.in2 ? st.cs - nci : st.cs, img);
+            if (!fg.resident) umma::tma_load_4d(base + fg.b_off, &tm_w, &full[buf], 0, 0, 2 * st.cs, 0);
+          }
+          issued = k + 1;
+        }
+      }
+      if (!ok) {
+        // the copies in flight land before the CTA's shared memory is released
+        for (int32_t kk = max(0, issued - nst); kk < issued; ++kk) umma::mbar_wait(&full[kk % nst], (kk / nst) & 1);
+        if (fg.resident) umma::mbar_wait(&wbar, 0);
+      }
+    }
+  } else if (warp >= 9) {
+    // all lanes run the loops (mma_bf16_lead)
+    const uint32_t lead = lane == 0;
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xFFFFFFFFu, ws_wait(bar, parity, abort_v)) != 0; };
+    const int32_t j = warp - 9;
+    const uint32_t idesc = umma::make_idesc_bf16(kTilePx, cout);
+    const uint32_t chunk16 = (uint32_t)(2 * fg.plane) >> 4;
+    const uint32_t btap16 = (uint32_t)((fg.resident ? 2 * nchunk : 2 * G) * cout);
+    const uint32_t bchunk16 = (uint32_t)(2 * cout);
+    const uint32_t row16 = (uint32_t)(2 * fg.prow);
+    if (fg.resident) ok = wait(&wbar, 0);
+    bool issued = false;
+    int32_t k = 0, i = 0;
+    for (int32_t b = blockIdx.x; b < fg.nblock && ok; b += gridDim.x, ++i) {
+      int32_t img, x0, t0;
+      flat_block(fg, b, img, x0, t0);
+      const int32_t nt = min(fg.T, fg.tiles - t0);
+      const int32_t off = t0 * 128 - t0 * 128 / fg.prow * fg.prow;
+      const int32_t half = i & 1;
+      if (i >= 2) ok = wait(&acc_empty[half], ((i >> 1) + 1) & 1);
+      for (int32_t sidx = 0; sidx < nsp && ok; ++sidx, ++k) {
+        const int32_t buf = k % nst;
+        ok = wait(&full[buf], (k / nst) & 1);
+        if (!ok) break;
+        umma::fence_after_sync();
+        const uint32_t base = stages0 + buf * fg.stage_bytes;
+        StageInfo st = {0, 0, nchunk};
+        if (G) st = stage_info(sidx, nci, nchunk, G);
+        const uint64_t bd0 = fg.resident ? umma::make_desc(s0, cout * 16, 128) + (uint64_t)(st.cs * bchunk16) : umma::make_desc(base + fg.b_off, cout * 16, 128);
+        for (int32_t t = j; t < nt; t += 2) {
+          const uint32_t acc = tmem + (uint32_t)((half * fg.T + t) * cout);
+          const uint64_t ad0 = umma::make_desc_sw32(base) + (uint64_t)(2 * (off + t * 128));
+          const uint64_t ad2 = umma::make_desc_sw32(base + fg.in2_off) + (uint64_t)(2 * (off + t * 128));
+          if (fg.by_row) {
+#pragma unroll 1
+            for (int32_t dy = 0; dy < 3; ++dy) {
+#pragma unroll 1
+              for (int32_t cc = 0; cc < nchunk; ++cc) {
+                const uint64_t ad = (cc < nci ? ad0 + cc * chunk16 : ad2 + (cc - nci) * chunk16) + (uint64_t)(dy * row16);
+                const uint64_t bd = bd0 + cc * bchunk16 + dy * 3 * btap16;
+                umma::mma_bf16_lead(lead, acc, ad, bd, idesc, (dy > 0 || cc > 0) ? 1u : 0u);
+                umma::mma_bf16_lead(lead, acc, ad + 2, bd + btap16, idesc, 1u);
+                umma::mma_bf16_lead(lead, acc, ad + 4, bd + 2 * btap16, idesc, 1u);
+              }
+            }
+          } else {
+#pragma unroll 1
+            for (int32_t cc = 0; cc < st.nc; ++cc) {
+              const uint64_t ad = (G || cc < nci) ? ad0 + cc * chunk16 : ad2 + (cc - nci) * chunk16;
+              const uint64_t bd = bd0 + cc * bchunk16;
+              umma::mma_bf16_lead(lead, acc, ad, bd, idesc, (sidx > 0 || cc > 0) ? 1u : 0u);
+#pragma unroll
+              for (int32_t tap = 1; tap < 9; ++tap) {
+                umma::mma_bf16_lead(lead, acc, ad + tap / 3 * row16 + 2 * (tap % 3), bd + tap * btap16, idesc, 1u);
+              }
+            }
+          }
+        }
+        umma::commit_lead(lead, &empty[buf]);
+        issued = true;
+      }
+      if (!ok) break;
+      umma::commit_lead(lead, &acc_full[half]);
+    }
+    if (!ok && issued) {
+      // the MMAs in flight complete before their operands and accumulators are released
+      umma::commit_lead(lead, &drain[j]);
+      umma::mbar_wait(&drain[j], 0);
+    }
+  } else {
+    // ---- epilogue: warp w reads accumulator rows (positions) 32 (w % 4) .. + 31 of tiles of its parity ----
+    const int32_t m = (warp & 3) * 32 + lane, parity = warp >> 2;
+    int32_t i = 0;
+    for (int32_t b = blockIdx.x; b < fg.nblock; b += gridDim.x, ++i) {
+      int32_t img, x0, t0;
+      flat_block(fg, b, img, x0, t0);
+      const int32_t nt = min(fg.T, fg.tiles - t0), half = i & 1;
+      ok = ws_wait(&acc_full[half], (i >> 1) & 1, abort_v, 32);
+      // tcgen05.ld is warp-collective
+      if (!__all_sync(0xFFFFFFFFu, ok)) {
+        ok = false;
+        *abort_v = 1;
+        break;
+      }
+      umma::fence_after_sync();
+      for (int32_t t = parity; t < nt; t += 2) {
+        const int32_t f = (t0 + t) * 128 + m;
+        const int32_t row = fg.row_magic ? (int32_t)__umulhi((uint32_t)f, fg.row_magic) : f / fg.prow, col = f - row * fg.prow;
+        const bool inside = col < fg.pitch && row < p.height;
+        const int64_t pix = ((int64_t)img * p.height + row) * p.width + x0 + col;
+        const uint32_t acc = tmem + (uint32_t)((half * fg.T + t) * cout) + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll 1
+        for (int32_t c0 = 0; c0 < cout; c0 += 32) {
+          const bool two = c0 + 32 <= cout;
+          uint4 mk[4];
+          if (p.mask && inside) {  // in flight while the accumulator is read
+            const uint4* src = reinterpret_cast<const uint4*>(p.mask + pix * cout + c0);
+            mk[0] = __ldg(src), mk[1] = __ldg(src + 1);
+            if (two) mk[2] = __ldg(src + 2), mk[3] = __ldg(src + 3);
+          }
+          float v[32];
+          if (two) {
+            umma::tmem_load32(acc + c0, v);
+          } else {
+            umma::tmem_load16(acc + c0, v);
+          }
+          if (!inside) continue;
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            if (hf && !two) break;
+            float* u = v + 16 * hf;
+            const int32_t c = c0 + 16 * hf;
+            if (p.bias) {
+#pragma unroll
+              for (int q = 0; q < 16; q += 4) {
+                const float4 bq = *reinterpret_cast<const float4*>(sbias + c + q);
+                u[q] += bq.x, u[q + 1] += bq.y, u[q + 2] += bq.z, u[q + 3] += bq.w;
+              }
+            }
+            if (p.relu) {
+#pragma unroll
+              for (int q = 0; q < 16; ++q) u[q] = fmaxf(u[q], 0.0f);
+            }
+            if (p.mask) {
+              const uint4 m0 = mk[2 * hf], m1 = mk[2 * hf + 1];
+              const uint32_t wv[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                if ((wv[q] & 0x8000u) || !(wv[q] & 0x7FFFu)) u[2 * q] = 0.0f;
+                if ((wv[q] & 0x80000000u) || !(wv[q] & 0x7FFF0000u)) u[2 * q + 1] = 0.0f;
+              }
+            }
+            if (p.out) store_bf16x16(p.out + pix * cout + c, u, fg.wide);
+            if (p.out_f32) store_f32x16(p.out_f32 + pix * cout + c, u, fg.wide);
+          }
+        }
+      }
+      // the half is free for the block after next once every warp has read its rows
+      umma::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(&acc_empty[half]);
+    }
+  }
+  if (!ok && tid % 32 == 0 && p.error_word) atomicOr(p.error_word, kErrWaitTimeout);
+  umma::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) umma::tmem_free(tmem, (uint32_t)fg.tmem_cols);
+}
+
 bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; }
 
 }  // namespace
@@ -657,12 +870,13 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-int encode(CUtensorMap* m, const void* base, cuuint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
+int encode(CUtensorMap* m, const void* base, cuuint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
+           CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE) {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return set_error(MJPBR_ERR_CUDA, "conv3x3: cuTensorMapEncodeTiled is unavailable");
   const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                        swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return set_error(MJPBR_ERR_CUDA, "conv3x3: cuTensorMapEncodeTiled failed (%d)", (int)r);
   return 0;
 }
@@ -678,6 +892,15 @@ int make_act_map(CUtensorMap* m, const void* base, int32_t ch, int32_t w, int32_
   return encode(m, base, 5, dims, strides, box);
 }
 
+// The same by 16-channel chunks in the 32-byte swizzle: a box of `chunks` x 16 channels x bw pixels x
+// bh rows lands as planes of bh x bw x 32 bytes, half the pieces of 16-byte planes.
+int make_chunk_map(CUtensorMap* m, const void* base, int32_t ch, int32_t w, int32_t h, int32_t n, int32_t bw, int32_t bh, int32_t chunks) {
+  const cuuint64_t dims[5] = {16, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)(ch / 16), (cuuint64_t)n};
+  const cuuint64_t strides[4] = {(cuuint64_t)ch * 2, (cuuint64_t)w * ch * 2, 32, (cuuint64_t)h * w * ch * 2};
+  const cuuint32_t box[5] = {16, (cuuint32_t)bw, (cuuint32_t)bh, (cuuint32_t)chunks, 1};
+  return encode(m, base, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_32B);
+}
+
 // Tensor map of the weights [c_out][9 taps][cin] as 4-D (8 channels, output channel, channel
 // group, tap): a box of `groups` channel groups lands as [tap][group][c_out] x 16 bytes, the
 // K-major B operand of every tap.
@@ -688,7 +911,7 @@ int make_weight_map(CUtensorMap* m, const void* base, int32_t cin, int32_t cout,
   return encode(m, base, 4, dims, strides, box);
 }
 
-// MJPBR_CONV_RING=0 keeps single-row tiles on the staged pipeline (kept for comparison).
+// MJPBR_CONV_RING=0 sums every layer chunk by chunk (kept for comparison).
 bool conv_ring_enabled() {
   static int enabled = -1;
   if (enabled < 0) {
@@ -709,6 +932,79 @@ bool conv_pipeline_enabled() {
 }
 
 }  // namespace
+
+// Plans and launches conv3x3_flat_kernel; kFlatUnsuitable when no plan fits. by_row: the accumulation
+// order (the row-ring layers').
+constexpr int kFlatUnsuitable = -1001;
+
+static int flat_launch(const MjpbrConv& c, const ConvGeom& g, bool by_row, cudaStream_t stream) {
+  FlatGeom fg = {};
+  fg.pitch = g.pitch;
+  fg.prow = g.pitch + 2;
+  fg.strips = c.width / g.pitch;
+  if ((int64_t)c.height * fg.prow > INT32_MAX - 1024) return kFlatUnsuitable;
+  fg.tiles = (c.height * fg.prow + 127) / 128;
+  fg.row_magic = c.height * fg.prow < (1 << 24) ? (uint32_t)((((uint64_t)1 << 32) + fg.prow - 1) / fg.prow) : 0u;
+  fg.by_row = by_row;
+  fg.wide = ((reinterpret_cast<uintptr_t>(c.out) | reinterpret_cast<uintptr_t>(c.out_f32)) & 31u) == 0;
+  const int32_t nchunk = g.cin / 16, nci = c.c_in / 16, cout = c.c_out;
+  auto round256 = [](size_t v) { return (v + 255) / 256 * 256; };
+  const size_t wbytes = (size_t)9 * 2 * nchunk * cout * 16;
+  // stages of a block of T tiles: all channels when two such stages fit, else G chunks at a time
+  auto plan = [&](int32_t T) {
+    fg.T = T;
+    fg.nrow = (T * 128 + fg.prow) / fg.prow + 3;
+    if (fg.nrow > 256) return false;
+    fg.plane = fg.nrow * fg.prow * 16;
+    fg.in2_off = (int32_t)round256((size_t)2 * nci * fg.plane);
+    const size_t whole = round256((size_t)fg.in2_off + (size_t)2 * (nchunk - nci) * fg.plane);
+    if (round256(wbytes) + 2 * whole <= kFlatSmem) {
+      fg.group = 0;
+      fg.resident = 1;
+      fg.stage_bytes = (int32_t)whole;
+    } else if (by_row) {
+      return false;
+    } else {
+      const size_t abytes = round256((size_t)2 * fg.plane);
+      fg.group = 1;
+      fg.resident = round256(wbytes) + 2 * abytes <= kFlatSmem;
+      fg.b_off = (int32_t)abytes;
+      fg.stage_bytes = (int32_t)(abytes + (fg.resident ? 0 : round256((size_t)9 * 2 * cout * 16)));
+    }
+    const size_t left = kFlatSmem - (fg.resident ? round256(wbytes) : 0);
+    fg.nstage = (int32_t)std::min<size_t>(kFlatMaxStages, left / fg.stage_bytes);
+    return fg.nstage >= 2;
+  };
+  // the tiles per block that give the busiest CTA the least to do: its blocks' tiles and, per block, about
+  // one tile's time for the halo rows and the hand-over; two blocks' accumulators fit tensor memory
+  const int64_t strips = (int64_t)c.nimg * fg.strips;
+  const int32_t sms = conv_sm_count();
+  int32_t best = 0;
+  int64_t best_cost = INT64_MAX;
+  for (int32_t T = std::min(MJPBR_FLAT_TILES, 256 / cout); T >= 1; --T) {
+    if (!plan(T)) continue;
+    const int64_t nblock = strips * ((fg.tiles + T - 1) / T);
+    if (nblock > INT32_MAX) continue;
+    const int64_t cost = (nblock + sms - 1) / sms * (T + 1);
+    if (cost < best_cost) best_cost = cost, best = T;
+  }
+  if (!best || !plan(best)) return kFlatUnsuitable;
+  fg.blocks = (fg.tiles + best - 1) / best;
+  fg.nblock = (int32_t)(strips * fg.blocks);
+  fg.tmem_cols = 32;
+  while (fg.tmem_cols < 2 * best * cout) fg.tmem_cols <<= 1;
+  CUtensorMap tm_in, tm_in2, tm_w;
+  memset(&tm_in2, 0, sizeof(tm_in2));
+  if (make_chunk_map(&tm_in, c.in, c.c_in, c.width, c.height, c.nimg, fg.prow, fg.nrow, fg.group ? fg.group : nci) != 0) return MJPBR_ERR_CUDA;
+  if (c.c_in2 > 0 && make_chunk_map(&tm_in2, c.in2, c.c_in2, c.width, c.height, c.nimg, fg.prow, fg.nrow, fg.group ? fg.group : nchunk - nci) != 0) {
+    return MJPBR_ERR_CUDA;
+  }
+  if (make_weight_map(&tm_w, c.weight, g.cin, cout, fg.resident ? 2 * nchunk : 2 * fg.group) != 0) return MJPBR_ERR_CUDA;
+  if (int rc = ensure_smem(reinterpret_cast<const void*>(conv3x3_flat_kernel), kPipeSmemMax, "conv3x3")) return rc;
+  const size_t smem = (fg.resident ? round256(wbytes) : 0) + (size_t)fg.nstage * fg.stage_bytes;
+  conv3x3_flat_kernel<<<(unsigned)std::min(fg.nblock, sms), kFlatThreads, smem, stream>>>(c, fg, tm_in, tm_in2, tm_w);
+  return check_launch("conv3x3_flat_kernel");
+}
 
 int conv3x3_launch(const MjpbrConv& c, cudaStream_t stream) {
   if (!c.in || !c.weight || (!c.out && !c.out_f32)) return set_error(MJPBR_ERR_ARG, "conv3x3: missing input, weight or output");
@@ -773,36 +1069,28 @@ int conv3x3_launch(const MjpbrConv& c, cudaStream_t stream) {
     wg.group = G;
     wg.nstage = nst;
     wg.resident = resident;
-    // the row ring, when tiles are single rows, the skip input (if any) has full resolution and
-    // the weights plus at least four row slots fit
-    wg.rowplane = wg.spitch * 16;
-    wg.in2_off = (int32_t)round128((size_t)2 * nci * wg.rowplane);
-    wg.slot_bytes = (int32_t)round128((size_t)wg.in2_off + (size_t)2 * (nchunk - nci) * wg.rowplane);
-    wg.nslot = (int32_t)std::min<size_t>(kMaxSlots, budget > wbytes ? (budget - wbytes) / wg.slot_bytes : 0);
-    wg.ring = conv_ring_enabled() && wg.single && (c.c_in2 == 0 || c.in2_full) && wg.nslot >= 4;
+    // Layers whose weights and four input rows fit this budget sum row by row of taps, the others chunk by
+    // chunk (results do not depend on which kernel takes a layer).
+    if (!half_in2) {
+      const size_t rowplane = (size_t)(g.pitch + 2) * 16;
+      const size_t slot = round128(round128(2 * nci * rowplane) + 2 * (nchunk - nci) * rowplane);
+      const bool by_row = conv_ring_enabled() && wg.single && budget > wbytes && (budget - wbytes) / slot >= 4;
+      const int rc = flat_launch(c, g, by_row, stream);
+      if (rc != kFlatUnsuitable) return rc;
+    }
     wg.abuf = (int32_t)round128((size_t)copies * 2 * G * wg.plane);
     wg.s2buf = half_in2 ? (int32_t)round128((size_t)2 * G * wg.s2plane) : 0;
     wg.bstage = resident ? 0 : 9 * 2 * G * c.c_out * 16;
     wg.s2_off = nst * wg.abuf;
     wg.b_off = wg.s2_off + nst * wg.s2buf;
-    if (wg.ring) {
-      wg.resident = 1;
-      wg.b_off = wg.nslot * wg.slot_bytes;
-    }
-    const size_t smem = wg.ring ? (size_t)wg.b_off + wbytes : fixed + (size_t)nst * stage_bytes(G, resident);
+    const size_t smem = fixed + (size_t)nst * stage_bytes(G, resident);
     if (smem > kPipeSmemMax) return set_error(MJPBR_ERR_ARG, "conv3x3: %zu bytes of shared memory needed", smem);
     if (int rc = ensure_smem(reinterpret_cast<const void*>(conv3x3_ws_kernel), kPipeSmemMax, "conv3x3")) return rc;
     CUtensorMap tm_in, tm_in2, tm_w;
     memset(&tm_in2, 0, sizeof(tm_in2));
-    if (wg.ring) {
-      // boxes of one row of all channel groups of each input
-      if (make_act_map(&tm_in, c.in, c.c_in, c.width, c.height, c.nimg, wg.spitch, 1, 2 * nci) != 0) return MJPBR_ERR_CUDA;
-      if (c.c_in2 > 0 && make_act_map(&tm_in2, c.in2, c.c_in2, c.width, c.height, c.nimg, wg.spitch, 1, 2 * (nchunk - nci)) != 0) return MJPBR_ERR_CUDA;
-    } else {
-      if (make_act_map(&tm_in, c.in, c.c_in, c.width, c.height, c.nimg, wg.spitch, g.rows + 2, 2 * G) != 0) return MJPBR_ERR_CUDA;
-      if (half_in2 && make_act_map(&tm_in2, c.in2, c.c_in2, c.width / 2, c.height / 2, c.nimg, wg.s2w, wg.s2h, 2 * G) != 0) return MJPBR_ERR_CUDA;
-      if (c.c_in2 > 0 && c.in2_full && make_act_map(&tm_in2, c.in2, c.c_in2, c.width, c.height, c.nimg, wg.spitch, g.rows + 2, 2 * G) != 0) return MJPBR_ERR_CUDA;
-    }
+    if (make_act_map(&tm_in, c.in, c.c_in, c.width, c.height, c.nimg, wg.spitch, g.rows + 2, 2 * G) != 0) return MJPBR_ERR_CUDA;
+    if (half_in2 && make_act_map(&tm_in2, c.in2, c.c_in2, c.width / 2, c.height / 2, c.nimg, wg.s2w, wg.s2h, 2 * G) != 0) return MJPBR_ERR_CUDA;
+    if (c.c_in2 > 0 && c.in2_full && make_act_map(&tm_in2, c.in2, c.c_in2, c.width, c.height, c.nimg, wg.spitch, g.rows + 2, 2 * G) != 0) return MJPBR_ERR_CUDA;
     if (make_weight_map(&tm_w, c.weight, g.cin, c.c_out, wg.resident ? 2 * nchunk : 2 * G) != 0) return MJPBR_ERR_CUDA;
     // resident CTAs per SM, limited by shared memory (1 KB of it reserved per CTA), registers
     // and the 512 tensor-memory columns (two accumulators per CTA)
@@ -1039,6 +1327,9 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const uint16_t* __restri
 // accumulators to grad_weight, four channels per reduction (a lane's 16 accumulators are 64
 // consecutive bytes of it). A launch covers the taps (in the order dx, dy) whose accumulators fit
 // the 512 tensor-memory columns; the launcher loops over tap ranges.
+//
+// 64 images of 128 x 128, 32 -> 32 channels: 190 us with an MMA per tap and a bias pass, 68 so; tiles of
+// two rows (67 at four, 82 at one: three staged rows for each).
 constexpr int kWgThreads = 256;
 constexpr int kWgMaxStages = 6;
 #ifndef MJPBR_WG_ROWS
@@ -1077,7 +1368,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
   const int32_t dx0 = wg.tap0 / 3, issuers = (wg.tap0 + wg.ntap - 1) / 3 - dx0 + 1;
   const bool bias = p.grad_bias && wg.tap0 == 0;  // warps 0-3 read grad_out too
   const uint32_t s0 = umma::smem_addr(smem);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
   // zero planes of the padded M rows (never written by the TMA)
   for (int32_t st = 0; st < nst; ++st) {
     for (int32_t i = (cout / 8) * (wg.gplane / 16) + tid; i < wg.a_bytes / 16; i += kWgThreads) {
@@ -1124,43 +1415,45 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv3x3_wgrad_ws_kernel(const _
       }
     }
   } else if (warp >= 5 && warp < 5 + issuers) {
-    if (lane == 0) {
-      const int32_t dx = dx0 + warp - 5;
-      const int32_t dy0 = max(wg.tap0 - dx * 3, 0), dy1 = min(wg.tap0 + wg.ntap - dx * 3, 3);
-      const uint32_t id = umma::make_idesc_bf16((uint32_t)wg.mpad, 0) | (1u << 15) | (1u << 16);
-      int32_t k = 0;
-      bool issued = false;
-      for (int32_t tile = blockIdx.x; tile < wg.ntiles && ok; tile += gridDim.x, ++k) {
-        const int32_t buf = k % nst;
-        ok = ws_wait(&full[buf], (k / nst) & 1, abort_v);
-        if (!ok) break;
-        umma::fence_after_sync();
-        const uint32_t base = s0 + buf * wg.stage_bytes;
-        const uint64_t a0 = umma::make_desc(base, 128, wg.gplane);
-        for (int32_t src = 0; src < (p.c_in2 > 0 ? 2 : 1); ++src) {
-          const int32_t c = src ? p.c_in2 : p.c_in;
-          const int32_t most = min(3, 256 / c);  // dy of one MMA
-          const uint64_t b0 = umma::make_desc(base + (src ? wg.in2_off : wg.in_off), 128, wg.rowplane);
-          const uint32_t row16 = (uint32_t)(c / 8 * wg.rowplane) >> 4;
-          for (int32_t dy = dy0; dy < dy1; dy += most) {
-            const int32_t n = min(most, dy1 - dy) * c;
-            const uint32_t idesc = id | ((uint32_t)n >> 3) << 17;
-            const uint32_t d = tmem + (uint32_t)((src ? wg.ntap * p.c_in : 0) + (dx * 3 + dy - wg.tap0) * c);
+    // all lanes run the loops (umma::mma_bf16_lead)
+    const uint32_t lead = lane == 0;
+    const int32_t dx = dx0 + warp - 5;
+    const int32_t dy0 = max(wg.tap0 - dx * 3, 0), dy1 = min(wg.tap0 + wg.ntap - dx * 3, 3);
+    const uint32_t id = umma::make_idesc_bf16((uint32_t)wg.mpad, 0) | (1u << 15) | (1u << 16);
+    int32_t k = 0;
+    bool issued = false;
+    for (int32_t tile = blockIdx.x; tile < wg.ntiles && ok; tile += gridDim.x, ++k) {
+      const int32_t buf = k % nst;
+      ok = __all_sync(0xFFFFFFFFu, ws_wait(&full[buf], (k / nst) & 1, abort_v)) != 0;
+      if (!ok) break;
+      umma::fence_after_sync();
+      const uint32_t base = s0 + buf * wg.stage_bytes;
+      const uint64_t a0 = umma::make_desc(base, 128, wg.gplane);
+      for (int32_t src = 0; src < (p.c_in2 > 0 ? 2 : 1); ++src) {
+        const int32_t c = src ? p.c_in2 : p.c_in;
+        const int32_t most = min(3, 256 / c);  // dy of one MMA
+        const uint64_t b0 = umma::make_desc(base + (src ? wg.in2_off : wg.in_off), 128, wg.rowplane);
+        const uint32_t row16 = (uint32_t)(c / 8 * wg.rowplane) >> 4;
+        for (int32_t dy = dy0; dy < dy1; dy += most) {
+          const int32_t n = min(most, dy1 - dy) * c;
+          const uint32_t idesc = id | ((uint32_t)n >> 3) << 17;
+          const uint32_t d = tmem + (uint32_t)((src ? wg.ntap * p.c_in : 0) + (dx * 3 + dy - wg.tap0) * c);
+          int32_t row = 0, x = 0;
 #pragma unroll 1
-            for (int32_t ks = 0; ks < wg.ksteps; ++ks) {
-              const int32_t row = ks * 16 / g.pitch;
-              const uint32_t at = (uint32_t)(row + dy) * row16 + (uint32_t)(ks * 16 - row * g.pitch + dx);
-              umma::mma_bf16(d, a0 + ks * 16, b0 + at, idesc, k > 0 || ks > 0);
-            }
+          for (int32_t ks = 0; ks < wg.ksteps; ++ks) {
+            const uint32_t at = (uint32_t)(row + dy) * row16 + (uint32_t)(x + dx);
+            umma::mma_bf16_lead(lead, d, a0 + ks * 16, b0 + at, idesc, k > 0 || ks > 0);
+            x += 16;
+            if (x == g.pitch) x = 0, ++row;
           }
         }
-        umma::commit(&empty[buf]);
-        issued = true;
       }
-      // done completes once every issuer's MMAs completed
-      umma::commit(&done);
-      if (!ok && issued) umma::mbar_wait(&done, 0);
+      umma::commit_lead(lead, &empty[buf]);
+      issued = true;
     }
+    // done completes once every issuer's MMAs completed
+    umma::commit_lead(lead, &done);
+    if (!ok && issued) umma::mbar_wait(&done, 0);
   } else if (warp < 4) {
     // ---- bias gradient: 128 / (c_out / 8) threads per channel group, each its pixels of every tile ----
     if (bias) {

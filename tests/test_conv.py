@@ -111,6 +111,62 @@ def test_conv3x3_matches_cpu(nimg, h, w, c1, c2, cout, use_bias, relu, use_mask,
   np.testing.assert_allclose(out.float().cpu().numpy(), ref, rtol=1e-2, atol=1e-2)
 
 
+# blocks of padded rows: one row, blocks of one tile and of several (more blocks than CTAs), a strip's ragged
+# last tile, images of several strips, all channels per stage and one chunk, weights resident and per stage,
+# the widest output, and an output that is 16 but not 32-byte aligned
+BLOCK_CASES = [
+  # nimg, h, w, c1, c2, cout, mask, offset of the outputs in values
+  (1, 1, 128, 16, 0, 16, False, 0),
+  (170, 7, 128, 32, 0, 32, True, 0),
+  (90, 5, 384, 16, 16, 48, False, 0),
+  (200, 16, 16, 96, 0, 96, True, 0),
+  (40, 30, 64, 48, 64, 48, False, 0),
+  (2, 8, 16, 64, 96, 256, False, 0),
+  (3, 12, 32, 64, 0, 64, True, 8),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("nimg,h,w,c1,c2,cout,use_mask,offset", BLOCK_CASES)
+def test_conv3x3_blocks_match_cpu(nimg, h, w, c1, c2, cout, use_mask, offset):
+  from mujoco_warp_pbr_gb300 import _lib
+
+  g = torch.Generator().manual_seed(nimg * 1000 + h * 10 + w + c1 + c2 + cout)
+  x = (torch.rand((nimg, h, w, c1), generator=g) * 2 - 1).to(torch.bfloat16)
+  x2 = (torch.rand((nimg, h, w, c2), generator=g) * 2 - 1).to(torch.bfloat16) if c2 else None
+  wt = ((torch.rand((cout, 9, c1 + c2), generator=g) * 2 - 1) / np.sqrt(9 * (c1 + c2))).to(torch.bfloat16)
+  bias = torch.rand(cout, generator=g) - 0.5
+  mask = (torch.rand((nimg, h, w, cout), generator=g) - 0.3).to(torch.bfloat16) if use_mask else None
+  pick = sorted({0, nimg // 2, nimg - 1})  # images compared; every image is checked for what it shares below
+  ref = conv_ref(
+    x[pick].float().numpy().astype(np.float64), wt.float().numpy().astype(np.float64), bias.numpy().astype(np.float64),
+    None if x2 is None else x2[pick].float().numpy().astype(np.float64), True, None if mask is None else mask[pick].float().numpy(),
+  )
+  dev = {k: (v.cuda() if v is not None else None) for k, v in {"x": x, "x2": x2, "w": wt, "b": bias, "m": mask}.items()}
+  n = nimg * h * w * cout
+  out = torch.full((n + offset,), -1.0, dtype=torch.bfloat16, device="cuda")[offset:]
+  out32 = torch.full((n + offset // 2,), -1.0, dtype=torch.float32, device="cuda")[offset // 2 :]
+  err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+  def ptr(t):
+    return t.data_ptr() if t is not None else None
+
+  c = _lib.Conv(
+    in_=ptr(dev["x"]), in2=ptr(dev["x2"]), weight=ptr(dev["w"]), bias=ptr(dev["b"]), out=ptr(out), out_f32=ptr(out32), mask=ptr(dev["m"]),
+    error_word=ptr(err), nimg=nimg, height=h, width=w, c_in=c1, c_in2=c2, c_out=cout, relu=1, in2_full=1,
+  )
+  _lib.call("mjpbr_conv3x3_bf16", ctypes.byref(c), torch.cuda.current_stream().cuda_stream)
+  torch.cuda.synchronize()
+  assert int(err.item()) == 0
+  got32 = out32.view(nimg, h, w, cout)
+  # 9 (c1 + c2) products (exact in FP32) whose partial sums stay below 4, each addition rounding by 2^-24 of them
+  atol = 9 * (c1 + c2) * 2.0**-24 * 4.0
+  np.testing.assert_allclose(got32[pick].cpu().numpy(), ref, rtol=0, atol=atol)
+  assert torch.equal(out.view(nimg, h, w, cout), got32.to(torch.bfloat16))
+  assert bool((got32 >= 0).all())  # written everywhere
+
+
 def wgrad_ref(x, dy, x2=None):
   if x2 is not None:
     up = x2 if x2.shape[1] == x.shape[1] else np.repeat(np.repeat(x2, 2, axis=1), 2, axis=2)
