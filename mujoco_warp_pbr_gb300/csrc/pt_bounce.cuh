@@ -224,6 +224,14 @@ struct PtCore {
   }
 };
 
+// A path's denoiser features before its first surface.
+MJ_DEV void start_features(PathState& ps) {
+  ps.albedo = v3(1.0f);
+  ps.normal = v3(0.0f);
+  ps.emission = v3(0.0f);
+  ps.base_color = v3(0.0f);
+}
+
 // Sample `sample` of a pixel: sample 0 through the centre of the 15 x 15 sub-pixel grid, the others
 // at a jittered cell (pathtrace.py:362-378).
 MJ_DEV void start_sample(PathState& ps, const MjpbrScene& s, const Pixel& p, uint32_t seed, const M3& R, V3 cpos,
@@ -245,10 +253,7 @@ MJ_DEV void start_sample(PathState& ps, const MjpbrScene& s, const Pixel& p, uin
   ps.sample = sample;
   ps.camera_ray = true;
   ps.delta = true;
-  ps.albedo = v3(1.0f);
-  ps.normal = v3(0.0f);
-  ps.emission = v3(0.0f);
-  ps.base_color = v3(0.0f);
+  start_features(ps);
 }
 
 MJ_DEV void clear_pixel(PixelAcc& acc) {

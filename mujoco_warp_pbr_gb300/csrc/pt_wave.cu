@@ -49,39 +49,37 @@ constexpr int kThreads = 256;
 #define MJPBR_PTW_SHADE_CTAS 3
 #endif
 
-// A path between stages: 80 bytes every bounce reads and writes, then the first surface's denoiser
-// features (48 bytes), read and written only by the bounce that can set them (a camera ray's).
-struct __align__(16) PathRec {
-  float4 o;     // origin, max_dist
-  float4 d;     // direction, pdf_prev
-  float4 beta;  // throughput, dcam_z
-  float4 rad;   // radiance, first-hit depth (sample 0)
-  int4 meta;    // depth, passes, sample, flags (1 camera ray, 2 delta)
-  float4 f0;    // first surface: albedo xyz, normal x
-  float4 f1;    // normal yz, emission xy
-  float4 f2;    // emission z, base colour xyz
+// A path between stages: 80 bytes every bounce reads and writes, and the first surface's denoiser
+// features (48 bytes), written by the bounces of a camera ray. Each 16-byte field is an array of its own
+// over the paths of the chunk, so that a warp's lanes, on neighbouring paths, move whole lines.
+enum PathField : int32_t {
+  kPathOrigin,      // origin, max_dist
+  kPathDir,         // direction, pdf_prev
+  kPathBeta,        // throughput, dcam_z
+  kPathRadiance,    // radiance, first-hit depth (sample 0)
+  kPathMeta,        // (int bits) depth, passes, sample, flags (1 camera ray, 2 delta)
+  kPathFeature0,    // first surface: albedo xyz, normal x
+  kPathFeature1,    // normal yz, emission xy
+  kPathFeature2,    // emission z, base colour xyz
+  kPathFields
 };
 
-struct __align__(16) HitRec {
-  float dist;
-  int32_t ref;  // -1: miss; else slot | (mesh + 1) << 16
-  int32_t face;
-  float u, v;
-  float nx, ny, nz;
-};
+// A path's hit: two such fields (distance, ref, face, u; v, normal), ref -1 a miss, else
+// slot | (mesh + 1) << 16.
+constexpr int32_t kHitFields = 2;
 
-struct __align__(16) ShadowEntry {
-  float4 o;  // origin, ray length
-  float4 d;  // direction, target (int bits): path * nslot + slot
-};
+// A shadow ray: two fields over the queue (origin, ray length; direction, target (int bits)), the
+// target slot * path_cap + path.
+constexpr int32_t kShadowFields = 2;
 
-static_assert(sizeof(PathRec) == 128 && sizeof(HitRec) == 32 && sizeof(ShadowEntry) == 32, "record sizes");
-
-// next-event record flags of a slot
-constexpr int32_t kNeeSkip = 0;      // inactive light: nothing added
-constexpr int32_t kNeeZero = 1;      // the light does not reach the point: zero added
-constexpr int32_t kNeeAdd = 2;       // unshadowed contribution: added
-constexpr int32_t kNeeIfVisible = 3; // added if its shadow ray is unoccluded
+// Next-event state of a path's slot, a byte: what its term does to the radiance. kNeeActive is set in the
+// last slot (the environment's) while the path has terms to be added.
+constexpr uint8_t kNeeSkip = 0;      // inactive light: nothing added
+constexpr uint8_t kNeeZero = 1;      // the light does not reach the point: zero added
+constexpr uint8_t kNeeAdd = 2;       // unshadowed contribution: added
+constexpr uint8_t kNeePending = 3;   // added if its shadow ray is unoccluded: zero added
+constexpr uint8_t kNeeVisible = 4;   // kNeePending whose ray was unoccluded: added
+constexpr uint8_t kNeeActive = 0x80;
 
 struct PtWaveMap {
   int32_t w0, nw;          // worlds of this chunk
@@ -91,12 +89,12 @@ struct PtWaveMap {
   int32_t nslot;           // next-event slots: nlight, the headlight, the environment
   int32_t pix_base[MJPBR_MAX_RENDER];  // first RGB pixel of each camera within a world (-1: no RGB)
   int32_t geo_base[MJPBR_MAX_RENDER + 1];  // pixels of the cameras without RGB (prefix sums)
-  PathRec* path;
-  HitRec* hit;
-  float4* nee;             // (npath, 1 + nslot): the bounce's throughput, then each slot's term and flag
-  uint8_t* vis;            // (npath, nslot)
+  float4* path;            // (kPathFields, path_cap)
+  float4* hit;             // (kHitFields, path_cap)
+  float4* nee;             // (1 + nslot, path_cap): the bounce's throughput, then each slot's term
+  uint8_t* state;          // (nslot, path_cap)
   int32_t* queue[2];
-  ShadowEntry* shadow;
+  float4* shadow;          // (kShadowFields, shadow_cap)
   int32_t* counters;       // [0], [1] queue lengths, [2] shadow entries; 64-bit fetch counters of extend [4..5], shadow [6..7]
   int64_t path_cap, shadow_cap;
 };
@@ -131,29 +129,33 @@ MJ_DEV uint32_t pixel_seed_of(const MjpbrScene& s, uint32_t seed, int32_t w, con
   return seed + (uint32_t)w * (uint32_t)s.total_rays + (uint32_t)(s.ray_adr[p.cam] + p.pixelid);
 }
 
-MJ_DEV void store_path_hot(PathRec& r, const PathState& ps, float first_depth) {
-  r.o = make_float4(ps.o.x, ps.o.y, ps.o.z, ps.max_dist);
-  r.d = make_float4(ps.d.x, ps.d.y, ps.d.z, ps.pdf_prev);
-  r.beta = make_float4(ps.beta.x, ps.beta.y, ps.beta.z, ps.dcam_z);
-  r.rad = make_float4(ps.radiance.x, ps.radiance.y, ps.radiance.z, first_depth);
-  r.meta = make_int4(ps.depth, ps.passes, ps.sample, (ps.camera_ray ? 1 : 0) | (ps.delta ? 2 : 0));
+MJ_DEV float4& path_field(const PtWaveMap& wm, PathField f, int32_t path) { return wm.path[f * wm.path_cap + path]; }
+
+MJ_DEV void store_path_radiance(const PtWaveMap& wm, int32_t path, const PathState& ps, float first_depth) {
+  path_field(wm, kPathRadiance, path) = make_float4(ps.radiance.x, ps.radiance.y, ps.radiance.z, first_depth);
 }
 
-MJ_DEV void store_path_features(PathRec& r, const PathState& ps) {
-  r.f0 = make_float4(ps.albedo.x, ps.albedo.y, ps.albedo.z, ps.normal.x);
-  r.f1 = make_float4(ps.normal.y, ps.normal.z, ps.emission.x, ps.emission.y);
-  r.f2 = make_float4(ps.emission.z, ps.base_color.x, ps.base_color.y, ps.base_color.z);
+// What the next bounce needs besides the radiance.
+MJ_DEV void store_path_live(const PtWaveMap& wm, int32_t path, const PathState& ps) {
+  path_field(wm, kPathOrigin, path) = make_float4(ps.o.x, ps.o.y, ps.o.z, ps.max_dist);
+  path_field(wm, kPathDir, path) = make_float4(ps.d.x, ps.d.y, ps.d.z, ps.pdf_prev);
+  path_field(wm, kPathBeta, path) = make_float4(ps.beta.x, ps.beta.y, ps.beta.z, ps.dcam_z);
+  path_field(wm, kPathMeta, path) = make_float4(__int_as_float(ps.depth), __int_as_float(ps.passes), __int_as_float(ps.sample),
+                                                __int_as_float((ps.camera_ray ? 1 : 0) | (ps.delta ? 2 : 0)));
 }
 
-MJ_DEV void store_path(PathRec& r, const PathState& ps, float first_depth) {
-  store_path_hot(r, ps, first_depth);
-  store_path_features(r, ps);
+MJ_DEV void store_path_features(const PtWaveMap& wm, int32_t path, const PathState& ps) {
+  path_field(wm, kPathFeature0, path) = make_float4(ps.albedo.x, ps.albedo.y, ps.albedo.z, ps.normal.x);
+  path_field(wm, kPathFeature1, path) = make_float4(ps.normal.y, ps.normal.z, ps.emission.x, ps.emission.y);
+  path_field(wm, kPathFeature2, path) = make_float4(ps.emission.z, ps.base_color.x, ps.base_color.y, ps.base_color.z);
 }
 
-MJ_DEV PathState load_path_hot(const PathRec& r, float* first_depth) {
+// The state of a path before a bounce. Its features are start_sample's until the bounce that ends its
+// camera ray sets them, so none are loaded.
+MJ_DEV PathState load_path(const PtWaveMap& wm, int32_t path, float* first_depth) {
   PathState ps;
-  const float4 o = r.o, d = r.d, beta = r.beta, rad = r.rad;
-  const int4 meta = r.meta;
+  const float4 o = path_field(wm, kPathOrigin, path), d = path_field(wm, kPathDir, path), beta = path_field(wm, kPathBeta, path);
+  const float4 rad = path_field(wm, kPathRadiance, path), meta = path_field(wm, kPathMeta, path);
   ps.o = V3{o.x, o.y, o.z};
   ps.max_dist = o.w;
   ps.d = V3{d.x, d.y, d.z};
@@ -162,57 +164,41 @@ MJ_DEV PathState load_path_hot(const PathRec& r, float* first_depth) {
   ps.dcam_z = beta.w;
   ps.radiance = V3{rad.x, rad.y, rad.z};
   *first_depth = rad.w;
-  ps.depth = meta.x;
-  ps.passes = meta.y;
-  ps.sample = meta.z;
-  ps.camera_ray = (meta.w & 1) != 0;
-  ps.delta = (meta.w & 2) != 0;
+  ps.depth = __float_as_int(meta.x);
+  ps.passes = __float_as_int(meta.y);
+  ps.sample = __float_as_int(meta.z);
+  const int32_t flags = __float_as_int(meta.w);
+  ps.camera_ray = (flags & 1) != 0;
+  ps.delta = (flags & 2) != 0;
+  start_features(ps);
   return ps;
 }
 
-MJ_DEV void load_path_features(const PathRec& r, PathState& ps) {
-  const float4 f0 = r.f0, f1 = r.f1, f2 = r.f2;
-  ps.albedo = V3{f0.x, f0.y, f0.z};
-  ps.normal = V3{f0.w, f1.x, f1.y};
-  ps.emission = V3{f1.z, f1.w, f2.x};
-  ps.base_color = V3{f2.y, f2.z, f2.w};
+MJ_DEV void store_hit(const PtWaveMap& wm, int32_t path, const Hit& h) {
+  const int32_t ref = h.geom == -1 ? -1 : (h.slot | ((h.mesh + 1) << 16));
+  wm.hit[path] = make_float4(h.dist, __int_as_float(ref), __int_as_float(h.face), h.u);
+  wm.hit[wm.path_cap + path] = make_float4(h.v, h.normal.x, h.normal.y, h.normal.z);
 }
 
-MJ_DEV PathState load_path(const PathRec& r, float* first_depth) {
-  PathState ps = load_path_hot(r, first_depth);
-  load_path_features(r, ps);
-  return ps;
-}
-
-MJ_DEV HitRec pack_hit(const Hit& h) {
-  HitRec r;
-  r.dist = h.dist;
-  r.ref = h.geom == -1 ? -1 : (h.slot | ((h.mesh + 1) << 16));
-  r.face = h.face;
-  r.u = h.u;
-  r.v = h.v;
-  r.nx = h.normal.x;
-  r.ny = h.normal.y;
-  r.nz = h.normal.z;
-  return r;
-}
-
-MJ_DEV Hit unpack_hit(const HitRec& r, const float* blk, const BlockLayout& L) {
+MJ_DEV Hit load_hit(const PtWaveMap& wm, int32_t path, const float* blk, const BlockLayout& L) {
+  const float4 a = wm.hit[path];
+  const int32_t ref = __float_as_int(a.y);
   Hit h;
-  h.dist = r.dist;
-  if (r.ref == -1) {
+  h.dist = a.x;
+  if (ref == -1) {
     h.geom = h.slot = h.mesh = h.face = -1;
     h.u = h.v = 0.0f;
     h.normal = v3(0.0f);
     return h;
   }
-  h.slot = r.ref & 0xffff;
-  h.mesh = (r.ref >> 16) - 1;
+  const float4 b = wm.hit[wm.path_cap + path];
+  h.slot = ref & 0xffff;
+  h.mesh = (ref >> 16) - 1;
   h.geom = __float_as_int(blk[L.geom_off + h.slot * kGeomFloats + 16]);
-  h.face = r.face;
-  h.u = r.u;
-  h.v = r.v;
-  h.normal = V3{r.nx, r.ny, r.nz};
+  h.face = __float_as_int(a.z);
+  h.u = a.w;
+  h.v = b.x;
+  h.normal = V3{b.y, b.z, b.w};
   return h;
 }
 
@@ -251,15 +237,14 @@ MJ_DEV int64_t cta_append(bool want, int32_t* counter, int64_t cap, int32_t* sca
 // its shadow ray appended to the shadow queue at once (one atomic per group of converged lanes);
 // the shadow stage traces the rays and the next extend (or resolve) adds the terms.
 struct RecordedNee {
-  float4* rec;  // [0] beta, active; [1 + k] slot k's contribution, flag
-  int32_t nslot, path;
+  int32_t path;
   V3 origin;
   const PtWaveMap* wm;
   int32_t* err;
-  MJ_DEV void begin(const PathState& ps, V3 o) {
-    rec[0] = make_float4(ps.beta.x, ps.beta.y, ps.beta.z, __int_as_float(0));
+  MJ_DEV uint8_t& state(int32_t slot) const { return wm->state[slot * wm->path_cap + path]; }
+  MJ_DEV void begin(const PathState&, V3 o) {
     origin = o;
-    for (int32_t k = 0; k < nslot; ++k) rec[1 + k].w = __int_as_float(kNeeSkip);
+    for (int32_t k = 0; k < wm->nslot - 1; ++k) state(k) = kNeeSkip;
   }
   MJ_DEV void shadow_ray(int32_t slot, V3 dir, float len) {
     cg::coalesced_group g = cg::coalesced_threads();
@@ -270,24 +255,27 @@ struct RecordedNee {
       *err |= kErrWorkQueue;
       return;
     }
-    ShadowEntry e;
-    e.o = make_float4(origin.x, origin.y, origin.z, len);
-    e.d = make_float4(dir.x, dir.y, dir.z, __int_as_float(path * nslot + slot));
-    wm->shadow[pos] = e;
+    wm->shadow[pos] = make_float4(origin.x, origin.y, origin.z, len);
+    wm->shadow[wm->shadow_cap + pos] = make_float4(dir.x, dir.y, dir.z, __int_as_float((int32_t)(slot * wm->path_cap + path)));
   }
-  MJ_DEV void none(int32_t slot) { rec[1 + slot].w = __int_as_float(kNeeZero); }
+  MJ_DEV void none(int32_t slot) { state(slot) = kNeeZero; }
   template <class F>
   MJ_DEV void light(RtCtx&, int32_t slot, bool shadowed, V3, V3 dir, float max_t, F contribution) {
     const V3 c = contribution();
-    rec[1 + slot] = make_float4(c.x, c.y, c.z, __int_as_float(shadowed ? kNeeIfVisible : kNeeAdd));
+    wm->nee[(1 + slot) * wm->path_cap + path] = make_float4(c.x, c.y, c.z, 0.0f);
+    state(slot) = shadowed ? kNeePending : kNeeAdd;
     if (shadowed) shadow_ray(slot, dir, max_t);
   }
-  MJ_DEV void lights_done(PathState&) { rec[0].w = __int_as_float(1); }
+  MJ_DEV void lights_done(PathState& ps) {
+    wm->nee[path] = make_float4(ps.beta.x, ps.beta.y, ps.beta.z, 0.0f);
+    state(wm->nslot - 1) = kNeeActive;
+  }
   template <class F>
   MJ_DEV void env(RtCtx&, PathState&, V3, V3 dir, F term) {
-    const int32_t slot = nslot - 1;
+    const int32_t slot = wm->nslot - 1;
     const V3 t = term();
-    rec[1 + slot] = make_float4(t.x, t.y, t.z, __int_as_float(kNeeIfVisible));
+    wm->nee[(1 + slot) * wm->path_cap + path] = make_float4(t.x, t.y, t.z, 0.0f);
+    state(slot) = kNeeActive | kNeePending;
     shadow_ray(slot, dir, kUnboundedShadow);
   }
 };
@@ -297,27 +285,35 @@ struct RecordedNee {
 // terms in light order, times the bounce's throughput, then the environment term), each one only
 // if its shadow ray was unoccluded, and marks the record applied. Run by the next bounce's extend
 // stage before the path's next hit, and by the resolve stage for the paths that ended: the same
-// additions in the same order as the persistent kernel.
-MJ_DEV void apply_nee(const PtWaveMap& wm, int32_t path, PathRec& r) {
-  float4* rec = wm.nee + (int64_t)path * (1 + wm.nslot);
-  const float4 head = rec[0];
-  if (__float_as_int(head.w) == 0) return;
+// additions in the same order as the persistent kernel. Returns the path's radiance field.
+MJ_DEV float4 apply_nee(const PtWaveMap& wm, int32_t path) {
+  float4 rad = path_field(wm, kPathRadiance, path);
   const int32_t nlights = wm.nslot - 1;  // the model's lights and the headlight
-  const uint8_t* vis = wm.vis + (int64_t)path * wm.nslot;
+  uint8_t& env = wm.state[nlights * wm.path_cap + path];
+  const uint8_t env_state = env;
+  if (!(env_state & kNeeActive)) return rad;
   V3 direct = v3(0.0f);
   for (int32_t k = 0; k < nlights; ++k) {
-    const float4 c = rec[1 + k];
-    const int32_t flag = __float_as_int(c.w);
-    if (flag == kNeeSkip) continue;
-    const bool add = flag == kNeeAdd || (flag == kNeeIfVisible && vis[k]);
-    direct += add ? V3{c.x, c.y, c.z} : v3(0.0f);
+    const uint8_t st = wm.state[k * wm.path_cap + path];
+    if (st == kNeeSkip) continue;
+    V3 c = v3(0.0f);
+    if (st == kNeeAdd || st == kNeeVisible) {
+      const float4 t = wm.nee[(1 + k) * wm.path_cap + path];
+      c = V3{t.x, t.y, t.z};
+    }
+    direct += c;
   }
-  V3 radiance{r.rad.x, r.rad.y, r.rad.z};
+  const float4 head = wm.nee[path];
+  V3 radiance{rad.x, rad.y, rad.z};
   radiance += cmul(V3{head.x, head.y, head.z}, direct);
-  const float4 e = rec[1 + nlights];
-  if (__float_as_int(e.w) == kNeeIfVisible && vis[nlights]) radiance += V3{e.x, e.y, e.z};
-  r.rad = make_float4(radiance.x, radiance.y, radiance.z, r.rad.w);
-  rec[0].w = __int_as_float(0);
+  if ((env_state & ~kNeeActive) == kNeeVisible) {
+    const float4 e = wm.nee[(1 + nlights) * wm.path_cap + path];
+    radiance += V3{e.x, e.y, e.z};
+  }
+  rad = make_float4(radiance.x, radiance.y, radiance.z, rad.w);
+  path_field(wm, kPathRadiance, path) = rad;
+  env = 0;
+  return rad;
 }
 
 // ---------------------------------------------------------------- cameras without RGB
@@ -426,28 +422,15 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_extend_kernel(const __grid_co
   int32_t path = -1;
   auto start = [&](int64_t item, float* max_dist) {
     path = wm.queue[cur][item];
-    PathRec& r = wm.path[path];
-    if (pending_nee) apply_nee(wm, path, r);
-    const float4 o = r.o, d = r.d;
+    if (pending_nee) apply_nee(wm, path);
+    const float4 o = path_field(wm, kPathOrigin, path), d = path_field(wm, kPathDir, path);
     blk = world_block(s, wm.w0 + (path / wm.nsample) / wm.pixels);
     *max_dist = o.w;
     return Ray{V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}};
   };
   auto finish = [&](const Hit& hit) {
-    wm.hit[path] = pack_hit(hit);
-    PathRec& r = wm.path[path];
-    const int4 meta = r.meta;
-    const int32_t sample = meta.z;
-    const int32_t passes = meta.y;
-    const bool camera_ray = (meta.w & 1) != 0;
-    if (camera_ray && passes == 0 && sample == 0) {
-      int32_t ww, smp;
-      Pixel p;
-      path_pixel(s, wm, path, &ww, &p, &smp);
-      const float dcam_z = r.beta.w;
-      write_geometry(s, ww, p, hit, dcam_z);
-      if (hit.geom != -1) r.rad.w = hit.dist * -dcam_z;
-    }
+    // the first hits, and the geometry they write, are ptw_first_extend_kernel's
+    store_hit(wm, path, hit);
   };
   closest_queue<kMesh, kScan>(s, st, L, cull, items, fetched, blk, start, finish, &err);
   if (err && s.error_word) atomicOr(s.error_word, err);
@@ -488,7 +471,7 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __g
     return Ray{ps.o, ps.d};
   };
   auto finish = [&](const Hit& hit) {
-    wm.hit[path] = pack_hit(hit);
+    store_hit(wm, path, hit);
     PathState ps;
     Pixel p;
     int32_t w, sample;
@@ -498,7 +481,8 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __g
       write_geometry(s, w, p, hit, ps.dcam_z);
       if (hit.geom != -1) first_depth = hit.dist * -ps.dcam_z;
     }
-    store_path(wm.path[path], ps, first_depth);
+    store_path_radiance(wm, path, ps, first_depth);
+    store_path_live(wm, path, ps);
   };
   closest_queue<kMesh, kScan>(s, st, L, cull, wm.npath, fetched, blk, start, finish, &err);
   if (err && s.error_word) atomicOr(s.error_word, err);
@@ -530,19 +514,17 @@ __global__ void __launch_bounds__(kThreads, MJPBR_PTW_SHADE_CTAS) ptw_shade_kern
       p.rec = blk + L.cam_off + p.cam * kCamFloats;
       const M3 R = cam_mat(p.rec);
       const V3 head_dir = -V3{R.m[2], R.m[5], R.m[8]};
-      PathRec& r = wm.path[path];
       float first_depth;
-      PathState ps = load_path_hot(r, &first_depth);
+      PathState ps = load_path(wm, path, &first_depth);
       // only a camera ray's bounce can set the first surface's features
       const bool features = ps.camera_ray;
-      if (features) load_path_features(r, ps);
-      const Hit hit = unpack_hit(wm.hit[path], blk, L);
-      float4* rec = wm.nee + (int64_t)path * (1 + wm.nslot);
-      rec[0].w = __int_as_float(0);
-      RecordedNee nee{rec, wm.nslot, path, v3(0.0f), &wm, &err};
+      const Hit hit = load_hit(wm, path, blk, L);
+      RecordedNee nee{path, v3(0.0f), &wm, &err};
+      nee.state(wm.nslot - 1) = 0;
       live = !PtCore<kMesh, kTex>::surface(c, nee, ps, hit, pixel_seed_of(s, seed, w, p), head_dir);
-      store_path_hot(r, ps, first_depth);
-      if (features) store_path_features(r, ps);
+      store_path_radiance(wm, path, ps, first_depth);
+      if (live) store_path_live(wm, path, ps);
+      if (features) store_path_features(wm, path, ps);
       err |= c.err;
     }
     // the paths that continue
@@ -567,19 +549,20 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_shadow_kernel(const __grid_co
   const float* blk = nullptr;
   int32_t target = -1;
   auto start = [&](int64_t item, float* max_dist) {
-    const ShadowEntry e = wm.shadow[item];
-    target = __float_as_int(e.d.w);
-    const int32_t path = target / wm.nslot;
+    const float4 o = wm.shadow[item], d = wm.shadow[wm.shadow_cap + item];
+    target = __float_as_int(d.w);
+    const int32_t path = target % (int32_t)wm.path_cap;
     blk = world_block(s, wm.w0 + (path / wm.nsample) / wm.pixels);
-    *max_dist = e.o.w;
-    return Ray{V3{e.o.x, e.o.y, e.o.z}, V3{e.d.x, e.d.y, e.d.z}};
+    *max_dist = o.w;
+    return Ray{V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}};
   };
+  auto visible = [&] { wm.state[target] += kNeeVisible - kNeePending; };  // the environment's keeps kNeeActive
   float max_dist;
   if constexpr (kScan && !kMesh) {
     uint32_t meshes;
     for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < items; i += (int64_t)gridDim.x * kThreads) {
       const Ray r = start(i, &max_dist);
-      wm.vis[target] = scan_any<false>(blk, L, r, max_dist, cull, &meshes) ? 0 : 1;
+      if (!scan_any<false>(blk, L, r, max_dist, cull, &meshes)) visible();
     }
   } else if constexpr (kScan) {
     const Stack st = wave_stack(s, smem);
@@ -591,11 +574,14 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_shadow_kernel(const __grid_co
           qq.sp = 0;
           const bool hit = scan_any<true>(blk, L, qq.r, qq.cut, cull, &qq.meshes);
           if (!hit && qq.meshes) return true;
-          wm.vis[target] = hit ? 0 : 1;
+          if (!hit) visible();
           return false;
         },
         [&](MeshWalk& qq) { return walk_any_step(qq, s, st, blk, L, &err); },
-        [&](MeshWalk&, int32_t res) { wm.vis[target] = res == kAnyClear ? 1 : 0; }, &err);
+        [&](MeshWalk&, int32_t res) {
+          if (res == kAnyClear) visible();
+        },
+        &err);
   } else {
     const Stack st = wave_stack(s, smem);
     AnyQuery q;
@@ -607,7 +593,10 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_shadow_kernel(const __grid_co
           return true;
         },
         [&](AnyQuery& qq) { return any_step<kMesh>(qq, s, st, blk, L, cull, &err); },
-        [&](AnyQuery&, int32_t res) { wm.vis[target] = res == kAnyClear ? 1 : 0; }, &err);
+        [&](AnyQuery&, int32_t res) {
+          if (res == kAnyClear) visible();
+        },
+        &err);
   }
   if (err && s.error_word) atomicOr(s.error_word, err);
 }
@@ -626,11 +615,17 @@ __global__ void __launch_bounds__(kThreads) ptw_resolve_kernel(const __grid_cons
   PixelAcc acc;
   clear_pixel(acc);
   for (int32_t k = 0; k < wm.nsample; ++k) {
-    float first_depth;
     const int32_t path = pix_all * wm.nsample + k;
-    apply_nee(wm, path, wm.path[path]);
-    const PathState ps = load_path(wm.path[path], &first_depth);
-    if (k == 0) acc.first_depth = first_depth;
+    const float4 rad = apply_nee(wm, path);
+    const float4 f0 = path_field(wm, kPathFeature0, path), f1 = path_field(wm, kPathFeature1, path), f2 = path_field(wm, kPathFeature2, path);
+    PathState ps;
+    ps.radiance = V3{rad.x, rad.y, rad.z};
+    ps.sample = k;
+    ps.albedo = V3{f0.x, f0.y, f0.z};
+    ps.normal = V3{f0.w, f1.x, f1.y};
+    ps.emission = V3{f1.z, f1.w, f2.x};
+    ps.base_color = V3{f2.y, f2.z, f2.w};
+    if (k == 0) acc.first_depth = rad.w;
     add_sample(acc, ps, s.settings.denoise != 0, c.exposure);
   }
   write_pixel(s, c, (int64_t)w * s.rgb_stride + s.rgb_adr[p.cam] + p.pixelid, acc, wm.nsample);
@@ -664,22 +659,22 @@ int64_t layout(PtWaveMap* wm, char* base, int64_t npath, int32_t nslot) {
     return p;
   };
   char* counters = take(256);
-  char* path = take(npath * (int64_t)sizeof(PathRec));
-  char* hit = take(npath * (int64_t)sizeof(HitRec));
+  char* path = take(npath * kPathFields * 16);
+  char* hit = take(npath * kHitFields * 16);
   char* nee = take(npath * (1 + (int64_t)nslot) * 16);
-  char* vis = take(npath * nslot);
+  char* state = take(npath * nslot);
   char* q0 = take(npath * 4);
   char* q1 = take(npath * 4);
-  char* shadow = take(npath * nslot * (int64_t)sizeof(ShadowEntry));
+  char* shadow = take(npath * nslot * kShadowFields * 16);
   if (wm) {
     wm->counters = reinterpret_cast<int32_t*>(counters);
-    wm->path = reinterpret_cast<PathRec*>(path);
-    wm->hit = reinterpret_cast<HitRec*>(hit);
+    wm->path = reinterpret_cast<float4*>(path);
+    wm->hit = reinterpret_cast<float4*>(hit);
     wm->nee = reinterpret_cast<float4*>(nee);
-    wm->vis = reinterpret_cast<uint8_t*>(vis);
+    wm->state = reinterpret_cast<uint8_t*>(state);
     wm->queue[0] = reinterpret_cast<int32_t*>(q0);
     wm->queue[1] = reinterpret_cast<int32_t*>(q1);
-    wm->shadow = reinterpret_cast<ShadowEntry*>(shadow);
+    wm->shadow = reinterpret_cast<float4*>(shadow);
     wm->path_cap = npath;
     wm->shadow_cap = npath * nslot;
   }
