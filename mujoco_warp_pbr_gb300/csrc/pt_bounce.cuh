@@ -15,6 +15,11 @@
 #include "kernel_common.cuh"
 #include "pt_sampling.cuh"
 
+// The parts of a bounce the persistent kernel keeps out of line (see MJPBR_PT_CALL, pt_sampling.cuh).
+#ifndef MJPBR_LIGHT_QUERY
+#define MJPBR_LIGHT_QUERY __noinline__
+#endif
+
 namespace mjpbr {
 
 struct PathState {
@@ -67,7 +72,7 @@ struct PtCore {
   // One punctual light (its bulb disc jittered by u0, u1 for soft shadows) seen from the point:
   // false when it does not reach it (behind the surface, outside its cone or range).
   // out of line: one copy of the light-sampling code in the bounce loop (1 % faster measured)
-  static __device__ __noinline__ bool light_query(RtCtx& c, Light light, V3 point, V3 normal, V3 t1, V3 t2, float u0, float u1,
+  static __device__ MJPBR_LIGHT_QUERY bool light_query(RtCtx& c, Light light, V3 point, V3 normal, V3 t1, V3 t2, float u0, float u1,
                                                   LightQuery* q) {
     const MjpbrSettings& st = c.s->settings;
     if (light.type != MJPBR_LIGHT_DIRECTIONAL && light.bulbradius > 0.0f) {
@@ -90,8 +95,8 @@ struct PtCore {
 
   // The unshadowed next-event estimate of a light that reaches the point.
   static MJ_DEV V3 light_contribution(const Lobes& lb, V3 v, const LightQuery& q) {
-    V3 diffuse = eval_bsdf_cos(lb.diffuse_color, v3(0.0f), lb.alpha, v3(0.0f), v, q.ll);
-    V3 specular = eval_bsdf_cos(v3(0.0f), lb.f0, lb.alpha, lb.energy_comp, v, q.ll);
+    V3 diffuse, specular;
+    eval_bsdf_lobes(lb.diffuse_color, lb.f0, lb.alpha, lb.energy_comp, v, q.ll, &diffuse, &specular);
     return cmul(diffuse, q.ds) + cmul(specular, q.ss);
   }
 

@@ -96,6 +96,33 @@ MJPBR_PT_CALL V3 eval_bsdf_cos(V3 diffuse_color, V3 f0, float alpha, V3 energy_c
   return (diffuse_color * (1.0f / kPi) + spec) * nol;
 }
 
+// eval_bsdf_cos of the diffuse lobe alone (f0 and energy_comp zero) and of the specular lobe alone
+// (diffuse_color zero), which share everything but the last products: the same values.
+MJPBR_PT_CALL void eval_bsdf_lobes(V3 diffuse_color, V3 f0, float alpha, V3 energy_comp, V3 v, V3 l, V3* diffuse, V3* specular) {
+  float nol = l.z;
+  float nov = fmaxf(v.z, 1.0e-4f);
+  if (nol <= 0.0f) {
+    *diffuse = *specular = v3(0.0f);
+    return;
+  }
+  V3 h = normalize(l + v);
+  float noh = fmaxf(h.z, 0.0f), loh = fmaxf(dot(l, h), 0.0f);
+  float a2 = alpha * alpha;
+  float fd = (noh * a2 - noh) * noh + 1.0f;
+  float D = a2 / (kPi * fd * fd);
+  float gv = nol * sqrtf(nov * nov * (1.0f - a2) + a2);
+  float gl = nov * sqrtf(nol * nol * (1.0f - a2) + a2);
+  float Vis = 0.5f / (gv + gl);
+  float x = 1.0f - loh;
+  float x2 = x * x;
+  float fc = x2 * x2 * x;
+  const float dv = D * Vis;
+  const float none = fc * dv * 0.0f;  // the diffuse lobe's specular term: zero, or NaN where D is not finite
+  *diffuse = (diffuse_color * (1.0f / kPi) + v3(none)) * nol;
+  V3 F = f0 * (1.0f - fc) + v3(fc);
+  *specular = cmul(F * dv, energy_comp) * nol;
+}
+
 // Solid-angle pdf of sample_bsdf: mixture of GGX VNDF and cosine-weighted hemisphere.
 MJPBR_PT_CALL float pdf_bsdf(float alpha, float p_spec, V3 v, V3 l) {
   if (l.z <= 0.0f) return 0.0f;

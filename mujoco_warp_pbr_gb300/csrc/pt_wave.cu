@@ -34,6 +34,13 @@
 #include "abi_internal.h"
 #include <cooperative_groups.h>
 
+// The shade stage is the only kernel here that calls these, each from few places: inline, so that lights,
+// hits and surfaces pass through registers.
+#define MJPBR_PT_INLINE
+#define MJPBR_LIGHT_QUERY __forceinline__
+#ifndef MJPBR_SURFACE_CALL
+#define MJPBR_SURFACE_CALL __forceinline__
+#endif
 #include "pt_bounce.cuh"
 #include "refill.cuh"
 #include "scan.cuh"
@@ -47,6 +54,9 @@ constexpr int kThreads = 256;
 // Resident CTAs per SM the shade stage's register allocation targets.
 #ifndef MJPBR_PTW_SHADE_CTAS
 #define MJPBR_PTW_SHADE_CTAS 3
+#endif
+#ifndef MJPBR_PTW_TEX_CTAS
+#define MJPBR_PTW_TEX_CTAS 2
 #endif
 
 // A path between stages: 80 bytes every bounce reads and writes, and the first surface's denoiser
@@ -490,7 +500,7 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __g
 
 // ---------------------------------------------------------------- shade
 template <bool kMesh, bool kTex>
-__global__ void __launch_bounds__(kThreads, MJPBR_PTW_SHADE_CTAS) ptw_shade_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
+__global__ void __launch_bounds__(kThreads, kTex ? MJPBR_PTW_TEX_CTAS : MJPBR_PTW_SHADE_CTAS) ptw_shade_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
                                                                 const __grid_constant__ PtWaveMap wm, int32_t cur) {
   __shared__ int32_t scan[kThreads / 32 + 1];
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);

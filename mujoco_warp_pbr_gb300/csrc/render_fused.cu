@@ -18,6 +18,8 @@
 #include <type_traits>
 
 #include "abi_internal.h"
+// one call in each kernel
+#define MJPBR_SURFACE_CALL __forceinline__
 #include "rt_shade.cuh"
 #include "scan.cuh"
 

@@ -36,6 +36,8 @@
 
 #include "abi_internal.h"
 #include "refill.cuh"
+// one call in each kernel
+#define MJPBR_SURFACE_CALL __forceinline__
 #include "rt_shade.cuh"
 #include "scan.cuh"
 

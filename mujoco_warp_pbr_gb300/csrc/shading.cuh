@@ -242,10 +242,15 @@ MJ_DEV float4 fetch_texel(const MjpbrTexture& t, const uint8_t* data, int level,
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
+// i modulo n (n > 0): a mask for the usual power-of-two sizes, where the general remainder is some
+// thirty instructions, several times per lookup.
 MJ_DEV int wrap_index(int i, int n) {
+  if ((n & (n - 1)) == 0) return i & (n - 1);
   int r = i % n;
   return r < 0 ? r + n : r;
 }
+// The index after a wrapped one.
+MJ_DEV int wrap_next(int i, int n) { return i + 1 == n ? 0 : i + 1; }
 
 MJ_DEV float4 lerp4(float4 a, float4 b, float t) {
   return make_float4(a.x + (b.x - a.x) * t, a.y + (b.y - a.y) * t, a.z + (b.z - a.z) * t, a.w + (b.w - a.w) * t);
@@ -261,14 +266,14 @@ MJ_DEV float4 sample_level(const MjpbrTexture& t, const uint8_t* data, int level
   int x0 = (int)x0f, y0 = (int)y0f, x1 = x0 + 1, y1 = y0 + 1;
   if (wrap_u) {
     x0 = wrap_index(x0, w);
-    x1 = wrap_index(x1, w);
+    x1 = wrap_next(x0, w);
   } else {
     x0 = min(max(x0, 0), w - 1);
     x1 = min(max(x1, 0), w - 1);
   }
   if (wrap_v) {
     y0 = wrap_index(y0, h);
-    y1 = wrap_index(y1, h);
+    y1 = wrap_next(y0, h);
   } else {
     y0 = min(max(y0, 0), h - 1);
     y1 = min(max(y1, 0), h - 1);
@@ -359,7 +364,7 @@ static __device__ __noinline__ V3 sample_prefiltered(const uint16_t* stack, int 
   float fx = u * (float)w - 0.5f, fy = v * (float)h - 0.5f;
   float x0f = floorf(fx), y0f = floorf(fy);
   float tx = fx - x0f, ty = fy - y0f;
-  int x0 = wrap_index((int)x0f, w), x1 = wrap_index((int)x0f + 1, w);
+  int x0 = wrap_index((int)x0f, w), x1 = wrap_next(x0, w);
   int y0 = min(max((int)y0f, 0), h - 1), y1 = min(max((int)y0f + 1, 0), h - 1);
   float4 r0 = lerp4(lerp4(stack_texel(stack, w, h, z0, x0, y0), stack_texel(stack, w, h, z0, x1, y0), tx),
                     lerp4(stack_texel(stack, w, h, z0, x0, y1), stack_texel(stack, w, h, z0, x1, y1), tx), ty);

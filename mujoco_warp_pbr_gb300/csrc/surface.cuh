@@ -10,6 +10,12 @@
 #include "shading.cuh"
 #include "trace.cuh"
 
+// Out of line in kernels that evaluate surfaces in several places; a kernel with one place defines this
+// as __forceinline__ (the hit and the surface then pass through registers, not local memory).
+#ifndef MJPBR_SURFACE_CALL
+#define MJPBR_SURFACE_CALL __noinline__
+#endif
+
 namespace mjpbr {
 
 constexpr float kSpecularAaVariance = 0.15f;
@@ -163,7 +169,7 @@ MJ_DEV float4 fetch_role(const MjpbrScene& s, int32_t tex_id, const TexFrame& f,
 
 // Surface and viewer-facing shading normal (world frame) at a hit (material.py:301-503).
 template <bool kMesh, bool kTex>
-__device__ __noinline__ Surface eval_surface(const MjpbrScene& s, const float* blk, const BlockLayout& L, int32_t w, const Hit& hit,
+__device__ MJPBR_SURFACE_CALL Surface eval_surface(const MjpbrScene& s, const float* blk, const BlockLayout& L, int32_t w, const Hit& hit,
                             int32_t slot, V3 point, V3 dir, float footprint, V3* shading_world) {
   Surface sf;
   sf.occlusion = 1.0f;
