@@ -34,6 +34,8 @@
 #include <type_traits>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "abi_internal.h"
 #include "refill.cuh"
 // one call in each kernel
@@ -43,6 +45,8 @@
 
 namespace mjpbr {
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr int kThreads = 256;
 constexpr int kTile = 16;  // pixel tiles of 16 x 16, addressed in Z order within the tile
@@ -76,7 +80,9 @@ struct __align__(16) SurfRec {
 struct __align__(16) MirrorEntry {
   float4 o;    // origin, cone footprint at the reflecting surface
   float4 d;    // direction, pixel spread
-  int4 index;  // x: sample
+  // x: sample. The other words serve the whole queue: y of entry i is the i-th entry whose meshes are still
+  // to be traced and z the mask of this entry's; w of entry i is the i-th entry that hit a surface.
+  int4 index;
 };
 
 struct __align__(16) ShadowEntry {
@@ -102,7 +108,8 @@ struct WaveMap {
   int32_t* vis;          // (sample, segment, light) unoccluded shadow rays
   MirrorEntry* mirror;
   ShadowEntry* shadow;
-  int32_t* counters;     // [0] mirror entries, [1] shadow entries; 64-bit fetch counters of the shadow [2..3] and mirror [4..5] stages
+  int32_t* counters;     // [0] mirror entries, [1] shadow entries; 64-bit fetch counters of the shadow [2..3] and mirror [4..5] stages;
+                         // [6] mirror entries with meshes to trace, [7] mirror entries that hit
   int64_t mirror_cap, shadow_cap;
 };
 
@@ -395,6 +402,24 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_SHADE_CTAS) wave_surface_
 #define MJPBR_SCAN_MIN_IDLE 8
 #endif
 
+// Result of mirror entry i: a miss is final (the resolve stage reads nothing else of it); a hit is listed
+// for the surface stage at list position pos (< 0: by one atomic per group of converged lanes), so that
+// its lanes all have a surface to evaluate.
+MJ_DEV void finish_mirror(const WaveMap& wm, int32_t i, int32_t sample, const Hit& h, int64_t pos) {
+  if (h.geom == -1) {
+    wm.surf[1][sample].c = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
+    return;
+  }
+  wm.hit[1][sample] = pack_hit(h);
+  if (pos < 0) {
+    cg::coalesced_group g = cg::coalesced_threads();
+    int32_t base = 0;
+    if (g.thread_rank() == 0) base = atomicAdd(wm.counters + 7, (int32_t)g.size());
+    pos = g.shfl(base, 0) + g.thread_rank();
+  }
+  wm.mirror[pos].index.w = i;
+}
+
 // Closest hit of every queued mirror ray, lanes refilled from the queue (refill.cuh).
 template <bool kMesh>
 __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_kernel(const __grid_constant__ MjpbrScene s,
@@ -407,53 +432,107 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_
   int32_t err = 0;
   ClosestQuery q;
   const float* blk = nullptr;
-  int32_t sample = -1;
+  int32_t sample = -1, entry = -1;
   refill_loop<MJPBR_WAVE_REFILL_STEPS>(
       items, reinterpret_cast<unsigned long long*>(wm.counters + 4), q,
       [&](int64_t item, ClosestQuery& qq) {
-        const MirrorEntry e = wm.mirror[item];
+        const MirrorEntry& e = wm.mirror[item];
+        const float4 o = e.o, d = e.d;
+        entry = (int32_t)item;
         sample = e.index.x;
         blk = s.world_blocks + (int64_t)(wm.w0 + sample / wm.per_world) * s.world_block_floats;
-        closest_begin(qq, st, Ray{V3{e.o.x, e.o.y, e.o.z}, V3{e.d.x, e.d.y, e.d.z}}, kMaxVal, &err);
+        closest_begin(qq, st, Ray{V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}}, kMaxVal, &err);
         return true;
       },
       [&](ClosestQuery& qq) { return closest_step<kMesh>(qq, s, st, blk, L, cull, &err); },
-      [&](ClosestQuery& qq, int32_t) { wm.hit[1][sample] = pack_hit(qq.h); }, &err);
+      [&](ClosestQuery& qq, int32_t) { finish_mirror(wm, entry, sample, qq.h, -1); }, &err);
   if (err && s.error_word) atomicOr(s.error_word, err);
 }
 
-// The mirror stage of scanned scenes (scan.cuh): the primitives when a ray is fetched, its meshes
-// resumably.
+// The mirror stage of scanned scenes (scan.cuh) in two kernels: the primitives of every entry, lanes
+// full; then the meshes of the entries whose ray passes some mesh's box, resumably, lanes refilled.
 __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_scan_kernel(const __grid_constant__ MjpbrScene s,
+                                                                                            const __grid_constant__ WaveMap wm) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ int32_t scan[kThreads / 32 + 1];
+  const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
+  const Stack st = wave_stack(s, smem);
+  const bool cull = s.settings.cull_backfaces != 0;
+  const int32_t count = (int32_t)min((int64_t)wm.counters[0], wm.mirror_cap);
+  int32_t err = 0;
+  const int32_t stride = gridDim.x * kThreads;
+  const int32_t rounds = (count + stride - 1) / stride;
+  for (int32_t round = 0; round < rounds; ++round) {
+    const int32_t i = round * stride + blockIdx.x * kThreads + threadIdx.x;
+    Hit h;
+    uint32_t meshes = 0;
+    int32_t sample = -1;
+    h.geom = -1;
+    if (i < count) {
+      const float4 o = wm.mirror[i].o, d = wm.mirror[i].d;
+      sample = wm.mirror[i].index.x;
+      const float* blk = s.world_blocks + (int64_t)(wm.w0 + sample / wm.per_world) * s.world_block_floats;
+      const Ray r{V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}};
+      bool tie;
+      meshes = scan_closest<true>(h, tie, NodeBoxes{blk, &L}, blk, L, r, kMaxVal, cull);
+      if (meshes) {
+        h.face = tie ? -2 : -1;  // no primitive's hit has a face: carries the mark
+        wm.hit[1][sample] = pack_hit(h);
+        wm.mirror[i].index.z = (int32_t)meshes;
+      } else if (tie) {
+        h = trace_ray<true>(s, st, blk, L, r, kMaxVal, cull, false, &err);
+      }
+    }
+    const int64_t pos = cta_append(meshes != 0, wm.counters + 6, wm.mirror_cap, scan, &err);
+    if (pos >= 0) wm.mirror[pos].index.y = i;
+    const bool hit = i < count && !meshes && h.geom != -1;
+    const int64_t at = cta_append(hit, wm.counters + 7, wm.mirror_cap, scan, &err);
+    if (i < count && !meshes) finish_mirror(wm, i, sample, h, at);
+  }
+  if (err && s.error_word) atomicOr(s.error_word, err);
+}
+
+__global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_mesh_kernel(const __grid_constant__ MjpbrScene s,
                                                                                             const __grid_constant__ WaveMap wm) {
   extern __shared__ __align__(16) float smem[];
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
   const Stack st = wave_stack(s, smem);
   const bool cull = s.settings.cull_backfaces != 0;
-  const int64_t items = min((int64_t)wm.counters[0], wm.mirror_cap);
+  const int64_t items = min((int64_t)wm.counters[6], wm.mirror_cap);
   int32_t err = 0;
   ClosestWalk q;
   const float* blk = nullptr;
-  int32_t sample = -1;
-  auto done = [&](ClosestWalk& qq) {
-    if (qq.tie) qq.h = trace_ray<true>(s, st, blk, L, qq.m.r, kMaxVal, cull, false, &err);
-    wm.hit[1][sample] = pack_hit(qq.h);
-  };
-  refill_loop<MJPBR_WAVE_REFILL_STEPS, MJPBR_SCAN_MIN_IDLE>(
+  int32_t sample = -1, entry = -1;
+  refill_loop<MJPBR_WAVE_REFILL_STEPS>(
       items, reinterpret_cast<unsigned long long*>(wm.counters + 4), q,
       [&](int64_t item, ClosestWalk& qq) {
-        const MirrorEntry e = wm.mirror[item];
-        sample = e.index.x;
+        entry = wm.mirror[item].index.y;
+        const float4 o = wm.mirror[entry].o, d = wm.mirror[entry].d;
+        sample = wm.mirror[entry].index.x;
         blk = s.world_blocks + (int64_t)(wm.w0 + sample / wm.per_world) * s.world_block_floats;
-        qq.m.r = Ray{V3{e.o.x, e.o.y, e.o.z}, V3{e.d.x, e.d.y, e.d.z}};
-        qq.m.meshes = scan_closest<true>(qq.h, qq.tie, NodeBoxes{blk, &L}, blk, L, qq.m.r, kMaxVal, cull);
+        qq.m.r = Ray{V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}};
+        qq.m.meshes = (uint32_t)wm.mirror[entry].index.z;
+        // the best primitive (no mesh, face or barycentrics)
+        const HitRec hr = wm.hit[1][sample];
+        qq.h.geom = qq.h.slot = qq.h.face = qq.h.mesh = -1;
+        qq.h.u = qq.h.v = 0.0f;
+        qq.h.dist = hr.dist;
+        qq.h.normal = V3{hr.nx, hr.ny, hr.nz};
+        if (hr.ref != -1) {
+          qq.h.slot = hr.ref & 0xffff;
+          qq.h.geom = __float_as_int(blk[L.geom_off + qq.h.slot * kGeomFloats + 16]);
+        }
+        qq.tie = hr.face == -2;
         qq.m.slot = -1;
         qq.m.sp = 0;
-        if (qq.m.meshes) return true;
-        done(qq);
-        return false;
+        return true;
       },
-      [&](ClosestWalk& qq) { return walk_closest_step(qq, s, st, blk, L, cull, &err); }, [&](ClosestWalk& qq, int32_t) { done(qq); }, &err);
+      [&](ClosestWalk& qq) { return walk_closest_step(qq, s, st, blk, L, cull, &err); },
+      [&](ClosestWalk& qq, int32_t) {
+        if (qq.tie) qq.h = trace_ray<true>(s, st, blk, L, qq.m.r, kMaxVal, cull, false, &err);
+        finish_mirror(wm, entry, sample, qq.h, -1);
+      },
+      &err);
   if (err && s.error_word) atomicOr(s.error_word, err);
 }
 
@@ -463,7 +542,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_SHADE_CTAS) wave_mirror_s
                                                                        const __grid_constant__ WaveMap wm) {
   __shared__ int32_t scan[kThreads / 32 + 1];
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
-  const int32_t count = (int32_t)min((int64_t)*wm.counters, wm.mirror_cap);
+  const int32_t count = (int32_t)min((int64_t)wm.counters[7], wm.mirror_cap);
   int32_t err = 0;
   // uniform trip count per CTA (the shadow entries are appended by whole CTAs)
   const int32_t stride = gridDim.x * kThreads;
@@ -475,22 +554,18 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_SHADE_CTAS) wave_mirror_s
     int32_t sample = 0;
     const float* blk = s.world_blocks;
     if (i < count) {
-      const MirrorEntry e = wm.mirror[i];
+      const MirrorEntry& e = wm.mirror[wm.mirror[i].index.w];
+      const float4 o = e.o, d = e.d;
       sample = e.index.x;
       const int32_t w = wm.w0 + sample / wm.per_world;
       blk = s.world_blocks + (int64_t)w * s.world_block_floats;
-      const HitRec hr = wm.hit[1][sample];
-      if (hr.ref == -1) {
-        wm.surf[1][sample] = missed_surface();
-      } else {
-        const Hit hit = unpack_hit(hr, blk, L);
-        const V3 so{e.o.x, e.o.y, e.o.z}, sd{e.d.x, e.d.y, e.d.z};
-        point = so + sd * hit.dist;
-        const float cone = e.o.w + e.d.w * hit.dist;
-        const Surface sf = eval_surface<kMesh, kTex>(s, blk, L, w, hit, hit.slot, point, sd, cone, &normal);
-        wm.surf[1][sample] = pack_surface(sf, normal, hit.dist, hit.slot);
-        shaded = true;
-      }
+      const Hit hit = unpack_hit(wm.hit[1][sample], blk, L);
+      const V3 so{o.x, o.y, o.z}, sd{d.x, d.y, d.z};
+      point = so + sd * hit.dist;
+      const float cone = o.w + d.w * hit.dist;
+      const Surface sf = eval_surface<kMesh, kTex>(s, blk, L, w, hit, hit.slot, point, sd, cone, &normal);
+      wm.surf[1][sample] = pack_surface(sf, normal, hit.dist, hit.slot);
+      shaded = true;
     }
     emit_shadows(s, wm, blk, L, shaded, point, normal, sample, 1, scan, &err);
   }
@@ -833,6 +908,11 @@ int launch_wave(const MjpbrScene& s, uint32_t seed, cudaStream_t stream, int32_t
   if (rc) return rc;
   const int sms = device_sm_count();
   const int g_mirror = sms * resident_ctas(k_mirror, stack);
+  int g_mesh = 0;
+  if constexpr (kScan) {
+    if ((rc = set_smem(wave_mirror_mesh_kernel, stack, "wavefront mirror meshes"))) return rc;
+    g_mesh = sms * resident_ctas(wave_mirror_mesh_kernel, stack);
+  }
   const int g_msurface = sms * resident_ctas(k_msurface, 0);
   const int g_shadow = sms * resident_ctas(k_shadow, stack);
   WaveMap wm;
@@ -858,7 +938,7 @@ int launch_wave(const MjpbrScene& s, uint32_t seed, cudaStream_t stream, int32_t
     }
     stage_mark(stream);
     if (rgb_tiles > 0) {
-      cudaError_t e = cudaMemsetAsync(wm.counters, 0, 6 * sizeof(int32_t), stream);  // queue lengths, fetch counters
+      cudaError_t e = cudaMemsetAsync(wm.counters, 0, 8 * sizeof(int32_t), stream);  // queue lengths, fetch counters
       if (e != cudaSuccess) return set_error(MJPBR_ERR_CUDA, "wavefront queue counters: %s", cudaGetErrorString(e));
       k_surface<<<dim3(rgb_tiles, wm.nw), kThreads, blk_bytes, stream>>>(s, wm);
       if ((rc = check_launch("wave_surface_kernel"))) return rc;
@@ -868,6 +948,10 @@ int launch_wave(const MjpbrScene& s, uint32_t seed, cudaStream_t stream, int32_t
     if (mirrors) {
       k_mirror<<<g_mirror, kThreads, stack, stream>>>(s, wm);
       if ((rc = check_launch("wave_mirror_kernel"))) return rc;
+      if constexpr (kScan) {
+        wave_mirror_mesh_kernel<<<g_mesh, kThreads, stack, stream>>>(s, wm);
+        if ((rc = check_launch("wave_mirror_mesh_kernel"))) return rc;
+      }
     }
     stage_mark(stream);
     if (mirrors) {
