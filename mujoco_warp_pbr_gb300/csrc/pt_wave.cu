@@ -395,6 +395,7 @@ MJ_DEV void closest_queue(const MjpbrScene& s, const Stack& st, const BlockLayou
           qq.m.meshes = scan_closest<true>(qq.h, qq.tie, NodeBoxes{blk, &L}, blk, L, qq.m.r, max_dist, cull);
           qq.m.slot = -1;
           qq.m.sp = 0;
+        qq.m.code = -1;
           if (qq.m.meshes) return true;
           done(qq);
           return false;
@@ -582,6 +583,7 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_shadow_kernel(const __grid_co
         [&](int64_t item, MeshWalk& qq) {
           qq.r = start(item, &qq.cut);
           qq.sp = 0;
+        qq.code = -1;
           const bool hit = scan_any<true>(blk, L, qq.r, qq.cut, cull, &qq.meshes);
           if (!hit && qq.meshes) return true;
           if (!hit) visible();

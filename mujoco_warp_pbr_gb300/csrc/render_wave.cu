@@ -525,6 +525,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_
         qq.tie = hr.face == -2;
         qq.m.slot = -1;
         qq.m.sp = 0;
+        qq.m.code = -1;
         return true;
       },
       [&](ClosestWalk& qq) { return walk_closest_step(qq, s, st, blk, L, cull, &err); },
@@ -650,6 +651,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_TRACE_CTAS) wave_shadow_s
         qq.r = r;
         qq.cut = max_dist;
         qq.sp = 0;
+        qq.code = -1;
         if (scan_any<true>(blk, L, r, max_dist, cull, &qq.meshes)) return false;
         if (qq.meshes) return true;
         atomicAdd(&wm.vis[target], 1);

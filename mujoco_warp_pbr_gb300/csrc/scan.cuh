@@ -247,6 +247,7 @@ struct MeshWalk {
   Ray r;
   uint32_t meshes;  // mesh geoms still to trace
   int32_t sp;
+  int32_t code;     // the node or leaf to visit, -1: the mesh (or the first one) is done
   int32_t slot;     // the mesh geom being traced, -1: none
   const float* nodes;
   const float* tris;
@@ -255,7 +256,7 @@ struct MeshWalk {
   float cut;        // hits at or past it do not count
 };
 
-MJ_DEV void walk_next(MeshWalk& q, const MjpbrScene& sc, const Stack& st, const float* blk, const BlockLayout& L, int32_t* err) {
+MJ_DEV void walk_next(MeshWalk& q, const MjpbrScene& sc, const float* blk, const BlockLayout& L) {
   const int32_t slot = __ffs(q.meshes) - 1;
   q.meshes &= q.meshes - 1u;
   const float* g = blk + L.geom_off + slot * kGeomFloats;
@@ -268,23 +269,23 @@ MJ_DEV void walk_next(MeshWalk& q, const MjpbrScene& sc, const Stack& st, const 
   q.ri = make_inv(Ray{lo, ld});
   q.slot = slot;
   q.sp = 0;
-  push(st, q.sp, 0, 0.0f, err);
+  q.code = 0;  // the root
 }
 
 // Any hit: q.cut = max_dist.
 MJ_DEV int32_t walk_any_step(MeshWalk& q, const MjpbrScene& sc, const Stack& st, const float* blk, const BlockLayout& L, int32_t* err) {
-  if (q.sp == 0) {
+  if (q.code < 0) {
     if (!q.meshes) return kAnyClear;
-    walk_next(q, sc, st, blk, L, err);
+    walk_next(q, sc, blk, L);
     return kAnyRunning;
   }
-  --q.sp;
-  if (st.t[q.sp * st.stride] >= q.cut) return kAnyRunning;
-  const int32_t code = st.code[q.sp * st.stride];
-  const int32_t ref = code >> 3, cnt = code & 7;
+  const int32_t ref = q.code >> 3, cnt = q.code & 7;
   if (cnt == 0) {
     const float* nd = q.nodes + (int64_t)ref * kNodeFloats;
-    expand(st, q.sp, q.ri, ldg4(nd), ldg4(nd + 4), ldg4(nd + 8), ldg4(nd + 12), q.cut, err);
+    if (!descend(st, q.sp, q.ri, ldg4(nd), ldg4(nd + 4), ldg4(nd + 8), ldg4(nd + 12), q.cut, &q.code, err) &&
+        !pop_near(st, q.sp, 0, q.cut, &q.code)) {
+      q.code = -1;
+    }
     return kAnyRunning;
   }
   for (int32_t i = ref; i < ref + cnt; ++i) {
@@ -294,6 +295,7 @@ MJ_DEV int32_t walk_any_step(MeshWalk& q, const MjpbrScene& sc, const Stack& st,
     MJPBR_COUNT(kOpTri);
     if (woop_hit(q.w, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, V3{c.x, c.y, c.z}, q.cut, &tu, &tv) >= 0.0f) return kAnyHit;
   }
+  if (!pop_near(st, q.sp, 0, q.cut, &q.code)) q.code = -1;
   return kAnyRunning;
 }
 
@@ -311,7 +313,7 @@ struct ClosestWalk {
 MJ_DEV int32_t walk_closest_step(ClosestWalk& q, const MjpbrScene& sc, const Stack& st, const float* blk, const BlockLayout& L, bool cull,
                                  int32_t* err) {
   MeshWalk& m = q.m;
-  if (m.sp == 0) {
+  if (m.code < 0) {
     if (m.slot >= 0) {  // the mesh is done
       if (q.face >= 0) {
         const float* g = blk + L.geom_off + m.slot * kGeomFloats;
@@ -320,19 +322,19 @@ MJ_DEV int32_t walk_closest_step(ClosestWalk& q, const MjpbrScene& sc, const Sta
       m.slot = -1;
     }
     if (!m.meshes) return kAnyClear;
-    walk_next(m, sc, st, blk, L, err);
+    walk_next(m, sc, blk, L);
     q.ld = mul_t(geom_frame(blk + L.geom_off + m.slot * kGeomFloats).mat, m.r.d);
     m.cut = scan_cut(q.h);
     q.face = -1;
     return kAnyRunning;
   }
-  --m.sp;
-  if (st.t[m.sp * st.stride] >= m.cut) return kAnyRunning;
-  const int32_t code = st.code[m.sp * st.stride];
-  const int32_t ref = code >> 3, cnt = code & 7;
+  const int32_t ref = m.code >> 3, cnt = m.code & 7;
   if (cnt == 0) {
     const float* nd = m.nodes + (int64_t)ref * kNodeFloats;
-    expand(st, m.sp, m.ri, ldg4(nd), ldg4(nd + 4), ldg4(nd + 8), ldg4(nd + 12), m.cut, err);
+    if (!descend(st, m.sp, m.ri, ldg4(nd), ldg4(nd + 4), ldg4(nd + 8), ldg4(nd + 12), m.cut, &m.code, err) &&
+        !pop_near(st, m.sp, 0, m.cut, &m.code)) {
+      m.code = -1;
+    }
     return kAnyRunning;
   }
   for (int32_t i = ref; i < ref + cnt; ++i) {
@@ -351,6 +353,7 @@ MJ_DEV int32_t walk_closest_step(ClosestWalk& q, const MjpbrScene& sc, const Sta
     q.u = tu;
     q.v = tv;
   }
+  if (!pop_near(st, m.sp, 0, m.cut, &m.code)) m.code = -1;
   return kAnyRunning;
 }
 

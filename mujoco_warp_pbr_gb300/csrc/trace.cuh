@@ -85,6 +85,39 @@ MJ_DEV void expand(const Stack& st, int& sp, const RayInv& ri, float4 alo, float
   if (tn >= 0.0f) push(st, sp, cn, tn, err);
 }
 
+// The same for traversals that keep the next entry in a register: the nearer hit child becomes *code, the
+// farther one is pushed; false when neither is hit. The nearer child is the entry expand's pushes would
+// pop next, so the order of the tests is expand's, without its way through the stack. For the resumable
+// walks (mirror rays of 24 x 200x150 worlds 313 -> 296 us, terrain shadows 1.46 -> 1.42 ms); the plain
+// loop of mesh_query is faster through the stack (camera rays 527 us, 554 so).
+MJ_DEV bool descend(const Stack& st, int& sp, const RayInv& ri, float4 alo, float4 ahi, float4 blo, float4 bhi, float cut, int32_t* code,
+                    int32_t* err) {
+  const int32_t acnt = __float_as_int(ahi.w), bcnt = __float_as_int(bhi.w);
+  if (acnt >= 0) MJPBR_COUNT(kOpBox);
+  if (bcnt >= 0) MJPBR_COUNT(kOpBox);
+  const float ta = acnt >= 0 ? box_entry(ri, alo.x, alo.y, alo.z, ahi.x, ahi.y, ahi.z, cut) : -1.0f;
+  const float tb = bcnt >= 0 ? box_entry(ri, blo.x, blo.y, blo.z, bhi.x, bhi.y, bhi.z, cut) : -1.0f;
+  const int32_t ca = (__float_as_int(alo.w) << 3) | acnt;
+  const int32_t cb = (__float_as_int(blo.w) << 3) | bcnt;
+  const bool swap = tb >= 0.0f && (ta < 0.0f || tb < ta);
+  const float tf = swap ? ta : tb;
+  if (tf >= 0.0f) push(st, sp, swap ? ca : cb, tf, err);
+  *code = swap ? cb : ca;
+  return (swap ? tb : ta) >= 0.0f;
+}
+
+// The next stack entry above sp0 nearer than cut; false when there is none.
+MJ_DEV bool pop_near(const Stack& st, int& sp, int sp0, float cut, int32_t* code) {
+  while (sp > sp0) {
+    --sp;
+    if (st.t[sp * st.stride] < cut) {
+      *code = st.code[sp * st.stride];
+      return true;
+    }
+  }
+  return false;
+}
+
 // Closest (or, with `any`, any) triangle of mesh `mesh` hit by the local ray in [0, tmax),
 // using stack entries above sp0. Returns the distance or -1; on a closest hit fills the local
 // geometric normal and the barycentrics of vertices 0 and 1. Any-hit queries do not cull.
