@@ -5,8 +5,10 @@
 // poses and sizes, then a bottom-up refit of each world's tree over the enabled geoms. The same
 // pass writes the world block (world_block.cuh) the render kernels stage into shared memory, so
 // the broadcasting of every batched table (worldid % nbatch) is resolved once per frame instead of
-// once per ray. One warp per world: lanes build geom, light and camera records in parallel, lane 0
-// sweeps the (small) tree bottom-up.
+// once per ray. Two warps per world: one builds the geom records and leaf boxes, its lanes in parallel,
+// and its lane 0 sweeps the (small) tree bottom-up; the other builds the light and camera records. Bound
+// by latency: the sweep's nodes stay in shared memory until it is done (16 worlds of 9 geoms 4.9 us, 17
+// through global memory and with one warp; 1024 of 12 8.7 us, 19 so).
 #include <cfloat>
 
 #include "abi_internal.h"
@@ -16,7 +18,7 @@
 namespace mjpbr {
 namespace {
 
-constexpr int kWarpsPerCta = 4;
+constexpr int kWorldsPerCta = 2;
 constexpr float kBigExtent = 1.0e6f;  // half extent of infinite planes
 
 // MuJoCo Warp's _geom_rgba: a geom with a material and the default rgba shows the material's.
@@ -117,79 +119,8 @@ __device__ __forceinline__ void geom_box(const MjpbrScene& s, const GeomBoxIn& i
   if (in.flags & kGeomFlagSkip) b[0] = FLT_MAX;  // marks an empty leaf
 }
 
-// kSmemBoxes: the lanes compute the leaf boxes into shared memory before lane 0's sweep; without
-// (worlds whose boxes do not fit), the sweep computes each leaf's box from its geom record.
-template <bool kSmemBoxes>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) refit_kernel(const __grid_constant__ MjpbrScene s) {
-  extern __shared__ float smem[];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int32_t w = blockIdx.x * kWarpsPerCta + warp;
-  if (w >= s.nworld) return;
-  const int32_t nbvh = s.nbvh_geom;
-  float* box = kSmemBoxes ? smem + (int64_t)warp * nbvh * 6 : nullptr;  // leaf AABBs of this world
-  BlockLayout L = block_layout(nbvh, s.nnode, s.nlight, s.nrender);
-  float* blk = s.world_blocks + (int64_t)w * s.world_block_floats;
-
-  // ---- geom records and leaf boxes
-  for (int32_t slot = lane; slot < nbvh; slot += 32) {
-    int32_t g = s.enabled_geom_ids[slot];
-    int32_t type = s.geom_type[g];
-    const float* xp = s.geom_xpos + ((int64_t)w * s.ngeom + g) * 3;
-    const float* xm = s.geom_xmat + ((int64_t)w * s.ngeom + g) * 9;
-    const float* sz = s.geom_size.ptr + ((int64_t)(w % s.geom_size.nbatch) * s.ngeom + g) * 3;
-    int32_t matid = s.geom_matid.ptr[(int64_t)(w % s.geom_matid.nbatch) * s.ngeom + g];
-    int32_t dataid = s.geom_dataid.ptr ? s.geom_dataid.ptr[(int64_t)(w % s.geom_dataid.nbatch) * s.ngeom + g] : -1;
-    float4 rgba = effective_rgba(s, w, g, matid);
-    float m[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) m[k] = xm[k];
-    V3 pos{xp[0], xp[1], xp[2]};
-    V3 size{sz[0], sz[1], sz[2]};
-    int32_t flags = 0;
-    // Triangle BVH of a mesh-like geom: the mesh's, or for a height field the one after the meshes.
-    int32_t blas = -1;
-    if (s.blas_root != nullptr && dataid >= 0) {
-      if ((type == MJPBR_GEOM_MESH || type == MJPBR_GEOM_SDF) && dataid < s.nmesh) blas = dataid;
-      if (type == MJPBR_GEOM_HFIELD && dataid < s.nhfield) blas = s.nmesh + dataid;
-    }
-    bool supported = type == MJPBR_GEOM_PLANE || type == MJPBR_GEOM_SPHERE || type == MJPBR_GEOM_CAPSULE ||
-                     type == MJPBR_GEOM_ELLIPSOID || type == MJPBR_GEOM_CYLINDER || type == MJPBR_GEOM_BOX || blas >= 0;
-    if (rgba.w == 0.0f || !supported) flags |= kGeomFlagSkip;
-    float* gr = blk + L.geom_off + slot * kGeomFloats;
-    gr[0] = pos.x;
-    gr[1] = pos.y;
-    gr[2] = pos.z;
-    gr[3] = __int_as_float(type);
-    gr[4] = m[0];
-    gr[5] = m[1];
-    gr[6] = m[2];
-    gr[7] = size.x;
-    gr[8] = m[3];
-    gr[9] = m[4];
-    gr[10] = m[5];
-    gr[11] = size.y;
-    gr[12] = m[6];
-    gr[13] = m[7];
-    gr[14] = m[8];
-    gr[15] = size.z;
-    gr[16] = __int_as_float(g);
-    gr[17] = __int_as_float(blas);
-    gr[18] = __int_as_float(matid);
-    gr[19] = __int_as_float(flags);
-
-    if constexpr (kSmemBoxes) {
-      GeomBoxIn in;
-      in.pos = pos;
-      for (int k = 0; k < 9; ++k) in.m[k] = m[k];
-      in.size = size;
-      in.type = type;
-      in.blas = blas;
-      in.flags = flags;
-      geom_box(s, in, box + slot * 6);
-    }
-  }
-
+// The light and camera records of a world, a lane each.
+__device__ __forceinline__ void refit_lights_cameras(const MjpbrScene& s, int32_t w, int lane, float* blk, const BlockLayout& L) {
   // ---- lights
   for (int32_t li = lane; li < s.nlight; li += 32) {
     float* lr = blk + L.light_off + li * kLightFloats;
@@ -262,6 +193,92 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) refit_kernel(const __grid_c
     cr[22] = 0.0f;
     cr[23] = 0.0f;
   }
+}
+
+// Where the sweep finds the leaf boxes and keeps the nodes: both in shared memory; the boxes (worlds
+// whose nodes do not fit beside them, a few hundred geoms); neither, each leaf's box computed from its geom
+// record (a few thousand geoms).
+enum RefitSmem { kSmemNone, kSmemBoxes, kSmemNodes };
+
+template <RefitSmem kSmem>
+__global__ void __launch_bounds__(kWorldsPerCta * 64) refit_kernel(const __grid_constant__ MjpbrScene s) {
+  extern __shared__ __align__(16) float smem[];
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int slot_in_cta = warp >> 1;
+  const int32_t w = blockIdx.x * kWorldsPerCta + slot_in_cta;
+  if (w >= s.nworld) return;
+  const int32_t nbvh = s.nbvh_geom;
+  const int32_t per_world = (kSmem == kSmemNodes ? s.nnode * kNodeFloats : 0) + nbvh * 6;
+  float* nodes = smem + (int64_t)slot_in_cta * ((per_world + 3) & ~3);
+  float* box = kSmem == kSmemNone ? nullptr : nodes + (kSmem == kSmemNodes ? s.nnode * kNodeFloats : 0);  // leaf AABBs of this world
+  BlockLayout L = block_layout(nbvh, s.nnode, s.nlight, s.nrender);
+  float* blk = s.world_blocks + (int64_t)w * s.world_block_floats;
+
+  if (warp & 1) {
+    refit_lights_cameras(s, w, lane, blk, L);
+    return;
+  }
+
+  // ---- geom records and leaf boxes
+  for (int32_t slot = lane; slot < nbvh; slot += 32) {
+    int32_t g = s.enabled_geom_ids[slot];
+    int32_t type = s.geom_type[g];
+    const float* xp = s.geom_xpos + ((int64_t)w * s.ngeom + g) * 3;
+    const float* xm = s.geom_xmat + ((int64_t)w * s.ngeom + g) * 9;
+    const float* sz = s.geom_size.ptr + ((int64_t)(w % s.geom_size.nbatch) * s.ngeom + g) * 3;
+    int32_t matid = s.geom_matid.ptr[(int64_t)(w % s.geom_matid.nbatch) * s.ngeom + g];
+    int32_t dataid = s.geom_dataid.ptr ? s.geom_dataid.ptr[(int64_t)(w % s.geom_dataid.nbatch) * s.ngeom + g] : -1;
+    float4 rgba = effective_rgba(s, w, g, matid);
+    float m[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) m[k] = xm[k];
+    V3 pos{xp[0], xp[1], xp[2]};
+    V3 size{sz[0], sz[1], sz[2]};
+    int32_t flags = 0;
+    // Triangle BVH of a mesh-like geom: the mesh's, or for a height field the one after the meshes.
+    int32_t blas = -1;
+    if (s.blas_root != nullptr && dataid >= 0) {
+      if ((type == MJPBR_GEOM_MESH || type == MJPBR_GEOM_SDF) && dataid < s.nmesh) blas = dataid;
+      if (type == MJPBR_GEOM_HFIELD && dataid < s.nhfield) blas = s.nmesh + dataid;
+    }
+    bool supported = type == MJPBR_GEOM_PLANE || type == MJPBR_GEOM_SPHERE || type == MJPBR_GEOM_CAPSULE ||
+                     type == MJPBR_GEOM_ELLIPSOID || type == MJPBR_GEOM_CYLINDER || type == MJPBR_GEOM_BOX || blas >= 0;
+    if (rgba.w == 0.0f || !supported) flags |= kGeomFlagSkip;
+    float* gr = blk + L.geom_off + slot * kGeomFloats;
+    gr[0] = pos.x;
+    gr[1] = pos.y;
+    gr[2] = pos.z;
+    gr[3] = __int_as_float(type);
+    gr[4] = m[0];
+    gr[5] = m[1];
+    gr[6] = m[2];
+    gr[7] = size.x;
+    gr[8] = m[3];
+    gr[9] = m[4];
+    gr[10] = m[5];
+    gr[11] = size.y;
+    gr[12] = m[6];
+    gr[13] = m[7];
+    gr[14] = m[8];
+    gr[15] = size.z;
+    gr[16] = __int_as_float(g);
+    gr[17] = __int_as_float(blas);
+    gr[18] = __int_as_float(matid);
+    gr[19] = __int_as_float(flags);
+
+    if constexpr (kSmem != kSmemNone) {
+      GeomBoxIn in;
+      in.pos = pos;
+      for (int k = 0; k < 9; ++k) in.m[k] = m[k];
+      in.size = size;
+      in.type = type;
+      in.blas = blas;
+      in.flags = flags;
+      geom_box(s, in, box + slot * 6);
+    }
+  }
+
   __syncwarp();
 
   // ---- bottom-up refit (children always follow their parent)
@@ -271,8 +288,9 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) refit_kernel(const __grid_c
     blk[2] = __int_as_float(s.nlight);
     blk[3] = __int_as_float(s.nrender);
     const int32_t* child = s.tlas_child.ptr + (int64_t)(w % s.tlas_child.nbatch) * s.nnode * 2;
+    float* node0 = kSmem == kSmemNodes ? nodes : blk + L.node_off;
     for (int32_t i = s.nnode - 1; i >= 0; --i) {
-      float* nd = blk + L.node_off + i * kNodeFloats;
+      float* nd = node0 + i * kNodeFloats;
       for (int k = 0; k < 2; ++k) {
         int32_t c = child[i * 2 + k];
         float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
@@ -283,7 +301,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) refit_kernel(const __grid_c
           int32_t slot = ~c;
           float tb[6];
           const float* b = tb;
-          if constexpr (kSmemBoxes) {
+          if constexpr (kSmem != kSmemNone) {
             b = box + slot * 6;
           } else {
             geom_box(s, geom_box_in(blk + L.geom_off + slot * kGeomFloats), tb);
@@ -297,7 +315,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) refit_kernel(const __grid_c
             cnt = 1;
           }
         } else {
-          const float* cn = blk + L.node_off + c * kNodeFloats;
+          const float* cn = node0 + c * kNodeFloats;
           int32_t ca = __float_as_int(cn[7]), cb = __float_as_int(cn[15]);
           if (ca >= 0 || cb >= 0) {
             for (int a = 0; a < 3; ++a) {
@@ -322,20 +340,28 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) refit_kernel(const __grid_c
       }
     }
   }
+  if constexpr (kSmem == kSmemNodes) {
+    __syncwarp();
+    const float4* src = reinterpret_cast<const float4*>(nodes);
+    float4* dst = reinterpret_cast<float4*>(blk + L.node_off);
+    for (int32_t i = lane; i < s.nnode * (kNodeFloats / 4); i += 32) dst[i] = src[i];
+  }
 }
 
 }  // namespace
 
 int refit_launch(const MjpbrScene& s, cudaStream_t stream) {
-  const size_t smem = (size_t)kWarpsPerCta * s.nbvh_geom * 6 * sizeof(float);
-  const int grid = (s.nworld + kWarpsPerCta - 1) / kWarpsPerCta;
-  if (smem <= 200 * 1024) {
-    if (int rc = ensure_smem(reinterpret_cast<const void*>(refit_kernel<true>), smem, "refit")) return rc;
-    refit_kernel<true><<<grid, kWarpsPerCta * 32, smem, stream>>>(s);
-  } else {
-    refit_kernel<false><<<grid, kWarpsPerCta * 32, 0, stream>>>(s);  // leaf boxes computed in the sweep
-  }
-  return check_launch("refit_kernel");
+  const int grid = (s.nworld + kWorldsPerCta - 1) / kWorldsPerCta;
+  auto launch = [&](auto kern, size_t smem) {
+    if (int rc = ensure_smem(reinterpret_cast<const void*>(kern), smem, "refit")) return rc;
+    kern<<<grid, kWorldsPerCta * 64, smem, stream>>>(s);
+    return check_launch("refit_kernel");
+  };
+  auto bytes = [&](int64_t floats) { return (size_t)kWorldsPerCta * ((floats + 3) & ~(int64_t)3) * sizeof(float); };
+  const size_t boxes = bytes((int64_t)s.nbvh_geom * 6), all = bytes((int64_t)s.nbvh_geom * 6 + (int64_t)s.nnode * kNodeFloats);
+  if (all <= 100 * 1024) return launch(refit_kernel<kSmemNodes>, all);
+  if (boxes <= 100 * 1024) return launch(refit_kernel<kSmemBoxes>, boxes);
+  return launch(refit_kernel<kSmemNone>, 0);
 }
 
 }  // namespace mjpbr
