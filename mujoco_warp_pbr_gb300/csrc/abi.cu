@@ -353,7 +353,7 @@ int mjpbr_upsample2_bf16(const uint16_t* in, uint16_t* out, int32_t nimg, int32_
 
 int mjpbr_kpcn_apply(const float* logits, const float* radiance, float* weights, float* out, int32_t nimg, int32_t h, int32_t w,
                      void* stream) {
-  return kpcn_apply_launch(logits, radiance, weights, out, nimg, h, w, static_cast<cudaStream_t>(stream));
+  return kpcn_apply_launch(logits, radiance, weights, out, nimg, h, w, (int64_t)h * w, (int64_t)h * w, static_cast<cudaStream_t>(stream));
 }
 
 int mjpbr_kpcn_loss(const float* out, const float* target, const float* scale, const float* offset, float* grad, float* sums,

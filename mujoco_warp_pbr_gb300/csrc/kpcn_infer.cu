@@ -25,7 +25,7 @@ constexpr Layer kLayers[MJPBR_KPCN_LAYERS] = {
 // The workspace of one chunk: activations NHWC (BF16 unless noted), each 256-byte aligned.
 struct Workspace {
   uint16_t *x0, *a0, *s0, *u0, *v0, *up0, *p1, *a1, *s1, *u1, *v1, *up1, *p2, *a2, *s2, *u2, *v2, *up2, *p3, *a3, *b3;
-  float *radiance, *logits, *out;
+  float* logits;
 };
 
 int64_t layout(int32_t nimg, int32_t h, int32_t w, char* base, Workspace* ws) {
@@ -39,13 +39,11 @@ int64_t layout(int32_t nimg, int32_t h, int32_t w, char* base, Workspace* ws) {
   auto f32 = [&](int32_t level, int32_t c) { return reinterpret_cast<float*>(take(level, c, 4)); };
   Workspace t;
   t.x0 = b16(0, kFeatures);
-  t.radiance = f32(0, 4);
   t.a0 = b16(0, 32), t.s0 = b16(0, 32), t.u0 = b16(0, 32), t.v0 = b16(0, 32), t.up0 = b16(0, 48);
   t.p1 = b16(1, 32), t.a1 = b16(1, 48), t.s1 = b16(1, 48), t.u1 = b16(1, 48), t.v1 = b16(1, 48), t.up1 = b16(1, 64);
   t.p2 = b16(2, 48), t.a2 = b16(2, 64), t.s2 = b16(2, 64), t.u2 = b16(2, 64), t.v2 = b16(2, 64), t.up2 = b16(2, 96);
   t.p3 = b16(3, 64), t.a3 = b16(3, 96), t.b3 = b16(3, 96);
   t.logits = f32(0, kLogits);
-  t.out = f32(0, 4);
   if (ws) *ws = t;
   return off;
 }
@@ -83,8 +81,10 @@ int conv(const MjpbrKpcnWeights& wts, int32_t k, const uint16_t* in, const uint1
   return conv3x3_launch(c, st);
 }
 
-// The U-Net forward pass of kpcn.KPCN.forward on ws.x0 / ws.radiance into ws.out.
-int forward(const MjpbrKpcnWeights& wts, const Workspace& ws, int32_t n, int32_t h, int32_t w, int32_t* err, cudaStream_t st) {
+// The U-Net forward pass of kpcn.KPCN.forward on ws.x0; its kernels applied to `radiance` into `out`, images
+// `stride` pixels apart (the denoiser's own buffers, read and written in place).
+int forward(const MjpbrKpcnWeights& wts, const Workspace& ws, const float* radiance, float* out, int64_t stride, int32_t n, int32_t h, int32_t w,
+            int32_t* err, cudaStream_t st) {
   int rc = 0;
   auto c = [&](int32_t k, const uint16_t* in, uint16_t* out, const uint16_t* in2 = nullptr, float* out_f32 = nullptr) {
     if (!rc) rc = conv(wts, k, in, in2, out, out_f32, n, h, w, err, st);
@@ -116,7 +116,7 @@ int forward(const MjpbrKpcnWeights& wts, const Workspace& ws, int32_t n, int32_t
   c(12, ws.s0, ws.u0, ws.up0);
   c(13, ws.u0, ws.v0);
   c(14, ws.v0, nullptr, nullptr, ws.logits);
-  if (!rc) rc = kpcn_apply_launch(ws.logits, ws.radiance, nullptr, ws.out, n, h, w, st);
+  if (!rc) rc = kpcn_apply_launch(ws.logits, radiance, nullptr, out, n, h, w, stride, stride, st);
   return rc;
 }
 
@@ -143,22 +143,15 @@ int denoise_learned_launch(const MjpbrScene& s, const MjpbrKpcnWeights& wts, voi
     const int64_t need = kpcn_workspace_bytes(nw_max, h, w);
     if (need < 0) return set_error(MJPBR_ERR_ARG, "denoise_learned: camera %d of %dx%d is not tiled by the network (use the a-trous filter)", cam, w, h);
     if (need > workspace_bytes) return set_error(MJPBR_ERR_ARG, "denoise_learned: workspace of %lld bytes, %lld needed", (long long)workspace_bytes, (long long)need);
-    const int64_t npix = (int64_t)w * h;
     for (int32_t w0 = 0; w0 < s.nworld; w0 += chunk) {
       const int32_t nw = std::min(chunk, s.nworld - w0);
       Workspace ws;
       layout(nw, h, w, static_cast<char*>(workspace), &ws);
       int rc = kpcn_features_launch(s, cam, w0, nw, ws.x0, st);
       if (rc) return rc;
-      const size_t pitch = (size_t)s.rgb_stride * 16, bytes = (size_t)npix * 16;
-      const float* src = s.denoise_buffers[0] + ((int64_t)w0 * s.rgb_stride + s.rgb_adr[cam]) * 4;
-      cudaError_t e = cudaMemcpy2DAsync(ws.radiance, bytes, src, pitch, bytes, nw, cudaMemcpyDeviceToDevice, st);
-      if (e != cudaSuccess) return set_error(MJPBR_ERR_CUDA, "denoise_learned: radiance copy: %s", cudaGetErrorString(e));
-      rc = forward(wts, ws, nw, h, w, s.error_word, st);
+      const int64_t first = ((int64_t)w0 * s.rgb_stride + s.rgb_adr[cam]) * 4;
+      rc = forward(wts, ws, s.denoise_buffers[0] + first, s.denoise_buffers[1] + first, s.rgb_stride, nw, h, w, s.error_word, st);
       if (rc) return rc;
-      float* dst = s.denoise_buffers[1] + ((int64_t)w0 * s.rgb_stride + s.rgb_adr[cam]) * 4;
-      e = cudaMemcpy2DAsync(dst, pitch, ws.out, bytes, bytes, nw, cudaMemcpyDeviceToDevice, st);
-      if (e != cudaSuccess) return set_error(MJPBR_ERR_CUDA, "denoise_learned: output copy: %s", cudaGetErrorString(e));
     }
   }
   // the a-trous filter's finish pass without filtering, on the network's radiance
