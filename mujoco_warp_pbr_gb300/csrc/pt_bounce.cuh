@@ -100,9 +100,17 @@ struct PtCore {
     return cmul(diffuse, q.ds) + cmul(specular, q.ss);
   }
 
-  // The bounce after its closest hit (pathtrace.py:230-337); true when the path has ended.
-  template <class Nee>
-  static MJ_DEV bool surface(RtCtx& c, Nee& nee, PathState& ps, const Hit& hit, uint32_t seed, V3 head_dir) {
+  // The bounce after its closest hit (pathtrace.py:230-337) in four phases: the surface, the lights'
+  // next-event estimates, the environment's, the continuation. A kernel whose warps run apart calls them
+  // one after the other (surface, below); the staged one keeps its warps in the same phase.
+  struct Vertex {
+    V3 point, normal, t1, t2, v;
+    Lobes lb;
+    float p_spec;
+  };
+  enum Status { kEnded, kLive, kShade };  // the path has ended; goes on without shading; the other phases follow
+
+  static MJ_DEV Status reach(RtCtx& c, PathState& ps, const Hit& hit, uint32_t seed, Vertex& x) {
     const MjpbrScene& s = *c.s;
     const MjpbrSettings& st = s.settings;
     if (hit.geom == -1) {
@@ -120,7 +128,7 @@ struct PtCore {
         }
         ps.radiance += cmul(ps.beta, env_light);
       }
-      return true;
+      return kEnded;
     }
     const V3 point = ps.o + ps.d * hit.dist;
     V3 normal;
@@ -131,11 +139,11 @@ struct PtCore {
         ps.o = point + ps.d * kRayOffset;
         ps.max_dist = ps.max_dist - hit.dist;
         ps.passes += 1;
-        return false;
+        return kLive;
       }
     }
     ps.radiance += cmul(ps.beta, sf.emissive / c.exposure);
-    if (ps.depth == st.max_depth) return true;
+    if (ps.depth == st.max_depth) return kEnded;
     ps.max_dist = kMaxVal;
     if (ps.camera_ray) {
       ps.albedo = sf.base_color;
@@ -152,22 +160,28 @@ struct PtCore {
         ps.o = point + normal * kRayOffset;
         ps.delta = true;
         ps.depth += 1;
-        return ps.depth > st.max_depth;
+        return ps.depth > st.max_depth ? kEnded : kLive;
       }
     }
-    V3 t1, t2;
-    orthonormal_basis(normal, &t1, &t2);
+    x.point = point;
+    x.normal = normal;
+    orthonormal_basis(normal, &x.t1, &x.t2);
     const V3 view = -ps.d;
-    const V3 v{dot(view, t1), dot(view, t2), dot(view, normal)};
-    const float nov = fmaxf(v.z, 1.0e-4f);
-    const Lobes lb = shading_lobes(s.dfg_lut, s.dfg_size, sf, nov);
-    const V3 spec_weight = cmul(lb.spec_albedo, lb.energy_comp);
-    const float p_spec = specular_probability(lb.diffuse_color, spec_weight);
-    if (ps.depth == 0 && camera_ray) ps.albedo = lb.diffuse_color + spec_weight;
+    x.v = V3{dot(view, x.t1), dot(view, x.t2), dot(view, normal)};
+    const float nov = fmaxf(x.v.z, 1.0e-4f);
+    x.lb = shading_lobes(s.dfg_lut, s.dfg_size, sf, nov);
+    const V3 spec_weight = cmul(x.lb.spec_albedo, x.lb.energy_comp);
+    x.p_spec = specular_probability(x.lb.diffuse_color, spec_weight);
+    if (ps.depth == 0 && camera_ray) ps.albedo = x.lb.diffuse_color + spec_weight;
+    return kShade;
+  }
 
-    // next-event estimation: MuJoCo lights (slots 0 .. nlight - 1), then the headlight (slot
-    // nlight: no shadow, display-relative), then the environment
-    const V3 origin = point + normal * kRayOffset;
+  // next-event estimation: MuJoCo lights (slots 0 .. nlight - 1), then the headlight (slot nlight: no
+  // shadow, display-relative), then the environment
+  template <class Nee>
+  static MJ_DEV void lights(RtCtx& c, Nee& nee, PathState& ps, const Vertex& x, uint32_t seed, V3 head_dir) {
+    const MjpbrSettings& st = c.s->settings;
+    const V3 origin = x.point + x.normal * kRayOffset;
     nee.begin(ps, origin);
     const int32_t nl = c.L.nlight + (st.headlight_active ? 1 : 0);
 #pragma unroll 1
@@ -182,41 +196,48 @@ struct PtCore {
         light = make_headlight(st, head_dir, c.exposure);
       }
       LightQuery q;
-      if (!light_query(c, light, point, normal, t1, t2, u0, u1, &q)) {
+      if (!light_query(c, light, x.point, x.normal, x.t1, x.t2, u0, u1, &q)) {
         nee.none(li);
         continue;
       }
-      nee.light(c, li, q.shadowed, origin, q.l, q.max_t, [&] { return light_contribution(lb, v, q); });
+      nee.light(c, li, q.shadowed, origin, q.l, q.max_t, [&] { return light_contribution(x.lb, x.v, q); });
     }
     nee.lights_done(ps);
+  }
 
-    if (kTex && st.has_env) {
+  template <class Nee>
+  static MJ_DEV void env_light(RtCtx& c, Nee& nee, PathState& ps, const Vertex& x, uint32_t seed) {
+    const MjpbrScene& s = *c.s;
+    if (kTex && s.settings.has_env) {
       float pdf_env;
       MJPBR_COUNT(kOpPtEnvSample);
       const int32_t h = s.cdf_height, w = s.cdf_width;
       V3 d_env = env_sample_direction(s.env_marginal + (int64_t)c.env * (h + 1), s.env_conditional + (int64_t)c.env * h * (w + 1),
                                       s.env_prob + (int64_t)c.env * h * w, h, w, c.env_yaw,
                                       pt_rand(seed, ps.sample, ps.depth, 2), pt_rand(seed, ps.sample, ps.depth, 3), &pdf_env);
-      V3 le{dot(d_env, t1), dot(d_env, t2), dot(d_env, normal)};
+      V3 le{dot(d_env, x.t1), dot(d_env, x.t2), dot(d_env, x.normal)};
       if (le.z > 0.0f && pdf_env > 0.0f) {
-        V3 f = eval_bsdf_cos(lb.diffuse_color, lb.f0, lb.alpha, lb.energy_comp, v, le);
+        V3 f = eval_bsdf_cos(x.lb.diffuse_color, x.lb.f0, x.lb.alpha, x.lb.energy_comp, x.v, le);
         const V3 beta = ps.beta;
-        nee.env(c, ps, origin, d_env, [&] {
-          float weight = power_heuristic(pdf_env, pdf_bsdf(lb.alpha, p_spec, v, le));
+        nee.env(c, ps, x.point + x.normal * kRayOffset, d_env, [&] {
+          float weight = power_heuristic(pdf_env, pdf_bsdf(x.lb.alpha, x.p_spec, x.v, le));
           return cmul(beta, cmul(f, environment(c, d_env))) * (weight / pdf_env);
         });
       }
     }
+  }
 
-    // continue the path by sampling the BSDF
-    const V3 l = sample_bsdf(lb.alpha, p_spec, v, pt_rand(seed, ps.sample, ps.depth, 12), pt_rand(seed, ps.sample, ps.depth, 13),
+  // Continues the path by sampling the BSDF; true when it has ended.
+  static MJ_DEV bool proceed(RtCtx& c, PathState& ps, const Vertex& x, uint32_t seed) {
+    const MjpbrSettings& st = c.s->settings;
+    const V3 l = sample_bsdf(x.lb.alpha, x.p_spec, x.v, pt_rand(seed, ps.sample, ps.depth, 12), pt_rand(seed, ps.sample, ps.depth, 13),
                              pt_rand(seed, ps.sample, ps.depth, 14));
     if (l.z <= 0.0f) return true;
-    const float pdf = pdf_bsdf(lb.alpha, p_spec, v, l);
+    const float pdf = pdf_bsdf(x.lb.alpha, x.p_spec, x.v, l);
     if (pdf <= 0.0f) return true;
-    ps.beta = cmul(ps.beta, eval_bsdf_cos(lb.diffuse_color, lb.f0, lb.alpha, lb.energy_comp, v, l) / pdf);
-    ps.d = normalize(t1 * l.x + t2 * l.y + normal * l.z);
-    ps.o = point + normal * kRayOffset;
+    ps.beta = cmul(ps.beta, eval_bsdf_cos(x.lb.diffuse_color, x.lb.f0, x.lb.alpha, x.lb.energy_comp, x.v, l) / pdf);
+    ps.d = normalize(x.t1 * l.x + x.t2 * l.y + x.normal * l.z);
+    ps.o = x.point + x.normal * kRayOffset;
     ps.pdf_prev = pdf;
     ps.delta = false;
     ps.depth += 1;
@@ -226,6 +247,17 @@ struct PtCore {
       ps.beta = ps.beta / q;
     }
     return ps.depth > st.max_depth;
+  }
+
+  // The whole bounce; true when the path has ended.
+  template <class Nee>
+  static MJ_DEV bool surface(RtCtx& c, Nee& nee, PathState& ps, const Hit& hit, uint32_t seed, V3 head_dir) {
+    Vertex x;
+    const Status status = reach(c, ps, hit, seed, x);
+    if (status != kShade) return status == kEnded;
+    lights(c, nee, ps, x, seed, head_dir);
+    env_light(c, nee, ps, x, seed);
+    return proceed(c, ps, x, seed);
   }
 };
 

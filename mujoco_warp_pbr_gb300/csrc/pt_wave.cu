@@ -56,7 +56,7 @@ constexpr int kThreads = 256;
 #define MJPBR_PTW_SHADE_CTAS 3
 #endif
 #ifndef MJPBR_PTW_TEX_CTAS
-#define MJPBR_PTW_TEX_CTAS 2
+#define MJPBR_PTW_TEX_CTAS 3
 #endif
 
 // A path between stages: 80 bytes every bounce reads and writes, and the first surface's denoiser
@@ -103,9 +103,13 @@ struct PtWaveMap {
   float4* hit;             // (kHitFields, path_cap)
   float4* nee;             // (1 + nslot, path_cap): the bounce's throughput, then each slot's term
   uint8_t* state;          // (nslot, path_cap)
-  int32_t* queue[2];
+  int32_t* live;           // paths to extend
+  int32_t* reached;        // extended paths: those that hit from the front, those that missed from the end (path_cap)
   float4* shadow;          // (kShadowFields, shadow_cap)
-  int32_t* counters;       // [0], [1] queue lengths, [2] shadow entries; 64-bit fetch counters of extend [4..5], shadow [6..7]
+  // [0], [1] length of `live` in even and odd bounces, [2] shadow entries, [3] hits and [8] misses in
+  // `reached`; 64-bit fetch counters of extend [4..5] and shadow [6..7]. Zero before the first bounce; then each
+  // stage clears what the stages before it are done with and the ones after it count again.
+  int32_t* counters;
   int64_t path_cap, shadow_cap;
 };
 
@@ -421,19 +425,23 @@ MJ_DEV void closest_queue(const MjpbrScene& s, const Stack& st, const BlockLayou
 // larger scenes walk the scene BVH resumably.
 template <bool kMesh, bool kScan>
 __global__ void __launch_bounds__(kThreads, 3) ptw_extend_kernel(const __grid_constant__ MjpbrScene s,
-                                                                 const __grid_constant__ PtWaveMap wm, int32_t cur, bool pending_nee) {
+                                                                 const __grid_constant__ PtWaveMap wm, int32_t parity) {
   extern __shared__ __align__(16) float smem[];
   const Stack st = wave_stack(s, smem);
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
   const bool cull = s.settings.cull_backfaces != 0;
-  const int64_t items = min((int64_t)wm.counters[cur], wm.path_cap);
+  const int64_t items = min((int64_t)wm.counters[parity], wm.path_cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    wm.counters[parity ^ 1] = 0;
+    wm.counters[2] = wm.counters[6] = wm.counters[7] = 0;
+  }
   unsigned long long* fetched = reinterpret_cast<unsigned long long*>(wm.counters + 4);
   int32_t err = 0;
   const float* blk = nullptr;
   int32_t path = -1;
   auto start = [&](int64_t item, float* max_dist) {
-    path = wm.queue[cur][item];
-    if (pending_nee) apply_nee(wm, path);
+    path = wm.live[item];
+    apply_nee(wm, path);
     const float4 o = path_field(wm, kPathOrigin, path), d = path_field(wm, kPathDir, path);
     blk = world_block(s, wm.w0 + (path / wm.nsample) / wm.pixels);
     *max_dist = o.w;
@@ -442,14 +450,27 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_extend_kernel(const __grid_co
   auto finish = [&](const Hit& hit) {
     // the first hits, and the geometry they write, are ptw_first_extend_kernel's
     store_hit(wm, path, hit);
+    // hits and misses apart: half the secondary rays miss, which a shading warp would wait out
+    const bool miss = hit.geom == -1;
+    cg::coalesced_group g = cg::coalesced_threads();
+    const unsigned misses = g.ballot(miss);
+    const int32_t nmiss = __popc(misses), rank = __popc(misses & ((1u << g.thread_rank()) - 1u));
+    int32_t at_hit = 0, at_miss = 0;
+    if (g.thread_rank() == 0) {
+      if (nmiss < (int32_t)g.size()) at_hit = atomicAdd(wm.counters + 3, (int32_t)g.size() - nmiss);
+      if (nmiss) at_miss = atomicAdd(wm.counters + 8, nmiss);
+    }
+    at_hit = g.shfl(at_hit, 0) + (int32_t)g.thread_rank() - rank;
+    at_miss = g.shfl(at_miss, 0) + rank;
+    wm.reached[miss ? wm.path_cap - 1 - at_miss : at_hit] = path;
   };
   closest_queue<kMesh, kScan>(s, st, L, cull, items, fetched, blk, start, finish, &err);
   if (err && s.error_word) atomicOr(s.error_word, err);
 }
 
 // The first bounce's extend, with the start folded in: each path's camera ray is generated where
-// it is traced (start_sample, pt_bounce.cuh) and the path record written once, after the hit; the
-// path queue of the shade stage is the identity.
+// it is traced (start_sample, pt_bounce.cuh) and the path record written once, after the hit. The shade
+// stage takes the paths in their own order: neighbouring camera rays mostly hit or miss together.
 template <bool kMesh, bool kScan>
 __global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
                                                                        const __grid_constant__ PtWaveMap wm) {
@@ -457,7 +478,6 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __g
   const Stack st = wave_stack(s, smem);
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
   const bool cull = s.settings.cull_backfaces != 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) wm.counters[0] = wm.npath;  // the shade stage's queue
   unsigned long long* fetched = reinterpret_cast<unsigned long long*>(wm.counters + 4);
   int32_t err = 0;
   const float* blk = nullptr;
@@ -472,7 +492,6 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __g
   };
   auto start = [&](int64_t item, float* max_dist) {
     path = (int32_t)item;
-    wm.queue[0][path] = path;
     PathState ps;
     Pixel p;
     int32_t w, sample;
@@ -502,45 +521,69 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __g
 // ---------------------------------------------------------------- shade
 template <bool kMesh, bool kTex>
 __global__ void __launch_bounds__(kThreads, kTex ? MJPBR_PTW_TEX_CTAS : MJPBR_PTW_SHADE_CTAS) ptw_shade_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
-                                                                const __grid_constant__ PtWaveMap wm, int32_t cur) {
+                                                                const __grid_constant__ PtWaveMap wm, int32_t parity, bool first) {
   __shared__ int32_t scan[kThreads / 32 + 1];
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
-  const int32_t next = cur ^ 1;
-  const int32_t count = (int32_t)min((int64_t)wm.counters[cur], wm.path_cap);
+  // the first bounce's paths in order, or the reached ones: the hits, then the misses
+  const int32_t hits = wm.counters[3];
+  const int32_t count = first ? wm.npath : (int32_t)min((int64_t)hits + wm.counters[8], wm.path_cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) wm.counters[4] = wm.counters[5] = 0;
   const int32_t stride = gridDim.x * kThreads;
   const int32_t rounds = (count + stride - 1) / stride;
   int32_t err = 0;
   for (int32_t round = 0; round < rounds; ++round) {
     const int32_t i = round * stride + blockIdx.x * kThreads + threadIdx.x;
+    const bool active = i < count;
     int32_t path = -1;
-    bool live = false;
-    if (i < count) {
-      path = wm.queue[cur][i];
+    bool features = false;
+    using Core = PtCore<kMesh, kTex>;
+    typename Core::Status status = Core::kEnded;
+    typename Core::Vertex x;
+    RtCtx c;
+    PathState ps;
+    float first_depth = 0.0f;
+    uint32_t pseed = 0;
+    V3 head_dir = v3(0.0f);
+    if (active) {
+      path = first ? i : wm.reached[i < hits ? i : (int32_t)wm.path_cap - 1 - (i - hits)];
       int32_t w, sample;
       Pixel p;
       path_pixel(s, wm, path, &w, &p, &sample);
       const float* blk = world_block(s, w);
-      RtCtx c;
       init_ctx(c, s, blk, L, w, kTex);
       p.rec = blk + L.cam_off + p.cam * kCamFloats;
       const M3 R = cam_mat(p.rec);
-      const V3 head_dir = -V3{R.m[2], R.m[5], R.m[8]};
-      float first_depth;
-      PathState ps = load_path(wm, path, &first_depth);
+      head_dir = -V3{R.m[2], R.m[5], R.m[8]};
+      pseed = pixel_seed_of(s, seed, w, p);
+      ps = load_path(wm, path, &first_depth);
       // only a camera ray's bounce can set the first surface's features
-      const bool features = ps.camera_ray;
+      features = ps.camera_ray;
       const Hit hit = load_hit(wm, path, blk, L);
-      RecordedNee nee{path, v3(0.0f), &wm, &err};
-      nee.state(wm.nslot - 1) = 0;
-      live = !PtCore<kMesh, kTex>::surface(c, nee, ps, hit, pixel_seed_of(s, seed, w, p), head_dir);
+      wm.state[(wm.nslot - 1) * wm.path_cap + path] = 0;
+      status = Core::reach(c, ps, hit, pseed, x);
+      if (features) store_path_features(wm, path, ps);
+    }
+    // The CTA's warps take each phase together: the stage's code is several times the instruction cache (on
+    // 1024 x 128x128 and, with environments, 128 x 2 x 256x256 paths: 8.7 and 14.5 ms, and 11.8 and 26.4
+    // with no barrier at all, paths appended by warps).
+    RecordedNee nee{path, v3(0.0f), &wm, &err};
+    __syncthreads();
+    if (status == Core::kShade) Core::lights(c, nee, ps, x, pseed, head_dir);
+    __syncthreads();
+    if (kTex) {
+      if (status == Core::kShade) Core::env_light(c, nee, ps, x, pseed);
+      __syncthreads();
+    }
+    bool live = status == Core::kLive;
+    if (status == Core::kShade) live = !Core::proceed(c, ps, x, pseed);
+    if (active) {
       store_path_radiance(wm, path, ps, first_depth);
       if (live) store_path_live(wm, path, ps);
-      if (features) store_path_features(wm, path, ps);
       err |= c.err;
     }
     // the paths that continue
-    const int64_t pos = cta_append(live, wm.counters + next, wm.path_cap, scan, &err);
-    if (pos >= 0) wm.queue[next][pos] = path;
+    const int64_t pos = cta_append(live, wm.counters + (parity ^ 1), wm.path_cap, scan, &err);
+    if (pos >= 0) wm.live[pos] = path;
   }
   if (err && s.error_word) atomicOr(s.error_word, err);
 }
@@ -555,6 +598,7 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_shadow_kernel(const __grid_co
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
   const bool cull = s.settings.cull_backfaces != 0;
   const int64_t items = min((int64_t)wm.counters[2], wm.shadow_cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) wm.counters[3] = wm.counters[8] = 0;
   unsigned long long* fetched = reinterpret_cast<unsigned long long*>(wm.counters + 6);
   int32_t err = 0;
   const float* blk = nullptr;
@@ -684,8 +728,8 @@ int64_t layout(PtWaveMap* wm, char* base, int64_t npath, int32_t nslot) {
     wm->hit = reinterpret_cast<float4*>(hit);
     wm->nee = reinterpret_cast<float4*>(nee);
     wm->state = reinterpret_cast<uint8_t*>(state);
-    wm->queue[0] = reinterpret_cast<int32_t*>(q0);
-    wm->queue[1] = reinterpret_cast<int32_t*>(q1);
+    wm->live = reinterpret_cast<int32_t*>(q0);
+    wm->reached = reinterpret_cast<int32_t*>(q1);
     wm->shadow = reinterpret_cast<float4*>(shadow);
     wm->path_cap = npath;
     wm->shadow_cap = npath * nslot;
@@ -732,7 +776,6 @@ int launch_pt_wave(const MjpbrScene& s, uint32_t seed, cudaStream_t stream, int3
   layout(&wm, static_cast<char*>(s.wave_scratch), (int64_t)chunk * pixels * wm.nsample, wm.nslot);
   const int32_t geo_pixels = wm.geo_base[s.nrender];
   const int32_t iterations = s.settings.max_depth + 1 + (s.settings.has_transparency ? 4 * s.settings.max_layers : 0);
-  const bool shadows = true;  // every bounce may ask for shadow rays (lights, environment)
   for (int32_t w0 = 0; w0 < s.nworld; w0 += chunk) {
     wm.w0 = w0;
     wm.nw = std::min(chunk, s.nworld - w0);
@@ -743,28 +786,22 @@ int launch_pt_wave(const MjpbrScene& s, uint32_t seed, cudaStream_t stream, int3
       if ((rc = check_launch("ptw_geometry_kernel"))) return rc;
     }
     if (wm.npath == 0) continue;
-    // queue lengths and the fetch counters; the first extend sets the shade stage's queue length
-    cudaError_t ez = cudaMemsetAsync(wm.counters, 0, 8 * sizeof(int32_t), stream);
+    cudaError_t ez = cudaMemsetAsync(wm.counters, 0, 9 * sizeof(int32_t), stream);
     if (ez != cudaSuccess) return set_error(MJPBR_ERR_CUDA, "path wavefront counters: %s", cudaGetErrorString(ez));
     for (int32_t it = 0; it < iterations; ++it) {
-      const int32_t cur = it & 1, next = cur ^ 1;
+      const int32_t parity = it & 1;
       if (it == 0) {
         k_first<<<g_first, kThreads, stack, stream>>>(s, seed, wm);
         if ((rc = check_launch("ptw_first_extend_kernel"))) return rc;
       } else {
-        k_extend<<<g_extend, kThreads, stack, stream>>>(s, wm, cur, true);
+        k_extend<<<g_extend, kThreads, stack, stream>>>(s, wm, parity);
         if ((rc = check_launch("ptw_extend_kernel"))) return rc;
       }
-      cudaError_t e = cudaMemsetAsync(wm.counters + next, 0, sizeof(int32_t), stream);
-      // shadow entries [2], the fetch counters of the next extend [4..5] and of the shadow stage [6..7]
-      if (e == cudaSuccess) e = cudaMemsetAsync(wm.counters + 2, 0, 6 * sizeof(int32_t), stream);
-      if (e != cudaSuccess) return set_error(MJPBR_ERR_CUDA, "path wavefront queue counters: %s", cudaGetErrorString(e));
-      k_shade<<<g_shade, kThreads, 0, stream>>>(s, seed, wm, cur);
+      k_shade<<<g_shade, kThreads, 0, stream>>>(s, seed, wm, parity, it == 0);
       if ((rc = check_launch("ptw_shade_kernel"))) return rc;
-      if (shadows) {
-        k_shadow<<<g_shadow, kThreads, stack, stream>>>(s, wm);
-        if ((rc = check_launch("ptw_shadow_kernel"))) return rc;
-      }
+      // every bounce may ask for shadow rays (lights, environment)
+      k_shadow<<<g_shadow, kThreads, stack, stream>>>(s, wm);
+      if ((rc = check_launch("ptw_shadow_kernel"))) return rc;
     }
     const int64_t npix = (int64_t)wm.nw * pixels;
     k_resolve<<<(unsigned)((npix + kThreads - 1) / kThreads), kThreads, 0, stream>>>(s, wm);
