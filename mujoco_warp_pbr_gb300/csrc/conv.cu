@@ -950,15 +950,21 @@ static int flat_launch(const MjpbrConv& c, const ConvGeom& g, bool by_row, cudaS
   const int32_t nchunk = g.cin / 16, nci = c.c_in / 16, cout = c.c_out;
   auto round256 = [](size_t v) { return (v + 255) / 256 * 256; };
   const size_t wbytes = (size_t)9 * 2 * nchunk * cout * 16;
-  // stages of a block of T tiles: all channels when two such stages fit, else G chunks at a time
+  // Stages of a block of T tiles: all channels when two such stages fit, else a chunk at a time. When every
+  // CTA has one block at most, resident weights would serve it once and its first MMA would wait for all of
+  // them: they come chunk by chunk with the input (16 images of 32 x 32, 64 + 96 -> 64: 23.9 us -> 14.4; 64 -> 64
+  // 12.3 -> 10.3); with more blocks a CTA, residency saves their reload.
+  const int64_t strips = (int64_t)c.nimg * fg.strips;
+  const int32_t sms = conv_sm_count();
   auto plan = [&](int32_t T) {
     fg.T = T;
+    const bool once = !by_row && strips * ((fg.tiles + T - 1) / T) <= sms;
     fg.nrow = (T * 128 + fg.prow) / fg.prow + 3;
     if (fg.nrow > 256) return false;
     fg.plane = fg.nrow * fg.prow * 16;
     fg.in2_off = (int32_t)round256((size_t)2 * nci * fg.plane);
     const size_t whole = round256((size_t)fg.in2_off + (size_t)2 * (nchunk - nci) * fg.plane);
-    if (round256(wbytes) + 2 * whole <= kFlatSmem) {
+    if (!once && round256(wbytes) + 2 * whole <= kFlatSmem) {
       fg.group = 0;
       fg.resident = 1;
       fg.stage_bytes = (int32_t)whole;
@@ -967,7 +973,7 @@ static int flat_launch(const MjpbrConv& c, const ConvGeom& g, bool by_row, cudaS
     } else {
       const size_t abytes = round256((size_t)2 * fg.plane);
       fg.group = 1;
-      fg.resident = round256(wbytes) + 2 * abytes <= kFlatSmem;
+      fg.resident = !once && round256(wbytes) + 2 * abytes <= kFlatSmem;
       fg.b_off = (int32_t)abytes;
       fg.stage_bytes = (int32_t)(abytes + (fg.resident ? 0 : round256((size_t)9 * 2 * cout * 16)));
     }
@@ -977,8 +983,6 @@ static int flat_launch(const MjpbrConv& c, const ConvGeom& g, bool by_row, cudaS
   };
   // the tiles per block that give the busiest CTA the least to do: its blocks' tiles and, per block, about
   // one tile's time for the halo rows and the hand-over; two blocks' accumulators fit tensor memory
-  const int64_t strips = (int64_t)c.nimg * fg.strips;
-  const int32_t sms = conv_sm_count();
   int32_t best = 0;
   int64_t best_cost = INT64_MAX;
   for (int32_t T = std::min(MJPBR_FLAT_TILES, 256 / cout); T >= 1; --T) {
