@@ -12,8 +12,9 @@
 //
 // Bound by instruction issue and fetch: the phases' code together is several times the instruction
 // cache, so a CTA's warps take each phase together (500 x 84 x 84 worlds: 1.42 ms without the barriers,
-// 1.24 with), and a light's rays share one test of the boxes (1.16). 2048 worlds with cameras of 64,
-// 128 and 256 pixels: 29.5 ms; the staged kernels with the same scan take 40.
+// 1.24 with), the more of them the better (1.10 -> 0.87 with CTAs of 512 threads for 256), and a light's
+// rays share one test of the boxes. 2048 worlds with cameras of 64, 128 and 256 pixels: 23.2 ms (28.5 with
+// CTAs of 256); the staged kernels with the same scan take 40.
 #include <algorithm>
 #include <type_traits>
 
@@ -26,14 +27,18 @@
 namespace mjpbr {
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kTile = 16;            // pixel tiles of 16 x 16, addressed in Z order within the tile
 constexpr int32_t kMaxLights = 16;   // shadow counts in shared memory, 1 KB per light
-#ifndef MJPBR_FUSED_CTAS
-#define MJPBR_FUSED_CTAS 3
-#endif
+// CTAs of 512 threads, two an SM, when there are kWideCtas of them per SM and they take no more lanes
+// than CTAs of 256, three an SM: phases taken by twice the warps are fetched half as often, but the
+// work comes in larger pieces. us a frame, 512 / 256 threads: worlds of 64 x 64 with 100 worlds (5 CTAs an
+// SM) 105 / 121, 64 worlds 78 / 80, 32 worlds 51 / 48, one 35 / 30; of 256 x 256 with 8 worlds 105 / 112, 4
+// worlds (3.4 CTAs an SM) 63 / 59; 2000 of 16 x 16, half of whose lanes would idle, 293 / 253.
+constexpr int kWide = 512, kNarrow = 256;
+constexpr int64_t kWideCtas = 4;
+constexpr size_t kFusedSmem = 100 * 1024;
 
-// CTAs of each camera: its tiles times the CTAs per tile.
+// CTAs of each camera: its pixels, tile by tile, kThreads / samples per CTA.
 struct FusedMap {
   int32_t w0;
   int32_t tiles_x[MJPBR_MAX_RENDER];
@@ -45,12 +50,14 @@ MJ_DEV int32_t z_y(int32_t q) { return ((q >> 1) & 1) | ((q >> 2) & 2) | ((q >> 
 
 // A surface parked in shared memory: word k of a thread at base[k * kThreads] (conflict-free).
 constexpr int32_t kSurfaceWords = 14;
+template <int kThreads>
 MJ_DEV void park_surface(float* base, const Surface& sf, V3 normal) {
   const float v[kSurfaceWords] = {sf.base_color.x, sf.base_color.y, sf.base_color.z, sf.metallic, sf.roughness, sf.reflectance, sf.occlusion,
                                   sf.emissive.x, sf.emissive.y, sf.emissive.z, sf.alpha, normal.x, normal.y, normal.z};
 #pragma unroll
   for (int k = 0; k < kSurfaceWords; ++k) base[k * kThreads] = v[k];
 }
+template <int kThreads>
 MJ_DEV Surface take_surface(const float* base, V3* normal) {
   float v[kSurfaceWords];
 #pragma unroll
@@ -68,6 +75,7 @@ MJ_DEV Surface take_surface(const float* base, V3* normal) {
 }
 
 // Shadow visibility from the counts of the thread's shadow rays, one word per light.
+template <int kThreads>
 struct CountedVis {
   const int32_t* counts;
   MJ_DEV float visibility(RtCtx& c, const Light& light, V3, V3, V3, float, uint32_t, int32_t, int32_t, int32_t li) {
@@ -76,10 +84,10 @@ struct CountedVis {
   }
 };
 
-template <bool kTex>
-__global__ void __launch_bounds__(kThreads, MJPBR_FUSED_CTAS) rt_fused_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
-                                                                              const __grid_constant__ FusedMap fm) {
-  using Shade = RtShade<kTex, CountedVis>;
+template <bool kTex, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads == kWide ? 2 : 3) rt_fused_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
+                                                                                       const __grid_constant__ FusedMap fm) {
+  using Shade = RtShade<kTex, CountedVis<kThreads>>;
   extern __shared__ __align__(16) float smem[];
   const int32_t w = fm.w0 + blockIdx.y;
   const MjpbrSettings& st = s.settings;
@@ -104,11 +112,10 @@ __global__ void __launch_bounds__(kThreads, MJPBR_FUSED_CTAS) rt_fused_kernel(co
   while (cam + 1 < s.nrender && (int32_t)blockIdx.x >= fm.cta_base[cam + 1]) ++cam;
   const bool rgb = s.render_rgb[cam] != 0;
   const int32_t n = rgb ? st.samples_per_axis : 1, nn = n * n;
-  const int32_t ppc = kThreads / nn, parts = (kTile * kTile + ppc - 1) / ppc;
-  const int32_t cta = blockIdx.x - fm.cta_base[cam];
-  const int32_t tile = cta / parts;
+  const int32_t ppc = kThreads / nn;
   const int32_t lp = threadIdx.x / nn, smp = threadIdx.x - lp * nn;
-  const int32_t q = (cta - tile * parts) * ppc + lp;
+  const int32_t pos = (blockIdx.x - fm.cta_base[cam]) * ppc + lp;
+  const int32_t tile = pos / (kTile * kTile), q = pos % (kTile * kTile);
   Pixel p;
   p.cam = cam;
   p.width = s.cam_res[cam][0];
@@ -117,7 +124,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_FUSED_CTAS) rt_fused_kernel(co
   p.px = (tile % fm.tiles_x[cam]) * kTile + z_x(q);
   p.py = (tile / fm.tiles_x[cam]) * kTile + z_y(q);
   p.pixelid = p.py * p.width + p.px;
-  const bool active = lp < ppc && q < kTile * kTile && p.px < p.width && p.py < p.height;
+  const bool active = lp < ppc && p.px < p.width && p.py < p.height;
   const bool cull = st.cull_backfaces != 0;
   RtCtx c;
   init_ctx(c, s, blk, L, w, kTex);
@@ -162,7 +169,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_FUSED_CTAS) rt_fused_kernel(co
         point = so + sd * hit.dist;
         cone = cone + spread * hit.dist;
         const Surface sf = eval_surface<false, kTex>(s, blk, L, w, hit, hit.slot, point, sd, cone, &normal);
-        park_surface(parked, sf, normal);
+        park_surface<kThreads>(parked, sf, normal);
         if (seg == 0) {
           albedo = sf.base_color;
           gnormal = normal;
@@ -202,8 +209,8 @@ __global__ void __launch_bounds__(kThreads, MJPBR_FUSED_CTAS) rt_fused_kernel(co
     }
     __syncthreads();
     if (live) {
-      const Surface sf = take_surface(parked, &normal);
-      CountedVis vis{counts};
+      const Surface sf = take_surface<kThreads>(parked, &normal);
+      CountedVis<kThreads> vis{counts};
       const V3 head_dir = -V3{R.m[2], R.m[5], R.m[8]};
       const V3 shaded = Shade::shade_surface(c, vis, sf, point, normal, -sd, head_dir, pseed, 2 * smp + seg);
       if (seg == 1) {
@@ -273,31 +280,36 @@ __global__ void __launch_bounds__(kThreads, MJPBR_FUSED_CTAS) rt_fused_kernel(co
   s.rgb_data[adr] = encode_display(display * inv_nn);
 }
 
-size_t fused_smem(const MjpbrScene& s) {
+size_t fused_smem(const MjpbrScene& s, int32_t threads) {
   const size_t nn = (size_t)s.settings.samples_per_axis * s.settings.samples_per_axis;
   const size_t words = (size_t)stack_entries(s.settings.stack_depth) * 2 + kSurfaceWords + std::max(s.nlight, 0) + (nn > 1 ? 6 : 0);
-  return (size_t)s.world_block_floats * sizeof(float) + words * kThreads * sizeof(float);
+  return (size_t)s.world_block_floats * sizeof(float) + words * threads * sizeof(float);
 }
 
-template <bool kTex>
-int launch_fused(const MjpbrScene& s, uint32_t seed, cudaStream_t stream) {
+FusedMap fused_map(const MjpbrScene& s, int32_t threads) {
   FusedMap fm;
+  fm.w0 = 0;
   fm.cta_base[0] = 0;
   for (int32_t c = 0; c < s.nrender; ++c) {
     const int32_t W = s.cam_res[c][0], H = s.cam_res[c][1];
     const int32_t n = s.render_rgb[c] ? s.settings.samples_per_axis : 1;
-    const int32_t ppc = kThreads / (n * n), parts = (kTile * kTile + ppc - 1) / ppc;
+    const int32_t ppc = threads / (n * n);
     const bool any = s.render_rgb[c] || s.render_depth[c] || s.render_seg[c];
     fm.tiles_x[c] = (W + kTile - 1) / kTile;
-    fm.cta_base[c + 1] = fm.cta_base[c] + (any ? fm.tiles_x[c] * ((H + kTile - 1) / kTile) * parts : 0);
+    const int64_t tiles = (int64_t)fm.tiles_x[c] * ((H + kTile - 1) / kTile);
+    fm.cta_base[c + 1] = fm.cta_base[c] + (any ? (int32_t)((tiles * kTile * kTile + ppc - 1) / ppc) : 0);
   }
-  if (fm.cta_base[s.nrender] == 0) return MJPBR_OK;
-  const size_t smem = fused_smem(s);
-  if (int rc = ensure_smem(reinterpret_cast<const void*>(rt_fused_kernel<kTex>), smem, "fused render")) return rc;
+  return fm;
+}
+
+template <bool kTex, int kThreads>
+int launch_fused(const MjpbrScene& s, uint32_t seed, FusedMap fm, cudaStream_t stream) {
+  const size_t smem = fused_smem(s, kThreads);
+  if (int rc = ensure_smem(reinterpret_cast<const void*>(rt_fused_kernel<kTex, kThreads>), smem, "fused render")) return rc;
   for (int32_t w0 = 0; w0 < s.nworld; w0 += kMaxGridWorlds) {
     fm.w0 = w0;
     const dim3 grid(fm.cta_base[s.nrender], std::min(kMaxGridWorlds, s.nworld - w0));
-    rt_fused_kernel<kTex><<<grid, kThreads, smem, stream>>>(s, seed, fm);
+    rt_fused_kernel<kTex, kThreads><<<grid, kThreads, smem, stream>>>(s, seed, fm);
     if (int rc = check_launch("rt_fused_kernel")) return rc;
   }
   return MJPBR_OK;
@@ -308,12 +320,19 @@ int launch_fused(const MjpbrScene& s, uint32_t seed, cudaStream_t stream) {
 bool fused_supported(const MjpbrScene& s) {
   const bool mesh = s.nmesh + s.nhfield > 0 && s.blas_root != nullptr;
   return !mesh && !s.settings.has_transparency && s.nbvh_geom <= kScanGeoms && s.nlight <= kMaxLights && s.settings.samples_per_axis <= 16 &&
-         fused_smem(s) <= 100 * 1024;
+         fused_smem(s, kNarrow) <= kFusedSmem;
 }
 
 int render_fused_launch(const MjpbrScene& s, uint32_t seed, cudaStream_t stream) {
   const bool tex = s.settings.textures || s.settings.has_env || s.settings.env_background;
-  return tex ? launch_fused<true>(s, seed, stream) : launch_fused<false>(s, seed, stream);
+  const FusedMap wide = fused_map(s, kWide);
+  if (wide.cta_base[s.nrender] == 0) return MJPBR_OK;
+  const FusedMap narrow = fused_map(s, kNarrow);
+  const int64_t nwide = wide.cta_base[s.nrender], nnarrow = narrow.cta_base[s.nrender];
+  if (fused_smem(s, kWide) <= kFusedSmem && nwide * s.nworld >= kWideCtas * device_sm_count() && nwide * kWide <= nnarrow * kNarrow * 9 / 8) {
+    return tex ? launch_fused<true, kWide>(s, seed, wide, stream) : launch_fused<false, kWide>(s, seed, wide, stream);
+  }
+  return tex ? launch_fused<true, kNarrow>(s, seed, narrow, stream) : launch_fused<false, kNarrow>(s, seed, narrow, stream);
 }
 
 }  // namespace mjpbr

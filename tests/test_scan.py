@@ -102,3 +102,16 @@ def test_path_scan_matches_the_bvh(ngeom, mesh):
   got = images(sc, schedule="wavefront", **options)
   for key in ("rgb", "depth", "seg", "hdr"):
     np.testing.assert_array_equal(got[key], ref[key], err_msg=key)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("nworld,samples", [(210, 1), (60, 2), (25, 3), (3, 16)])
+def test_large_frames_match_the_bvh(nworld, samples):
+  """Frames of at least four 512-thread CTAs per SM are rendered by them: the same images, at sample counts that
+  divide 512 and 256 and one that divides neither."""
+  sc = scene(9, mirror=True, nworld=nworld)
+  ref = images(sc, schedule="queue", samples_per_pixel=samples)
+  got = images(sc, schedule="wavefront", samples_per_pixel=samples)
+  for key in ("rgb", "depth", "seg", "hdr"):
+    np.testing.assert_array_equal(got[key], ref[key], err_msg=key)
