@@ -6,9 +6,10 @@
 //                 depth / segmentation of the pixel from its first sample
 //   2. surface 0  eval_surface at the primary hit -> surface record; every light the shading will
 //                 ask about appends one shadow entry, a reflective surface one mirror ray
-//   3. mirror     closest hit of every queued mirror ray -> hit record (persistent; lanes take a
-//                 new ray as soon as theirs is done: refill.cuh)
-//   4. surface 1  eval_surface at the mirror hit -> surface record, shadow entries
+//   3. mirror     closest hit of every queued mirror ray -> hit record, hits listed (persistent; lanes take a
+//                 new ray as soon as theirs is done: refill.cuh). Scenes of few geoms: the primitives by the
+//                 warp-wide scan (scan.cuh), then the listed rays' meshes, a kernel each
+//   4. surface 1  eval_surface at the listed mirror hits -> surface record, shadow entries
 //   5. shadow     every shadow entry's rays (any hit, persistent with lane refill) -> count of
 //                 unoccluded rays
 //   6. resolve    one thread per camera sample: the shading of both segments with the stored
@@ -24,7 +25,7 @@
 // with the shadow visibility read from the counts instead of traced where it is needed, and the
 // rays of stages 3-5 are set up by the same functions, so the images are bit-identical to the
 // megakernel's. Translucent layers are not staged: contexts with has_transparency render with the
-// megakernel.
+// megakernel. Scenes of few geoms without meshes need no stages at all (render_fused.cu).
 //
 // Scratch (MjpbrScene.wave_scratch): per sample of a chunk two hit records (32 B), two surface
 // records (64 B), a mirror queue entry (48 B) and per model light two visibility counts (8 B) and
@@ -398,6 +399,8 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_SHADE_CTAS) wave_surface_
 #define MJPBR_WAVE_REFILL_STEPS 32
 #endif
 // Idle lanes before a warp of the scanned stages fetches again.
+// Idle lanes before a warp of the mirror rays' mesh stage fetches again (voted_loop).
+constexpr int32_t kVoteIdle = 16;
 #ifndef MJPBR_SCAN_MIN_IDLE
 #define MJPBR_SCAN_MIN_IDLE 8
 #endif
@@ -503,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_
   ClosestWalk q;
   const float* blk = nullptr;
   int32_t sample = -1, entry = -1;
-  refill_loop<MJPBR_WAVE_REFILL_STEPS>(
+  voted_loop<kVoteIdle>(
       items, reinterpret_cast<unsigned long long*>(wm.counters + 4), q,
       [&](int64_t item, ClosestWalk& qq) {
         entry = wm.mirror[item].index.y;
@@ -528,6 +531,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_
         qq.m.code = -1;
         return true;
       },
+      [&](const ClosestWalk& qq) { return walk_kind(qq.m); },
       [&](ClosestWalk& qq) { return walk_closest_step(qq, s, st, blk, L, cull, &err); },
       [&](ClosestWalk& qq, int32_t) {
         if (qq.tie) qq.h = trace_ray<true>(s, st, blk, L, qq.m.r, kMaxVal, cull, false, &err);

@@ -256,6 +256,9 @@ struct MeshWalk {
   float cut;        // hits at or past it do not count
 };
 
+// What a walk's next step does: 0 visits a node, 1 a leaf, 2 ends a mesh and takes the next.
+MJ_DEV int32_t walk_kind(const MeshWalk& q) { return q.code < 0 ? 2 : ((q.code & 7) != 0 ? 1 : 0); }
+
 MJ_DEV void walk_next(MeshWalk& q, const MjpbrScene& sc, const float* blk, const BlockLayout& L) {
   const int32_t slot = __ffs(q.meshes) - 1;
   q.meshes &= q.meshes - 1u;
