@@ -11,6 +11,8 @@ import ctypes
 import threading
 from pathlib import Path
 
+import torch
+
 LIBRARY = Path(__file__).resolve().parent / "libmjpbr.so"
 ABI_VERSION = 3
 MAX_RENDER = 16
@@ -451,6 +453,14 @@ def _lib_or_raise() -> ctypes.CDLL:
   if _lib is None:
     raise RuntimeError("libmjpbr is not loaded")
   return _lib
+
+
+def current_stream(device: torch.device) -> int:
+  """The device's current stream, as torch.cuda.current_stream(device).cuda_stream without the Stream
+  object (0.2 us for 3; a small frame asks five times). A CUDA tensor on the device has initialised CUDA."""
+  if device.type != "cuda" or device.index is None:
+    return torch.cuda.current_stream(device).cuda_stream
+  return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def call(name: str, *args) -> None:

@@ -190,7 +190,7 @@ class KPCN:
 
   # ---------------------------------------------------------------- primitives
   def _stream(self) -> int:
-    return torch.cuda.current_stream(self.device).cuda_stream
+    return _lib.current_stream(self.device)
 
   def _conv(self, name: str, x: torch.Tensor, out: torch.Tensor | None, x2: torch.Tensor | None = None, out_f32: torch.Tensor | None = None) -> None:
     """x2: the skip input at the resolution of x (already upsampled)."""

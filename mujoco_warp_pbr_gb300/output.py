@@ -30,11 +30,11 @@ def _scene(rc: PbrRenderContext) -> _lib.Scene:
   cached = rc._host_cache.get("scene")
   if cached is None:
     raise ValueError("render the context before reading its outputs")
-  return cached[2]
+  return cached[1]
 
 
 def _stream(rc: PbrRenderContext) -> int:
-  return torch.cuda.current_stream(rc.device).cuda_stream
+  return _lib.current_stream(rc.device)
 
 
 def get_rgb(rc: PbrRenderContext, camera_index: int, rgb_out: torch.Tensor) -> None:

@@ -10,6 +10,7 @@ like the reference's launch-input cache, mujoco_warp_pbr/_src/launch.py:89-115).
 
 from __future__ import annotations
 
+import operator
 import warnings
 from typing import Any
 
@@ -248,28 +249,26 @@ def scene_fields(m: Any, d: Any, rc: PbrRenderContext) -> dict[str, Any]:
 
 
 def _sources(m: Any, d: Any, rc: PbrRenderContext) -> tuple:
-  public = [v for k, v in vars(rc).items() if not k.startswith("_")]
+  public = [v for k, v in vars(rc).items() if k[0] != "_"]
   return (*vars(m).values(), *vars(d).values(), *public, *vars(rc.base).values())
 
 
 def scene(m: Any, d: Any, rc: PbrRenderContext) -> _lib.Scene:
   """The (cached) MjpbrScene of a frame."""
   sources = _sources(m, d, rc)
-  ids = tuple(map(id, sources))
   cached = rc._host_cache.get("scene")
-  if cached is not None and cached[1] == ids:
-    return cached[2]
+  if cached is not None and len(cached[0]) == len(sources) and all(map(operator.is_, cached[0], sources)):
+    return cached[1]
   _check_env_id(rc)
   _warn_ignored_overrides(m, rc)
   fields = scene_fields(m, d, rc)
   struct = _scene.fill_scene(fields)
   if _ensure_wave_scratch(rc, struct):
     sources = _sources(m, d, rc)
-    ids = tuple(map(id, sources))
     fields = scene_fields(m, d, rc)
     struct = _scene.fill_scene(fields)
   # the cache holds the sources and the converted tensors so their addresses stay valid
-  rc._host_cache["scene"] = (sources, ids, struct, fields)
+  rc._host_cache["scene"] = (sources, struct, fields)
   return struct
 
 
@@ -351,7 +350,7 @@ def _check_env_id(rc: PbrRenderContext) -> None:
 
 
 def _stream(rc: PbrRenderContext) -> int:
-  return torch.cuda.current_stream(rc.device).cuda_stream
+  return _lib.current_stream(rc.device)
 
 
 def refit_bvh(m: Any, d: Any, rc: PbrRenderContext) -> None:

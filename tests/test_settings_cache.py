@@ -163,3 +163,16 @@ def test_override_warning_rules():
     _warn_ignored_overrides(_M(half.clone()), rc)
     rc.mat_reflectance = torch.tensor([[0.5, 0.3]])
     _warn_ignored_overrides(_M(half.clone()), rc)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("side", [False, True])
+def test_launches_follow_the_current_stream(side):
+  from mujoco_warp_pbr_gb300 import _lib
+
+  device = torch.device("cuda", torch.cuda.current_device())
+  with torch.cuda.stream(torch.cuda.Stream(device) if side else torch.cuda.default_stream(device)):
+    expected = torch.cuda.current_stream(device).cuda_stream
+    assert _lib.current_stream(device) == expected
+    assert _lib.current_stream(torch.device("cuda")) == expected
