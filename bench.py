@@ -551,7 +551,7 @@ def run(args) -> None:
     if args.workload == "path":
       kernel = "path wavefront: ptw_first_extend, ptw_extend, ptw_shade, ptw_shadow, ptw_resolve per chunk, one frame"
     elif wave:
-      kernel = "wavefront render: wave_primary, wave_surface, wave_mirror, wave_mirror_surface, wave_shadow, wave_resolve per chunk, one frame"
+      kernel = "wavefront render: wave_primary, wave_surface, wave_mirror (scan, mesh), wave_mirror_surface, wave_shadow, wave_resolve per chunk, one frame"
     else:
       kernel = "rt_kernel"
     line = {
@@ -638,6 +638,8 @@ def render_launches(rc, chunks: int, nlight: int) -> int:
     return 1
   rgb = any(rc.base.render_rgb)
   per = 1 + (2 if rgb else 0) + (2 if rgb and rc.has_reflection else 0)
+  if rgb and rc.has_reflection and rc.enabled_geom_ids.shape[0] <= 32:
+    per += 1  # the mirror rays' meshes, apart from their primitives
   if rgb and rc.use_shadows and nlight > 0:
     per += 1
   return per * max(chunks, 1)

@@ -4,11 +4,12 @@
 //
 //   geometry depth / segmentation of cameras without RGB (one ray per pixel)
 //   per bounce, over the queue of live paths:
-//     extend   closest hit of every path (persistent, lanes refilled from the queue: refill.cuh);
+//     extend   closest hit of every path (scenes of few geoms by the warp-wide scan, scan.cuh; meshes and
+//              larger scenes with lanes refilled from the queue: refill.cuh), hits and misses queued apart;
 //              depth / segmentation from sample 0's first hit; the first bounce's extend starts
 //              the paths itself, one per (pixel, sample) of the RGB cameras (pt_bounce.cuh
 //              start_sample), and writes each path record once, after its hit
-//     shade    the bounce after the hit (PtCore::surface): emission, mirror lobe, next-event
+//     shade    the bounce after the hit (PtCore's phases, taken by a CTA's warps together): emission, mirror lobe, next-event
 //              estimation recorded per path (each light's unshadowed contribution, the environment
 //              sample's term) with each shadow ray appended to the shadow queue as it is recorded
 //              (one atomic per group of converged lanes), the BSDF sample and Russian roulette;
