@@ -59,7 +59,10 @@ constexpr int kTile = 16;  // pixel tiles of 16 x 16, addressed in Z order withi
 #ifndef MJPBR_WAVE_MIRROR_CTAS
 #define MJPBR_WAVE_MIRROR_CTAS 3
 #endif
-constexpr int kMirrorScanCtas = 4;
+// The scanned stages run better at four (64 registers; they hold no traversal state while they scan): 1024
+// mesh worlds of 128 x 128 with 2 x 2 samples, primary 7.84 -> 7.56 ms, shadow 5.70 -> 5.31, and 300
+// terrain worlds of 96 x 96, 0.85 -> 0.76 and 1.43 -> 1.33; at two 8.9 and 7.5.
+constexpr int kScanCtas = 4;
 #ifndef MJPBR_WAVE_SHADE_CTAS
 #define MJPBR_WAVE_SHADE_CTAS 3
 #endif
@@ -285,7 +288,7 @@ MJ_DEV void emit_shadows(const MjpbrScene& s, const WaveMap& wm, const float* bl
 
 // ---------------------------------------------------------------- 1. primary rays
 template <bool kMesh, bool kStaged, bool kScan>
-__global__ void __launch_bounds__(kThreads, MJPBR_WAVE_TRACE_CTAS) wave_primary_kernel(const __grid_constant__ MjpbrScene s,
+__global__ void __launch_bounds__(kThreads, kScan ? kScanCtas : MJPBR_WAVE_TRACE_CTAS) wave_primary_kernel(const __grid_constant__ MjpbrScene s,
                                                                 const __grid_constant__ WaveMap wm) {
   extern __shared__ __align__(16) float smem[];
   const int32_t w = wm.w0 + blockIdx.y;
@@ -475,7 +478,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_
 // The first is bound by the latency of the entries and world blocks (4.8 warps of 9 waited for loads, 3.6
 // at barriers): its lists are appended by warps, without barriers, and it runs four CTAs an SM (1024 mesh
 // worlds of 128 x 128, 2 x 2 samples: 3.7 -> 3.1 ms by warps, 2.75 at four CTAs; 3.05 at five).
-__global__ void __launch_bounds__(kThreads, kMirrorScanCtas) wave_mirror_scan_kernel(const __grid_constant__ MjpbrScene s,
+__global__ void __launch_bounds__(kThreads, kScanCtas) wave_mirror_scan_kernel(const __grid_constant__ MjpbrScene s,
                                                                                             const __grid_constant__ WaveMap wm) {
   extern __shared__ __align__(16) float smem[];
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
@@ -653,7 +656,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_TRACE_CTAS) wave_shadow_k
 
 // The shadow stage of scanned scenes (scan.cuh): the primitives when a ray is fetched, its meshes
 // resumably.
-__global__ void __launch_bounds__(kThreads, MJPBR_WAVE_TRACE_CTAS) wave_shadow_scan_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
+__global__ void __launch_bounds__(kThreads, kScanCtas) wave_shadow_scan_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
                                                                                            const __grid_constant__ WaveMap wm) {
   extern __shared__ __align__(16) float smem[];
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
