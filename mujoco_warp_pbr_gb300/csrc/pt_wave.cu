@@ -60,6 +60,11 @@ constexpr int kThreads = 256;
 #define MJPBR_PTW_TEX_CTAS 3
 #endif
 
+// Resident CTAs per SM of the scanned trace stages (scan.cuh): they wait for path records and world blocks
+// more than they need registers. 1024 x 128 x 128 paths at three, four and five: extend 3.08, 2.67, 2.64 ms;
+// two 256 x 256 cameras of 128 worlds 2.60, 2.30, 2.25 and, the first extend, 2.11, 2.03, 2.09.
+constexpr int kScanCtas = 4;
+
 // A path between stages: 80 bytes every bounce reads and writes, and the first surface's denoiser
 // features (48 bytes), written by the bounces of a camera ray. Each 16-byte field is an array of its own
 // over the paths of the chunk, so that a warp's lanes, on neighbouring paths, move whole lines.
@@ -425,7 +430,7 @@ MJ_DEV void closest_queue(const MjpbrScene& s, const Stack& st, const BlockLayou
 // the queue, with them the meshes are traced resumably, lanes refilled from the queue (refill.cuh);
 // larger scenes walk the scene BVH resumably.
 template <bool kMesh, bool kScan>
-__global__ void __launch_bounds__(kThreads, 3) ptw_extend_kernel(const __grid_constant__ MjpbrScene s,
+__global__ void __launch_bounds__(kThreads, kScan ? kScanCtas : 3) ptw_extend_kernel(const __grid_constant__ MjpbrScene s,
                                                                  const __grid_constant__ PtWaveMap wm, int32_t parity) {
   extern __shared__ __align__(16) float smem[];
   const Stack st = wave_stack(s, smem);
@@ -473,7 +478,7 @@ __global__ void __launch_bounds__(kThreads, 3) ptw_extend_kernel(const __grid_co
 // it is traced (start_sample, pt_bounce.cuh) and the path record written once, after the hit. The shade
 // stage takes the paths in their own order: neighbouring camera rays mostly hit or miss together.
 template <bool kMesh, bool kScan>
-__global__ void __launch_bounds__(kThreads, 3) ptw_first_extend_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
+__global__ void __launch_bounds__(kThreads, kScan ? kScanCtas : 3) ptw_first_extend_kernel(const __grid_constant__ MjpbrScene s, uint32_t seed,
                                                                        const __grid_constant__ PtWaveMap wm) {
   extern __shared__ __align__(16) float smem[];
   const Stack st = wave_stack(s, smem);
@@ -593,7 +598,7 @@ __global__ void __launch_bounds__(kThreads, kTex ? MJPBR_PTW_TEX_CTAS : MJPBR_PT
 // Any hit of every recorded shadow ray: scanned (scan.cuh; without meshes the lanes stride over the
 // queue) or, past kScanGeoms geoms, by the scene BVH, lanes refilled from the queue (refill.cuh).
 template <bool kMesh, bool kScan>
-__global__ void __launch_bounds__(kThreads, 3) ptw_shadow_kernel(const __grid_constant__ MjpbrScene s,
+__global__ void __launch_bounds__(kThreads, kScan ? kScanCtas : 3) ptw_shadow_kernel(const __grid_constant__ MjpbrScene s,
                                                                  const __grid_constant__ PtWaveMap wm) {
   extern __shared__ __align__(16) float smem[];
   const BlockLayout L = block_layout(s.nbvh_geom, s.nnode, s.nlight, s.nrender);
