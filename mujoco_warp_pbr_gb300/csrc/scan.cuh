@@ -15,9 +15,9 @@
 // (128 x 128, 2 x 2 samples) 11.0 -> 7.8 ms, 300 terrain worlds (96 x 96) 3.96 -> 2.92 ms a frame.
 //
 // kScanGeoms = 32: one mask word, and the scan is the faster of the two up to there (256 worlds of
-// 128 x 128, ms a frame, scan / BVH): primitives 0.79 / 1.53 at 4 geoms, 1.52 / 1.73 at 17, 1.96 /
-// 2.09 at 32; with a third of them meshes 1.80 / 1.87, 3.24 / 3.78 and 4.39 / 5.26; path-traced 9.61 /
-// 9.84 and with meshes 23.4 / 25.1 at 32. The leaf boxes are read from the scene BVH's nodes (each child
+// 128 x 128, ms a frame, scan / BVH): primitives 0.63 / 1.53 at 4 geoms, 1.13 / 1.72 at 17, 1.47 /
+// 2.08 at 32; with a third of them meshes 1.85 / 1.84, 3.02 / 3.71 and 4.17 / 5.19; path-traced 7.48 /
+// 9.37 and with meshes 23.4 / 25.9 at 32. The leaf boxes are read from the scene BVH's nodes (each child
 // of a node with count 1 is a leaf; hidden geoms have none), whose bounds the leaf's ancestors
 // contain, so the boxes that pass are those the traversal reaches.
 #pragma once
