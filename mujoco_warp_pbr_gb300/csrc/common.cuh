@@ -75,6 +75,7 @@ MJ_HD V3 vmax(V3 a, V3 b) { return V3{fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.
 MJ_HD V3 vmin(V3 a, V3 b) { return V3{fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z)}; }
 MJ_HD float clampf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
 MJ_HD float vmax3(V3 a) { return fmaxf(a.x, fmaxf(a.y, a.z)); }
+MJ_HD V3 vabs(V3 a) { return V3{fabsf(a.x), fabsf(a.y), fabsf(a.z)}; }
 
 // Shading-only fused helpers.
 MJ_DEV float fdot(V3 a, V3 b) { return __fmaf_rn(a.x, b.x, __fmaf_rn(a.y, b.y, a.z * b.z)); }

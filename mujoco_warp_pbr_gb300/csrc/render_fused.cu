@@ -12,9 +12,10 @@
 //
 // Bound by instruction issue and fetch: the phases' code together is several times the instruction
 // cache, so a CTA's warps take each phase together (500 x 84 x 84 worlds: 1.42 ms without the barriers,
-// 1.24 with), the more of them the better (1.10 -> 0.87 with CTAs of 512 threads for 256), and a light's
-// rays share one test of the boxes. 2048 worlds with cameras of 64, 128 and 256 pixels: 23.2 ms (28.5 with
-// CTAs of 256); the staged kernels with the same scan take 40.
+// 1.24 with), the more of them the better (1.10 -> 0.87 with CTAs of 512 threads for 256), and a bulb's
+// rays test only the boxes around its centre's ray (500 x 84 x 84: 942 us a frame with one test for all of a
+// light's rays, 930 so). 2048 worlds with cameras of 64, 128 and 256 pixels: 23.2 ms (28.5 with CTAs of 256); the
+// staged kernels with the same scan take 40.
 #include <algorithm>
 #include <type_traits>
 
@@ -186,23 +187,29 @@ __global__ void __launch_bounds__(kThreads, kThreads == kWide ? 2 : 3) rt_fused_
         float dist;
         if (!light.active || !shadow_setup(st, light, point, normal, &l, &dist)) continue;
         const int32_t rays = shadow_ray_count(light, ns);
-        // the rays to a bulb's disc share the boxes around the ray to its centre: positions along it in
-        // fractions of the way, so that a ray to a point of the disc is at most the bulb's radius off
-        uint32_t around = 0;
+        // a bulb's rays test only the boxes around the ray to its centre: positions along it in fractions of the
+        // way, so that a ray to a point of the disc is at most the bulb's radius off, and the rounding of
+        // both box tests, some ulp of the coordinates, further
+        uint32_t around = slots.valid;
         if (rays > 1) {
           const V3 to = light.pos - origin;
-          around = slots.mask_around(scan_inv(Ray{origin, to}), 1.0f + kRayTolRel, fabsf(light.bulbradius) * 1.001f + 1.0e-5f);
+          const float rounding = 1.0e-6f * (vmax3(vabs(origin)) + vmax3(vabs(to)) + fabsf(light.bulbradius));
+          around = slots.mask_around(origin, to, 1.0f + kRayTolRel, fabsf(light.bulbradius) * 1.001f + 1.0e-5f + rounding);
         }
         int32_t visible = 0;
+        if (around == 0) {
+          visible = rays;
+        } else {
 #pragma unroll 1
-        for (int32_t k = 0; k < rays; ++k) {
-          Ray r;
-          float len;
-          r.o = origin;
-          shadow_ray(light, ns, origin, l, dist, pseed, 2 * smp + seg, L.nlight, li, k, &r.d, &len);
-          uint32_t meshes;
-          const uint32_t mask = rays > 1 ? around : slots.mask(scan_inv(r), len * (1.0f + kRayTolRel) + kRayTolAbs);
-          if (!scan_any<false>(mask, blk, L, r, len, cull, &meshes)) ++visible;
+          for (int32_t k = 0; k < rays; ++k) {
+            Ray r;
+            float len;
+            r.o = origin;
+            shadow_ray(light, ns, origin, l, dist, pseed, 2 * smp + seg, L.nlight, li, k, &r.d, &len);
+            uint32_t meshes;
+            const uint32_t mask = SlotBoxes{slots.box, around}.mask(make_inv(r), len * (1.0f + kRayTolRel) + kRayTolAbs);
+            if (!scan_any<false>(mask, blk, L, r, len, cull, &meshes)) ++visible;
+          }
         }
         counts[li * kThreads] = visible;
       }

@@ -32,15 +32,10 @@ constexpr int32_t kScanGeoms = 32;
 // tolerance, and past the traversal's cut-off.
 MJ_DEV float scan_window(float dist) { return 2.5f * kRayTolRel * fmaxf(dist, 1.0f); }
 
-// Reciprocal direction of the box tests. The boxes are padded by 1e-5 of their coordinates, a
-// hundred times what the approximate reciprocal moves a slab by.
-MJ_DEV RayInv scan_inv(const Ray& r) {
-  auto rcp = [](float x) { return approx_rcp(fabsf(x) > 1.0e-30f ? x : (x >= 0.0f ? 1.0e-30f : -1.0e-30f)); };
-  RayInv ri;
-  ri.inv = V3{rcp(r.d.x), rcp(r.d.y), rcp(r.d.z)};
-  ri.oinv = cmul(r.o, ri.inv);
-  return ri;
-}
+// The box tests are trace_ray's, reciprocals included (make_inv). An approximate reciprocal moves a slab by
+// 1e-7 of its distance, which the boxes' padding, 1e-5 of their own coordinates, covers only near them: 5 of
+// 204,800 camera rays from 4 km at axis-aligned boxes lost their hit by it. Three divisions a ray cost less
+// than 1 % of a frame.
 
 // The geoms a ray may hit before cut, as a mask of slots, from the scene BVH's nodes in a world block.
 struct NodeBoxes {
@@ -81,9 +76,13 @@ struct SlotBoxes {
     }
     return mask;
   }
-  // The slots any ray from the same origin to within `radius` of this ray's end may hit: on its way
-  // such a ray stays within radius of this one.
-  MJ_DEV uint32_t mask_around(const RayInv& ri, float cut, float radius) const {
+  // The slots any ray from o to within `radius` of o + to may hit: on its way such a ray stays within radius
+  // of this one. radius has to cover the rounding of the tests too, the approximate reciprocals' among it.
+  static MJ_DEV float around_rcp(float x) { return approx_rcp(fabsf(x) > 1.0e-30f ? x : (x >= 0.0f ? 1.0e-30f : -1.0e-30f)); }
+  MJ_DEV uint32_t mask_around(V3 o, V3 to, float cut, float radius) const {
+    RayInv ri;
+    ri.inv = V3{around_rcp(to.x), around_rcp(to.y), around_rcp(to.z)};
+    ri.oinv = cmul(o, ri.inv);
     const float gx = radius * fabsf(ri.inv.x), gy = radius * fabsf(ri.inv.y), gz = radius * fabsf(ri.inv.z);
     uint32_t mask = 0;
 #pragma unroll 1
@@ -159,7 +158,7 @@ MJ_DEV uint32_t scan_closest(Hit& h, bool& tie, const Boxes& boxes, const float*
   h.face = -1;
   h.mesh = -1;
   tie = false;
-  const uint32_t mask = boxes.mask(scan_inv(r), max_dist * (1.0f + kRayTolRel) + kRayTolAbs);
+  const uint32_t mask = boxes.mask(make_inv(r), max_dist * (1.0f + kRayTolRel) + kRayTolAbs);
   uint32_t meshes = 0;
   for (uint32_t todo = scan_union(mask); todo; todo &= todo - 1u) {
     const int32_t slot = __ffs(todo) - 1;
@@ -237,7 +236,7 @@ MJ_DEV bool scan_any(uint32_t mask, const float* blk, const BlockLayout& L, cons
 
 template <bool kMesh>
 MJ_DEV bool scan_any(const float* blk, const BlockLayout& L, const Ray& r, float max_dist, bool cull, uint32_t* meshes) {
-  return scan_any<kMesh>(NodeBoxes{blk, &L}.mask(scan_inv(r), max_dist * (1.0f + kRayTolRel) + kRayTolAbs), blk, L, r, max_dist, cull, meshes);
+  return scan_any<kMesh>(NodeBoxes{blk, &L}.mask(make_inv(r), max_dist * (1.0f + kRayTolRel) + kRayTolAbs), blk, L, r, max_dist, cull, meshes);
 }
 
 // ---------------------------------------------------------------- resumable mesh part

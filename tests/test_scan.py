@@ -115,3 +115,35 @@ def test_large_frames_match_the_bvh(nworld, samples):
   got = images(sc, schedule="wavefront", samples_per_pixel=samples)
   for key in ("rgb", "depth", "seg", "hdr"):
     np.testing.assert_array_equal(got[key], ref[key], err_msg=key)
+
+
+def far_scene(distance, mesh, nworld=8, res=160):
+  """Axis-aligned boxes around the origin (every third geom a mesh of one) seen, and lit, from `distance` metres
+  away. Their silhouettes are their leaf boxes': rays pass them by less than the rounding of the distance, and a
+  box test that rounds otherwise loses hits."""
+  sc = scene(17, mesh=mesh, nworld=nworld)
+  boxes = sc.mjm.geom_type != synthetic.GEOM_MESH
+  boxes[0] = False
+  sc.mjm.geom_type[boxes] = synthetic.GEOM_BOX
+  sc.mjd.geom_xmat[:, boxes] = np.eye(3, dtype=np.float32).reshape(9)
+  eye = np.array([0.3, -0.8, 0.5]) * distance
+  sc.mjm.cam_fovy[:] = np.degrees(2.0 * np.arctan(1.3 / np.linalg.norm(eye)))
+  sc.mjd.cam_xpos[:] = eye
+  sc.mjd.cam_xmat[:] = synthetic.look_at(eye, np.array([0.0, 0.0, 0.4])).reshape(9)
+  sc.mjd.light_xpos[:, 1] = (0.2 * distance, 0.3 * distance, 0.9 * distance)
+  sc.options["cam_res"] = (res, res)
+  return sc
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("mesh", [False, True])
+@pytest.mark.parametrize("distance", [50.0, 400.0, 4000.0])
+def test_far_cameras_match_the_bvh(distance, mesh):
+  sc = far_scene(distance, mesh)
+  for options, schedule in (({}, "queue"), ({"tier": 1, "path_samples": 1, "max_depth": 1}, "grid")):
+    ref = images(sc, schedule=schedule, **options)
+    got = images(sc, schedule="wavefront", **options)
+    assert (ref["seg"][..., 0] > 0).mean() > 0.1
+    for key in ("rgb", "depth", "seg", "hdr"):
+      np.testing.assert_array_equal(got[key], ref[key], err_msg=key)
