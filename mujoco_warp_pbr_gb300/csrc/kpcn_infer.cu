@@ -82,9 +82,11 @@ int conv(const MjpbrKpcnWeights& wts, int32_t k, const uint16_t* in, const uint1
 }
 
 // The U-Net forward pass of kpcn.KPCN.forward on ws.x0; its kernels applied to `radiance` into `out`, images
-// `stride` pixels apart (the denoiser's own buffers, read and written in place).
-int forward(const MjpbrKpcnWeights& wts, const Workspace& ws, const float* radiance, float* out, int64_t stride, int32_t n, int32_t h, int32_t w,
-            int32_t* err, cudaStream_t st) {
+// `stride` pixels apart (the denoiser's own buffers, read and written in place). Where the two overlap, the
+// kernels read a copy (a pixel's 5 x 5 neighbours may be written by then), in place of the network's input,
+// which is twice its size and consumed.
+int forward(const MjpbrKpcnWeights& wts, const Workspace& ws, const float* radiance, float* out, int64_t stride, bool overlap, int32_t n, int32_t h,
+            int32_t w, int32_t* err, cudaStream_t st) {
   int rc = 0;
   auto c = [&](int32_t k, const uint16_t* in, uint16_t* out, const uint16_t* in2 = nullptr, float* out_f32 = nullptr) {
     if (!rc) rc = conv(wts, k, in, in2, out, out_f32, n, h, w, err, st);
@@ -116,8 +118,16 @@ int forward(const MjpbrKpcnWeights& wts, const Workspace& ws, const float* radia
   c(12, ws.s0, ws.u0, ws.up0);
   c(13, ws.u0, ws.v0);
   c(14, ws.v0, nullptr, nullptr, ws.logits);
-  if (!rc) rc = kpcn_apply_launch(ws.logits, radiance, nullptr, out, n, h, w, stride, stride, st);
-  return rc;
+  if (rc) return rc;
+  int64_t radiance_stride = stride;
+  if (overlap) {
+    const size_t bytes = (size_t)h * w * 16;
+    const cudaError_t e = cudaMemcpy2DAsync(ws.x0, bytes, radiance, (size_t)stride * 16, bytes, n, cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) return set_error(MJPBR_ERR_CUDA, "denoise_learned: radiance copy: %s", cudaGetErrorString(e));
+    radiance = reinterpret_cast<const float*>(ws.x0);
+    radiance_stride = (int64_t)h * w;
+  }
+  return kpcn_apply_launch(ws.logits, radiance, nullptr, out, n, h, w, radiance_stride, stride, st);
 }
 
 }  // namespace
@@ -136,6 +146,8 @@ int denoise_learned_launch(const MjpbrScene& s, const MjpbrKpcnWeights& wts, voi
   for (int32_t k = 0; k < MJPBR_KPCN_LAYERS; ++k) {
     if (!wts.weight[k] || !wts.bias[k]) return set_error(MJPBR_ERR_ARG, "denoise_learned: layer %d has no weights", k);
   }
+  const int64_t floats = (int64_t)s.nworld * s.rgb_stride * 4;
+  const bool overlap = s.denoise_buffers[0] < s.denoise_buffers[1] + floats && s.denoise_buffers[1] < s.denoise_buffers[0] + floats;
   for (int32_t cam = 0; cam < s.nrender; ++cam) {
     if (!s.render_rgb[cam]) continue;
     const int32_t w = s.cam_res[cam][0], h = s.cam_res[cam][1];
@@ -150,7 +162,7 @@ int denoise_learned_launch(const MjpbrScene& s, const MjpbrKpcnWeights& wts, voi
       int rc = kpcn_features_launch(s, cam, w0, nw, ws.x0, st);
       if (rc) return rc;
       const int64_t first = ((int64_t)w0 * s.rgb_stride + s.rgb_adr[cam]) * 4;
-      rc = forward(wts, ws, s.denoise_buffers[0] + first, s.denoise_buffers[1] + first, s.rgb_stride, nw, h, w, s.error_word, st);
+      rc = forward(wts, ws, s.denoise_buffers[0] + first, s.denoise_buffers[1] + first, s.rgb_stride, overlap, nw, h, w, s.error_word, st);
       if (rc) return rc;
     }
   }

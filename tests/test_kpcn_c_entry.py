@@ -64,3 +64,35 @@ def test_c_entry_matches_the_python_denoiser():
   # a workspace one byte short and a chunk of zero are rejected before any launch
   assert lib.mjpbr_denoise_learned(ctypes.byref(scene), ctypes.byref(wts), ctypes.c_void_p(ws.data_ptr()), nbytes - 1, 4, stream) == _lib.ERR_ARG
   assert lib.mjpbr_denoise_learned(ctypes.byref(scene), ctypes.byref(wts), ctypes.c_void_p(ws.data_ptr()), nbytes, 0, stream) == _lib.ERR_ARG
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+def test_one_buffer_for_radiance_and_result():
+  """A caller may give the same buffer for the radiance and the filtered radiance (denoise_buffers[0] and [1]): the
+  images are those of two buffers."""
+  from pathlib import Path
+
+  import mujoco_warp_pbr_gb300 as mjpbr
+  from mujoco_warp_pbr_gb300 import kpcn, synthetic
+  from tests import helpers
+
+  sc = synthetic.path_scene(seed=4, nworld=6, res=128, ncam=2)
+  m, d, rc = helpers.gpu_scene(sc, denoise=True)
+  net = kpcn.KPCN.load(Path(kpcn.__file__).resolve().parent / "weights" / "kpcn_path.npz")
+  two = rc.denoise_buffers
+
+  def frame():
+    rc.base.rgb_data.zero_()
+    mjpbr.refit_bvh(m, d, rc)
+    mjpbr.render(m, d, rc, seed=3, denoise=False)
+    net.denoise(m, d, rc, chunk=4)
+    torch.cuda.synchronize()
+    assert mjpbr.check_errors(rc) == 0
+    return rc.base.rgb_data.cpu().numpy().copy(), rc.hdr_data.cpu().numpy().copy()
+
+  ref = frame()
+  rc.denoise_buffers = (two[0], two[0])
+  got = frame()
+  for a, b in zip(got, ref):
+    np.testing.assert_array_equal(a, b)
