@@ -281,9 +281,10 @@ MJ_HD void box_axis(float lp, float lv, float sz, float* tn, float* tf, float* e
 // The six face crossings of ray_box_faces cost a division and two face tests each, and nearly every
 // ray misses the box or enters it well inside one face: the estimated crossings of the three slabs
 // decide those by a margin, and only the entered face is computed, as ray_box_faces does. Rays
-// within the margin of an edge, from inside or along an axis take ray_box_faces.
+// within the margin of an edge, from inside, along an axis or with a NaN (each compared, since a
+// minimum passes over one; a frame with a NaN in one column gives one axis of it) take ray_box_faces.
 MJ_HD float ray_box_local(V3 lo, V3 ld, V3 size, int* axis, float* dir) {
-  if (fminf(fminf(fabsf(ld.x), fabsf(ld.y)), fabsf(ld.z)) > 1.0e-10f) {
+  if (fabsf(ld.x) > 1.0e-10f && fabsf(ld.y) > 1.0e-10f && fabsf(ld.z) > 1.0e-10f) {
     float nx, ny, nz, fx, fy, fz, ex, ey, ez;
     box_axis(lo.x, ld.x, size.x, &nx, &fx, &ex);
     box_axis(lo.y, ld.y, size.y, &ny, &fy, &ey);

@@ -192,3 +192,21 @@ def test_more_geoms_than_the_wavefront_packs(tier):
   np.testing.assert_array_equal(gpu["seg"], ref["seg"])
   np.testing.assert_allclose(gpu["depth"], ref["depth"], rtol=1e-5, atol=1e-6)
   assert helpers.rgb_diff(gpu["rgb"], ref["rgb"]).max() <= 1
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("schedule", ["grid", "wavefront"])
+@pytest.mark.parametrize("entry", [0, 5, 7])
+def test_box_with_a_nan_in_its_frame_is_not_hit(schedule, entry):
+  """A box whose frame holds a NaN is in no ray's way, as if it were hidden (the face tests fail on a NaN)."""
+  images = []
+  for broken in (False, True):
+    rgba = np.array([[[0.6, 0.6, 0.6, 1], [0.8, 0.2, 0.2, 1], [0.2, 0.3, 0.9, 1.0 if broken else 0.0]]], np.float32)
+    sc = _scene("nan", lambda b: _basic(b, (48, 40), target=(0.5, 0.2, 0.15)), per_world={"geom_rgba": rgba}, schedule=schedule)
+    if broken:
+      sc.mjd.geom_xmat[..., 2, entry] = np.nan
+    m, d, rc = helpers.gpu_scene(sc)
+    images.append(helpers.render_gpu(m, d, rc, seed=1))
+  for key in ("seg", "depth", "rgb"):
+    np.testing.assert_array_equal(images[1][key], images[0][key], err_msg=key)
