@@ -6,7 +6,7 @@
 //
 // GB300 layout: the path tracer already wrote the demodulated radiance + variance (one float4 per
 // pixel) into denoise_buffers[0] and the filter's guide as one 16-byte record per pixel (normal and
-// albedo as half floats, depth). Passes of steps up to 8 stage a 16 x 16 tile and its 2-step border in
+// albedo as half floats, depth). Passes of steps up to 4 (launch_pass) stage a 16 x 16 tile and its 2-step border in
 // shared memory once, unpacked and with the luminance, 48 bytes a pixel: a tap is three 128-bit loads at
 // constant offsets, without conversions, bounds (pixels outside the image have a zero normal, so zero
 // weight) or addresses. Bound by the taps' arithmetic (some 55 instructions; 86 where every tap loads and
@@ -221,13 +221,18 @@ int launch_tile(const MjpbrScene& s, const Images& im, const Filter& f, const fl
   return check_launch("atrous_tile_kernel");
 }
 
+// Passes by tile up to step 4, and at 8 if it is the last: a tile and its border are then 110 KB, two CTAs an SM,
+// and a plain pass takes 853 us where the taps from global memory take 740; with the finish 898 and 916 (512
+// worlds of 128 x 128).
 template <bool kFinish>
 int launch_pass(const MjpbrScene& s, const Images& im, const Filter& f, const float4* src, float4* dst, dim3 grid, cudaStream_t stream) {
   switch (f.step) {
     case 1: return launch_tile<1, kFinish>(s, im, f, src, dst, grid, stream);
     case 2: return launch_tile<2, kFinish>(s, im, f, src, dst, grid, stream);
     case 4: return launch_tile<4, kFinish>(s, im, f, src, dst, grid, stream);
-    case 8: return launch_tile<8, kFinish>(s, im, f, src, dst, grid, stream);
+    case 8:
+      if constexpr (kFinish) return launch_tile<8, true>(s, im, f, src, dst, grid, stream);
+      [[fallthrough]];
     default:
       atrous_kernel<kFinish><<<grid, kTile * kTile, 0, stream>>>(s, im, f, src, dst);
       return check_launch("atrous_kernel");

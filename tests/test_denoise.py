@@ -151,3 +151,11 @@ def test_features_match_oracle():
   demod, ref_demod = rc.denoise_buffers[0].cpu().numpy(), ref["aov_demod"]
   err = np.abs(demod[..., :3] - ref_demod[..., :3]).mean()
   assert err <= 0.01 * np.abs(ref_demod[..., :3]).mean()
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("iterations", [2, 4, 6])
+def test_filter_of_even_pass_counts_matches_oracle(iterations):
+  """Last passes of steps 2, 8 and 32 (test_filter_matches_oracle has 1, 4 and 16)."""
+  test_filter_matches_oracle(iterations)
