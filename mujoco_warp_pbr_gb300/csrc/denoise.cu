@@ -223,10 +223,12 @@ int launch_tile(const MjpbrScene& s, const Images& im, const Filter& f, const fl
 
 // Passes by tile up to step 4, and at 8 if it is the last: a tile and its border are then 110 KB, two CTAs an SM,
 // and a plain pass takes 853 us where the taps from global memory take 740; with the finish 898 and 916 (512
-// worlds of 128 x 128).
+// worlds of 128 x 128). Negative sigmas, whose weights grow with the distance, never by tile: a pixel outside
+// the image would count 0 x infinity there.
 template <bool kFinish>
 int launch_pass(const MjpbrScene& s, const Images& im, const Filter& f, const float4* src, float4* dst, dim3 grid, cudaStream_t stream) {
-  switch (f.step) {
+  const bool decays = f.sigma_color >= 0.0f && f.sigma_albedo >= 0.0f;
+  switch (decays ? f.step : 0) {
     case 1: return launch_tile<1, kFinish>(s, im, f, src, dst, grid, stream);
     case 2: return launch_tile<2, kFinish>(s, im, f, src, dst, grid, stream);
     case 4: return launch_tile<4, kFinish>(s, im, f, src, dst, grid, stream);

@@ -159,3 +159,34 @@ def test_features_match_oracle():
 def test_filter_of_even_pass_counts_matches_oracle(iterations):
   """Last passes of steps 2, 8 and 32 (test_filter_matches_oracle has 1, 4 and 16)."""
   test_filter_matches_oracle(iterations)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("sigma", ["denoise_sigma_color", "denoise_sigma_albedo"])
+def test_negative_sigma_leaves_the_border_finite(sigma):
+  """A negative sigma makes a weight grow with the difference it stands for; pixels outside the image, as
+  different as they come, still have none: one pass over a flat floor gives the floor."""
+  import mujoco_warp_pbr_gb300 as mjpbr
+
+  b = Builder()
+  floor = b.material(rgba=(0.5, 0.5, 0.5, 1), roughness=0.8)
+  b.geom(GEOM_PLANE, (9, 9, 0.1), matid=floor)
+  b.camera(pos=(0, -1.0, 1.5), target=(0, 0, 0), fovy=40.0, resolution=(40, 24))
+  mjm, mjd = b.build()
+  m = mjpbr.put_model(mjm)
+  d = mjpbr.put_data(mjm, mjd, nworld=1)
+  rc = mjpbr.create_render_context(mjm, 1, data=mjd, path_samples=2, denoise=True, denoise_iterations=1, render_rgb=True, **PATH)
+  mjpbr.refit_bvh(m, d, rc)
+  mjpbr.render(m, d, rc, seed=3, denoise=False)
+  rc.denoise_buffers[0][..., :3] = 0.25  # a flat image of no variance
+  rc.denoise_buffers[0][..., 3] = 0.0
+  images = []
+  for value in (getattr(rc, sigma), -1.0e-3):
+    setattr(rc, sigma, value)
+    if sigma == "denoise_sigma_color":  # its tolerance is sigma times the noise
+      rc.denoise_buffers[0][..., 3] = 1.0
+    mjpbr.denoise(m, d, rc)
+    images.append(rc.hdr_data.cpu().numpy().copy())
+  assert np.isfinite(images[0]).all() and images[0].max() > 0.0
+  np.testing.assert_allclose(images[1], images[0], rtol=1e-5)
