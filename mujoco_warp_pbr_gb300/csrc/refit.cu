@@ -5,8 +5,8 @@
 // poses and sizes, then a bottom-up refit of each world's tree over the enabled geoms. The same
 // pass writes the world block (world_block.cuh) the render kernels stage into shared memory, so
 // the broadcasting of every batched table (worldid % nbatch) is resolved once per frame instead of
-// once per ray. Two warps per world: one builds the geom records and leaf boxes, its lanes in parallel,
-// and its lane 0 sweeps the (small) tree bottom-up; the other builds the light and camera records. Bound
+// once per ray. Two warps per world (one in worlds of many geoms): one builds the geom records and leaf boxes,
+// its lanes in parallel, and its lane 0 sweeps the tree bottom-up; the other builds the light and camera records. Bound
 // by latency: the sweep's nodes stay in shared memory until it is done (16 worlds of 9 geoms 4.9 us, 17
 // through global memory and with one warp; 1024 of 12 8.7 us, 19 so).
 #include <cfloat>
@@ -19,6 +19,7 @@ namespace mjpbr {
 namespace {
 
 constexpr int kWorldsPerCta = 2;
+constexpr int kSmSharedBytes = 228 * 1024, kCtaSharedBytes = 1024;  // an SM's shared memory; what a CTA reserves of it
 constexpr float kBigExtent = 1.0e6f;  // half extent of infinite planes
 
 // MuJoCo Warp's _geom_rgba: a geom with a material and the default rgba shows the material's.
@@ -195,17 +196,21 @@ __device__ __forceinline__ void refit_lights_cameras(const MjpbrScene& s, int32_
   }
 }
 
-// Where the sweep finds the leaf boxes and keeps the nodes: both in shared memory; the boxes (worlds
-// whose nodes do not fit beside them, a few hundred geoms); neither, each leaf's box computed from its geom
-// record (a few thousand geoms).
+// Where the sweep finds the leaf boxes and keeps the nodes: both in shared memory; the boxes (a few hundred
+// geoms: see refit_launch); neither, each leaf's box computed from its geom record (a few thousand geoms).
 enum RefitSmem { kSmemNone, kSmemBoxes, kSmemNodes };
 
+// The second warp is for the latency of few geoms; with many, whose sweeps take their time, it would halve the
+// worlds resident on an SM.
 template <RefitSmem kSmem>
-__global__ void __launch_bounds__(kWorldsPerCta * 64) refit_kernel(const __grid_constant__ MjpbrScene s) {
+constexpr int kWorldWarps = kSmem == kSmemNodes ? 2 : 1;
+
+template <RefitSmem kSmem>
+__global__ void __launch_bounds__(kWorldsPerCta * 32 * kWorldWarps<kSmem>) refit_kernel(const __grid_constant__ MjpbrScene s) {
   extern __shared__ __align__(16) float smem[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  const int slot_in_cta = warp >> 1;
+  const int slot_in_cta = warp / kWorldWarps<kSmem>;
   const int32_t w = blockIdx.x * kWorldsPerCta + slot_in_cta;
   if (w >= s.nworld) return;
   const int32_t nbvh = s.nbvh_geom;
@@ -215,10 +220,8 @@ __global__ void __launch_bounds__(kWorldsPerCta * 64) refit_kernel(const __grid_
   BlockLayout L = block_layout(nbvh, s.nnode, s.nlight, s.nrender);
   float* blk = s.world_blocks + (int64_t)w * s.world_block_floats;
 
-  if (warp & 1) {
-    refit_lights_cameras(s, w, lane, blk, L);
-    return;
-  }
+  if (kWorldWarps<kSmem> == 1 || (warp & 1)) refit_lights_cameras(s, w, lane, blk, L);
+  if (kWorldWarps<kSmem> == 2 && (warp & 1)) return;
 
   // ---- geom records and leaf boxes
   for (int32_t slot = lane; slot < nbvh; slot += 32) {
@@ -352,16 +355,22 @@ __global__ void __launch_bounds__(kWorldsPerCta * 64) refit_kernel(const __grid_
 
 int refit_launch(const MjpbrScene& s, cudaStream_t stream) {
   const int grid = (s.nworld + kWorldsPerCta - 1) / kWorldsPerCta;
-  auto launch = [&](auto kern, size_t smem) {
+  auto launch = [&](auto kern, int warps, size_t smem) {
     if (int rc = ensure_smem(reinterpret_cast<const void*>(kern), smem, "refit")) return rc;
-    kern<<<grid, kWorldsPerCta * 64, smem, stream>>>(s);
+    kern<<<grid, kWorldsPerCta * 32 * warps, smem, stream>>>(s);
     return check_launch("refit_kernel");
   };
   auto bytes = [&](int64_t floats) { return (size_t)kWorldsPerCta * ((floats + 3) & ~(int64_t)3) * sizeof(float); };
   const size_t boxes = bytes((int64_t)s.nbvh_geom * 6), all = bytes((int64_t)s.nbvh_geom * 6 + (int64_t)s.nnode * kNodeFloats);
-  if (all <= 100 * 1024) return launch(refit_kernel<kSmemNodes>, all);
-  if (boxes <= 100 * 1024) return launch(refit_kernel<kSmemBoxes>, boxes);
-  return launch(refit_kernel<kSmemNone>, 0);
+  // Nodes in shared memory halve a world's latency, and cost residency: with fewer than six CTAs an SM (above 220
+  // geoms) two waves of them take as long as one with the boxes alone, three longer. us, nodes / boxes: 200
+  // geoms and 12,000 worlds (7 waves) 615 / 653; 300 and 16 worlds 113 / 201, 2048 (2 waves) 242 / 285, 4096
+  // (4 waves) 465 / 389; 450 and 1024 (2 waves) 322 / 345, 4096 1101 / 825; 580 and 4096 1420 / 1019.
+  const int64_t resident = (int64_t)kSmSharedBytes / (all + kCtaSharedBytes);
+  const int64_t wave = resident * kWorldsPerCta * device_sm_count();
+  if (all <= 100 * 1024 && (resident >= 6 || s.nworld <= 2 * wave)) return launch(refit_kernel<kSmemNodes>, kWorldWarps<kSmemNodes>, all);
+  if (boxes <= 100 * 1024) return launch(refit_kernel<kSmemBoxes>, kWorldWarps<kSmemBoxes>, boxes);
+  return launch(refit_kernel<kSmemNone>, kWorldWarps<kSmemNone>, 0);
 }
 
 }  // namespace mjpbr
