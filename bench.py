@@ -547,13 +547,8 @@ def run(args) -> None:
     achieved = alg / (render_avg / 1000.0) / 1e9
     peak = float(peaks.get("hbm_gbs", 6800.0))
     traffic = _traffic(sc.name)
-    launches = render_launches(rc, int(chunks.value), int(scene.nlight))
-    if args.workload == "path":
-      kernel = "path wavefront: ptw_first_extend, ptw_extend, ptw_shade, ptw_shadow, ptw_resolve per chunk, one frame"
-    elif wave:
-      kernel = "wavefront render: wave_primary, wave_surface, wave_mirror (scan, mesh), wave_mirror_surface, wave_shadow, wave_resolve per chunk, one frame"
-    else:
-      kernel = "rt_kernel"
+    launches = render_launches(rc, scene, int(chunks.value))
+    kernel = render_kernel(rc, scene)
     line = {
       "metric": PATH_METRIC if args.workload == "path" else METRIC,
       "value": value,
@@ -627,22 +622,41 @@ def frame_chunks(m, d, rc) -> int:
   return int(chunks.value)
 
 
-def render_launches(rc, chunks: int, nlight: int) -> int:
+def scanned(rc) -> bool:
+  """Whether the wavefront's stages scan the geoms of a mesh scene (up to 32 geoms) instead of walking the
+  scene BVH: the mirror stage is then two kernels."""
+  return rc.enabled_geom_ids.shape[0] <= 32 and bool(rc.mesh_nface or rc.nhfield)
+
+
+def render_launches(rc, scene, chunks: int) -> int:
   """Kernels one render call launches: the wavefront's stages per chunk of worlds (primary, and
   with RGB cameras surface + resolve, mirror + mirror surface with reflections, shadow with
-  shadowing lights), else the single fused kernel (scenes of up to 32 geoms without meshes) /
-  megakernel / path kernel."""
-  if not (rc.tier == 0 and rc.schedule == 2 and not rc.has_transparency):
-    return 1
-  if rc.enabled_geom_ids.shape[0] <= 32 and not rc.mesh_nface and not rc.nhfield and nlight <= 16:
+  shadowing lights), else the single fused kernel / megakernel / path kernel."""
+  from mujoco_warp_pbr_gb300 import _lib
+
+  if not (rc.tier == 0 and rc.schedule == 2 and not rc.has_transparency) or _lib.load().mjpbr_wave_fused(scene) == 1:
     return 1
   rgb = any(rc.base.render_rgb)
   per = 1 + (2 if rgb else 0) + (2 if rgb and rc.has_reflection else 0)
-  if rgb and rc.has_reflection and rc.enabled_geom_ids.shape[0] <= 32:
+  if rgb and rc.has_reflection and scanned(rc):
     per += 1  # the mirror rays' meshes, apart from their primitives
-  if rgb and rc.use_shadows and nlight > 0:
+  if rgb and rc.use_shadows and scene.nlight > 0:
     per += 1
   return per * max(chunks, 1)
+
+
+def render_kernel(rc, scene) -> str:
+  """What a frame of rc is rendered by."""
+  from mujoco_warp_pbr_gb300 import _lib
+
+  if rc.tier == 1:
+    return "path wavefront: ptw_first_extend, ptw_extend, ptw_shade, ptw_shadow, ptw_resolve per chunk, one frame"
+  if rc.schedule != 2 or rc.has_transparency:
+    return "rt_queue_kernel" if rc.schedule == 1 else "rt_kernel"
+  if _lib.load().mjpbr_wave_fused(scene) == 1:
+    return "rt_fused_kernel, one frame"
+  mirror = "wave_mirror_scan, wave_mirror_mesh" if scanned(rc) else "wave_mirror"
+  return f"wavefront render: wave_primary, wave_surface, {mirror}, wave_mirror_surface, wave_shadow, wave_resolve per chunk, one frame"
 
 
 def rt_fp32_roofline(args, dev, npix: int, render_ms: float, count_worlds: int = 256) -> dict:
@@ -807,7 +821,10 @@ def measure_batched(args, dev, nworld: int, steps: int, warmup: int, cpu_budget:
   synthetic.apply_per_world(sc, m, rc)
   tuned = mjpbr.autotune(m, d, rc, frames=3)
   npix = sc.nworld * sum(w * h for w, h in rc.base.cam_res)
-  launches = 1 + render_launches(rc, frame_chunks(m, d, rc), int(mjpbr.scene_descriptor(m, d, rc).nlight))  # refit + render
+  scene = mjpbr.scene_descriptor(m, d, rc)
+  launches = 1 + render_launches(rc, scene, frame_chunks(m, d, rc))  # refit + render
+  kernel = render_kernel(rc, scene)
+  shape = "wavefront" if kernel.startswith("rt_fused") else tuned["best"]  # a fused frame has no chunks
   poses = d.geom_xpos.clone()
   poses[:, 1:, 2] += 0.01  # the "next" poses the step copies in
   graph = mjpbr.capture_frame(m, d, rc, seed=7, step=lambda: d.geom_xpos.copy_(poses))
@@ -874,7 +891,7 @@ def measure_batched(args, dev, nworld: int, steps: int, warmup: int, cpu_budget:
             "d2h_bytes_per_step": int(copier.d2h), "output": copier.describe()},
     "roofline": {
       "bound": "hbm",
-      "kernel": f"render ({tuned['best']}), whole graph timed",
+      "kernel": f"{kernel} (autotuned: {shape}), whole graph timed",
       "achieved": achieved,
       "peak": peak,
       "unit": "GB/s",

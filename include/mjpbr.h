@@ -84,9 +84,10 @@ enum MjpbrTier { MJPBR_TIER_REALTIME = 0, MJPBR_TIER_PATH = 1 };
 enum MjpbrRenderOrder { MJPBR_ORDER_ROW = 0, MJPBR_ORDER_TILED = 1, MJPBR_ORDER_WORLD = 2 };
 /* Schedules. Real-time tier: one CTA per (camera tile, world); a persistent launch whose warps
  * pull work items (settings.queue_item pixels of one camera image of one world) from a device
- * counter (scene.work_counter[1]); or a staged wavefront (primary rays, surfaces, mirror rays,
+ * counter (scene.work_counter[1]); or a wavefront: staged (primary rays, surfaces, mirror rays,
  * shadow rays and shading as separate kernels over compacted ray queues, chunks of worlds at a
- * time in scene.wave_scratch; translucent layers render with the grid schedule). Path tier: GRID
+ * time in scene.wave_scratch), or for scenes of few geoms without triangle BVHs one fused kernel without
+ * scratch (mjpbr_wave_fused); translucent layers render with the grid schedule. Path tier: GRID
  * and QUEUE select the persistent path kernel, WAVEFRONT the staged bounce loop (extend, shade,
  * shadow, next-event kernels over compacted path queues in scene.wave_scratch). Every schedule of
  * a tier renders identical images. */
@@ -352,7 +353,7 @@ typedef struct MjpbrScene {
   int32_t* error_word;             /* device int32, kernels OR error bits into it (may be NULL) */
   int32_t* work_counter;           /* device int32[4] scratch of the persistent kernels' work queues
                                       (the library zeroes it on the stream before each use) */
-  void* wave_scratch;              /* wavefront schedule: device scratch, 256-byte aligned (NULL otherwise) */
+  void* wave_scratch;              /* staged wavefronts: device scratch, 256-byte aligned (NULL otherwise) */
   int64_t wave_scratch_bytes;      /* its size; mjpbr_wave_scratch_bytes gives the size for a chunk of worlds */
 
   MjpbrSettings settings;
@@ -378,6 +379,11 @@ int32_t mjpbr_world_block_floats(int32_t nbvh_geom, int32_t nnode, int32_t nligh
  * or -1. Host only; reads the scene's counts and settings, no device pointer. New with the
  * wavefront schedule (the reference renders every world in one megakernel launch). */
 int64_t mjpbr_wave_scratch_bytes(const MjpbrScene* scene, int32_t worlds);
+
+/* 1 if the wavefront schedule renders this real-time scene as one fused kernel (few geoms, no triangle
+ * BVHs, opaque, few lights), which uses no wave_scratch: it may then be NULL. 0 otherwise, -1 for NULL. Host
+ * only, as mjpbr_wave_scratch_bytes. */
+int32_t mjpbr_wave_fused(const MjpbrScene* scene);
 
 /* Stage profile of the wavefront schedule, for tools: after mjpbr_wave_profile_begin, every
  * wavefront render issued from this host thread records CUDA events (the library's own, reused) on

@@ -318,6 +318,7 @@ _SIGNATURES = {
   "mjpbr_struct_layout": (None, [ctypes.POINTER(ctypes.c_int64)]),
   "mjpbr_world_block_floats": (c_i32, [c_i32, c_i32, c_i32, c_i32]),
   "mjpbr_wave_scratch_bytes": (ctypes.c_int64, [ctypes.POINTER(Scene), c_i32]),
+  "mjpbr_wave_fused": (c_i32, [ctypes.POINTER(Scene)]),
   "mjpbr_env_sh9": (ctypes.c_int, [c_vp, c_i32, c_i32, c_vp, c_vp, c_vp]),
   "mjpbr_env_sampling_tables": (ctypes.c_int, [c_vp, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp]),
   "mjpbr_wait_probe": (ctypes.c_int, [ctypes.c_uint32, c_vp, c_vp, c_vp]),

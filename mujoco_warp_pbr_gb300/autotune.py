@@ -6,7 +6,7 @@ tiles; the megakernel as a persistent launch whose warps pull work items of 32, 
 from a device counter (the queue's item size is its ray-sort granularity: the pixels a warp
 renders back to back from one world block); and the staged wavefront (one kernel per stage over
 compacted ray queues, a chunk of worlds at a time: the chunk size trades scratch memory and L2
-locality against launches). Every candidate renders the same image; the autotuner times each on
+locality against launches; scenes of few geoms without meshes take one fused kernel and have no chunks). Every candidate renders the same image; the autotuner times each on
 the context's own scene and keeps the fastest. Results are cached per scene signature for the
 process.
 
@@ -109,6 +109,8 @@ def autotune(
   skipped: dict[str, str] = {}
   for shape in candidates:
     apply(rc, shape)
+    if shape.schedule == WAVEFRONT and shape.wave_chunk_worlds and _lib.load().mjpbr_wave_fused(scene_descriptor(m, d, rc)) == 1:
+      continue  # one fused kernel: there are no chunks
     t0 = time.perf_counter()
     try:
       render(m, d, rc)

@@ -1025,6 +1025,13 @@ int render_wave_launch(const MjpbrScene& s, uint32_t seed, cudaStream_t stream) 
   }
   const int32_t per_world = samples_per_world(s);
   if (per_world < 0) return set_error(MJPBR_ERR_ARG, "wavefront: too many samples per world");
+  if (fused_supported(s)) {
+    // the whole frame is one kernel, without scratch: the profile's first stage
+    stage_mark(stream);
+    const int rc = render_fused_launch(s, seed, stream);
+    for (int k = 0; k < kStages; ++k) stage_mark(stream);
+    return rc;
+  }
   if (!s.wave_scratch || (reinterpret_cast<uintptr_t>(s.wave_scratch) & 255u)) {
     return set_error(MJPBR_ERR_ARG, "the wavefront schedule needs wave_scratch (256-byte aligned)");
   }
@@ -1053,13 +1060,6 @@ int render_wave_launch(const MjpbrScene& s, uint32_t seed, cudaStream_t stream) 
   }
   const bool mesh = s.nmesh + s.nhfield > 0 && s.blas_root != nullptr;
   const bool tex = s.settings.textures || s.settings.has_env || s.settings.env_background;
-  if (fused_supported(s)) {
-    // the whole frame is one kernel: the profile's first stage
-    stage_mark(stream);
-    const int rc = render_fused_launch(s, seed, stream);
-    for (int k = 0; k < kStages; ++k) stage_mark(stream);
-    return rc;
-  }
   const size_t stack = (size_t)kThreads * stack_entries(s.settings.stack_depth) * 8;
   const bool staged = world_block_staged(s.world_block_floats, stack);
   auto launch = [&](auto m, auto t, auto b, auto scan) {
@@ -1119,6 +1119,13 @@ extern "C" int mjpbr_wave_profile_end(double* stage_ms, int32_t* chunks) {
 extern "C" int64_t mjpbr_wave_scratch_bytes(const MjpbrScene* scene, int32_t worlds) {
   if (!scene) return -1;
   return mjpbr::wave_scratch_bytes(*scene, worlds);
+}
+
+extern "C" int32_t mjpbr_wave_fused(const MjpbrScene* scene) {
+  using namespace mjpbr;
+  if (!scene) return -1;
+  return scene->settings.tier == MJPBR_TIER_REALTIME && scene->settings.schedule == MJPBR_SCHEDULE_WAVEFRONT && wave_supported(*scene) &&
+         fused_supported(*scene);
 }
 
 #ifdef MJPBR_COUNT_OPS

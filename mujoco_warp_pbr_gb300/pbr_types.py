@@ -187,8 +187,8 @@ class PbrRenderContext:
   schedule: int = 0
   queue_item: int = 64
   wave_chunk_worlds: int = 0
-  # the wavefront schedule's ray queues and records (uint8, allocated at the first render that
-  # needs them, sized by mjpbr_wave_scratch_bytes)
+  # the staged wavefronts' ray queues and records (uint8, allocated at the first render that needs them, sized
+  # by mjpbr_wave_scratch_bytes; fused frames need none)
   wave_scratch: torch.Tensor | None = None
   # accepted for compatibility with the reference's signature; the GB300 kernels choose their own
   block_dim: int | None = None

@@ -284,7 +284,7 @@ WAVE_CHUNK_PATHS = 1 << 25
 def _ensure_wave_scratch(rc: PbrRenderContext, struct: _lib.Scene) -> bool:
   """Allocates (or grows) the wavefront schedule's scratch for a context using it: wave_chunk_worlds
   worlds per chunk, or about WAVE_CHUNK_SAMPLES camera samples (real-time tier) / WAVE_CHUNK_PATHS
-  paths (path tier). Returns True when rc.wave_scratch changed."""
+  paths (path tier). Frames of one fused kernel use none. Returns True when rc.wave_scratch changed."""
   if rc.schedule != 2 or (rc.tier == 0 and rc.has_transparency):
     return False
   lib = _lib.load()
@@ -301,6 +301,8 @@ def _ensure_wave_scratch(rc: PbrRenderContext, struct: _lib.Scene) -> bool:
   need = int(lib.mjpbr_wave_scratch_bytes(struct, chunk))
   if need < 0 or per_world < 0:
     raise ValueError("the wavefront schedule cannot render this scene")
+  if lib.mjpbr_wave_fused(struct) == 1:
+    return False
   if rc.wave_scratch is not None and rc.wave_scratch.numel() >= need:
     return False
   rc.wave_scratch = torch.empty(need, dtype=torch.uint8, device=rc.device)

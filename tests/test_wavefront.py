@@ -46,6 +46,60 @@ def test_wave_scratch_size_is_exported():
   assert fn(None, 1) == -1
 
 
+def test_fused_scenes_are_told():
+  """mjpbr_wave_fused is host-only: opaque scenes of up to 32 geoms without triangle BVHs and up to 16 lights."""
+  import ctypes
+
+  from mujoco_warp_pbr_gb300 import _lib
+
+  lib = _lib.load()
+
+  def fused(**changes):
+    s = _lib.Scene()
+    s.abi_version = _lib.ABI_VERSION
+    s.nworld, s.nrender, s.nlight, s.nbvh_geom, s.nnode = 8, 1, 2, 32, 31
+    s.world_block_floats = lib.mjpbr_world_block_floats(32, 31, 2, 1)
+    s.cam_res[0][0], s.cam_res[0][1] = 64, 32
+    s.render_rgb[0] = 1
+    s.settings.samples_per_axis, s.settings.schedule, s.settings.stack_depth = 2, 2, 8
+    for name, value in changes.items():
+      setattr(s if hasattr(s, name) else s.settings, name, value)
+    return lib.mjpbr_wave_fused(ctypes.byref(s))
+
+  assert fused() == 1 and fused(nlight=16) == 1 and fused(nmesh=2) == 1  # meshes without BVHs
+  assert fused(samples_per_axis=16) == 1
+  for change in ({"nbvh_geom": 33}, {"nlight": 17}, {"nmesh": 1, "blas_root": 0x1000}, {"nhfield": 1, "blas_root": 0x1000},
+                 {"has_transparency": 1}, {"samples_per_axis": 17}, {"schedule": 0}, {"schedule": 1}, {"tier": 1},
+                 {"world_block_floats": 1 << 20}):
+    assert fused(**change) == 0, change
+  assert lib.mjpbr_wave_fused(None) == -1
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+def test_fused_frames_take_no_scratch():
+  """A context whose frame is one fused kernel allocates no ray queues, and the library renders it without;
+  one of more geoms gets them."""
+  import mujoco_warp_pbr_gb300 as mjpbr
+  from mujoco_warp_pbr_gb300 import synthetic
+  from tests import helpers
+  from tests.test_scan import scene
+
+  sc = synthetic.batched_scene(seed=1, nworld=5, res=(16, 40, 72))
+  m, d, rc = helpers.gpu_scene(sc, render_hdr=True, render_guides=True)
+  ref = _frame(m, d, rc, seed=9)
+  rc.schedule = 2
+  got = _frame(m, d, rc, seed=9)
+  assert rc.wave_scratch is None and not mjpbr.scene_descriptor(m, d, rc).wave_scratch
+  for key in ref:
+    np.testing.assert_array_equal(got[key], ref[key], err_msg=key)
+  result = mjpbr.autotune(m, d, rc, frames=1, use_cache=False)
+  assert len([k for k in result["ms"] if k.startswith("wavefront")]) == 1  # there are no chunks to choose
+  m, d, rc = helpers.gpu_scene(scene(33), schedule="wavefront")
+  helpers.render_gpu(m, d, rc)
+  assert rc.wave_scratch is not None
+
+
 def _outputs(rc):
   out = {
     "rgb": rc.base.rgb_data.cpu().numpy().view(np.uint32).copy(),
