@@ -173,15 +173,16 @@ def algorithmic_bytes(rc) -> int:
   return int(out + inputs)
 
 
-def _traffic(workload: str) -> float | None:
+def _traffic(workload: str, kernels: list[str] | None = None) -> float | None:
   """DRAM bytes of one frame's render kernels from an ncu launch list (profiles/ncu_traffic.txt:
-  workload, bytes per frame, kernels), or None."""
+  workload, bytes per frame, kernels): of the first line for the workload, or of the one for these
+  kernels; or None."""
   p = ROOT / "profiles" / "ncu_traffic.txt"
   if not p.exists():
     return None
   for line in p.read_text().splitlines():
-    parts = line.split("#", 1)[0].split()
-    if len(parts) >= 2 and parts[0] == workload:
+    parts = line.split("#", 1)[0].split(None, 2)
+    if len(parts) >= 2 and parts[0] == workload and (kernels is None or (len(parts) == 3 and [k.strip() for k in parts[2].split(",")] == kernels)):
       try:
         return float(parts[1])
       except ValueError:
@@ -546,9 +547,10 @@ def run(args) -> None:
     alg = algorithmic_bytes(rc)
     achieved = alg / (render_avg / 1000.0) / 1e9
     peak = float(peaks.get("hbm_gbs", 6800.0))
-    traffic = _traffic(sc.name)
+    kernels = render_kernels(rc, scene)
+    traffic = _traffic(sc.name, kernels)
     launches = render_launches(rc, scene, int(chunks.value))
-    kernel = render_kernel(rc, scene)
+    kernel = ", ".join(kernels) + ": one frame"
     line = {
       "metric": PATH_METRIC if args.workload == "path" else METRIC,
       "value": value,
@@ -622,41 +624,37 @@ def frame_chunks(m, d, rc) -> int:
   return int(chunks.value)
 
 
-def scanned(rc) -> bool:
-  """Whether the wavefront's stages scan the geoms of a mesh scene (up to 32 geoms) instead of walking the
-  scene BVH: the mirror stage is then two kernels."""
-  return rc.enabled_geom_ids.shape[0] <= 32 and bool(rc.mesh_nface or rc.nhfield)
+def render_kernels(rc, scene) -> list[str]:
+  """The kernels a frame of rc is rendered by, "(scan)" where up to 32 geoms are scanned instead of the scene
+  BVH walked."""
+  from mujoco_warp_pbr_gb300 import _lib
+
+  scan = " (scan)" if scene.nbvh_geom <= 32 else ""
+  if rc.tier == 1:
+    return ["pt"] if rc.schedule != 2 else [f"ptw_first_extend{scan}", f"ptw_extend{scan}", "ptw_shade", f"ptw_shadow{scan}", "ptw_resolve"]
+  if rc.schedule != 2 or rc.has_transparency:
+    return ["rt_queue" if rc.schedule == 1 and not rc.has_transparency else "rt"]
+  if _lib.load().mjpbr_wave_fused(scene) == 1:
+    return ["rt_fused"]
+  scan = scan if rc.mesh_nface or rc.nhfield else ""
+  rgb = any(rc.base.render_rgb)
+  names = [f"wave_primary{scan}"]
+  if rgb:
+    names.append("wave_surface")
+  if rgb and rc.has_reflection:
+    names += ["wave_mirror_scan", "wave_mirror_mesh"] if scan else ["wave_mirror"]
+    names.append("wave_mirror_surface")
+  if rgb and rc.use_shadows and scene.nlight > 0:
+    names.append(f"wave_shadow{scan}")
+  if rgb:
+    names.append("wave_resolve")
+  return names
 
 
 def render_launches(rc, scene, chunks: int) -> int:
-  """Kernels one render call launches: the wavefront's stages per chunk of worlds (primary, and
-  with RGB cameras surface + resolve, mirror + mirror surface with reflections, shadow with
-  shadowing lights), else the single fused kernel / megakernel / path kernel."""
-  from mujoco_warp_pbr_gb300 import _lib
-
-  if not (rc.tier == 0 and rc.schedule == 2 and not rc.has_transparency) or _lib.load().mjpbr_wave_fused(scene) == 1:
-    return 1
-  rgb = any(rc.base.render_rgb)
-  per = 1 + (2 if rgb else 0) + (2 if rgb and rc.has_reflection else 0)
-  if rgb and rc.has_reflection and scanned(rc):
-    per += 1  # the mirror rays' meshes, apart from their primitives
-  if rgb and rc.use_shadows and scene.nlight > 0:
-    per += 1
-  return per * max(chunks, 1)
-
-
-def render_kernel(rc, scene) -> str:
-  """What a frame of rc is rendered by."""
-  from mujoco_warp_pbr_gb300 import _lib
-
-  if rc.tier == 1:
-    return "path wavefront: ptw_first_extend, ptw_extend, ptw_shade, ptw_shadow, ptw_resolve per chunk, one frame"
-  if rc.schedule != 2 or rc.has_transparency:
-    return "rt_queue_kernel" if rc.schedule == 1 else "rt_kernel"
-  if _lib.load().mjpbr_wave_fused(scene) == 1:
-    return "rt_fused_kernel, one frame"
-  mirror = "wave_mirror_scan, wave_mirror_mesh" if scanned(rc) else "wave_mirror"
-  return f"wavefront render: wave_primary, wave_surface, {mirror}, wave_mirror_surface, wave_shadow, wave_resolve per chunk, one frame"
+  """Kernels one render call of the real-time tier launches: its stages per chunk of worlds (1 for the
+  path tier, whose stages are launched per bounce)."""
+  return 1 if rc.tier == 1 else len(render_kernels(rc, scene)) * max(chunks, 1)
 
 
 def rt_fp32_roofline(args, dev, npix: int, render_ms: float, count_worlds: int = 256) -> dict:
@@ -823,8 +821,8 @@ def measure_batched(args, dev, nworld: int, steps: int, warmup: int, cpu_budget:
   npix = sc.nworld * sum(w * h for w, h in rc.base.cam_res)
   scene = mjpbr.scene_descriptor(m, d, rc)
   launches = 1 + render_launches(rc, scene, frame_chunks(m, d, rc))  # refit + render
-  kernel = render_kernel(rc, scene)
-  shape = "wavefront" if kernel.startswith("rt_fused") else tuned["best"]  # a fused frame has no chunks
+  kernels = render_kernels(rc, scene)
+  shape = "wavefront" if kernels == ["rt_fused"] else tuned["best"]  # a fused frame has no chunks
   poses = d.geom_xpos.clone()
   poses[:, 1:, 2] += 0.01  # the "next" poses the step copies in
   graph = mjpbr.capture_frame(m, d, rc, seed=7, step=lambda: d.geom_xpos.copy_(poses))
@@ -891,12 +889,12 @@ def measure_batched(args, dev, nworld: int, steps: int, warmup: int, cpu_budget:
             "d2h_bytes_per_step": int(copier.d2h), "output": copier.describe()},
     "roofline": {
       "bound": "hbm",
-      "kernel": f"{kernel} (autotuned: {shape}), whole graph timed",
+      "kernel": f"{', '.join(kernels)} (autotuned: {shape}), whole graph timed",
       "achieved": achieved,
       "peak": peak,
       "unit": "GB/s",
       "frac": achieved / peak,
-      "traffic": _traffic(sc.name),
+      "traffic": _traffic(sc.name, kernels),
       "algorithmic_bytes_per_launch": alg,
       "peak_source": "measured" if "fallback" not in peaks else "fallback",
     },
