@@ -7,10 +7,10 @@
 // K-major core-matrix layout (8 pixels x 16 bytes), so that the A operand of tap (dy, dx) is one
 // descriptor with a uniform 16-byte row stride.
 //
-// conv3x3_flat_kernel (the default, further below) and conv3x3_ws_kernel (half-resolution skips) are
-// persistent warp-specialised kernels whose operands arrive by TMA. conv3x3_kernel, directly below, is
-// the first version: one CTA per tile staging three dx-shifted copies of its rows with plain loads
-// (MJPBR_CONV_PIPELINE=0 selects it, as do batches of more than 2^31 pixels).
+// conv3x3_flat_kernel (every layer without a half-resolution skip, further below) and conv3x3_ws_kernel
+// (half-resolution skips) are persistent warp-specialised kernels whose operands arrive by TMA.
+// conv3x3_kernel, directly below, is the first version: one CTA per tile staging three dx-shifted copies of
+// its rows with plain loads (MJPBR_CONV_PIPELINE=0 selects it, as do batches of more than 2^31 pixels).
 //
 // The U-Net's skip concatenation is read in place: channels past c_in come from in2, either at
 // the output resolution (in2_full) or at half of it, upsampled x2 (nearest) while staging.
@@ -180,13 +180,13 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_kernel(const __grid_c
   if (warp == 0) umma::tmem_free(tmem, ncols);
 }
 
-// ---- warp-specialised variant: persistent CTAs of six warps. Warp 4 loads operands with the
+// ---- warp-specialised variant, of layers with a half-resolution in2: persistent CTAs of six warps. Warp 4 loads operands with the
 // tensor memory accelerator (TMA) into up to kMaxStages stage buffers, warp 5 issues the MMAs,
 // warps 0-3 run the epilogue; two accumulators in tensor memory let a tile's epilogue overlap
 // the next tile's MMAs. The roles hand over through mbarriers:
 //   full[s]   the TMA loads of the stage in buffer s landed (expect-tx arrival by the loader)
-//   ready[s]  the loader is done with it: at once, or after upsampling a half-resolution in2
-//             into its planes (one arrival; the MMA warp waits on full[s] and ready[s])
+//   ready[s]  the loader is done with it: at once, or after upsampling in2 into its planes (one
+//             arrival; the MMA warp waits on full[s] and ready[s])
 //   empty[s]  its MMAs completed (tcgen05.commit)
 //   acc_full[b] / acc_empty[b]  accumulator b holds a finished tile / was read (128 arrivals)
 //
@@ -196,9 +196,8 @@ __global__ void __launch_bounds__(kConvThreads, 2) conv3x3_kernel(const __grid_c
 // dx shift of a tap is a one-pixel (16-byte) offset of the A descriptor; tiles of several short
 // rows stage three dx-shifted copies (spitch = pitch), since a shifted start would wrap from one
 // image row into the next. Outside the image the TMA reads zeros. A stage holds chunks of `in`
-// or of the half-resolution in2, which is loaded as one box per stage covering the tile's
-// footprint and upsampled x2 (nearest) into the planes by the loader warp; a full-resolution in2
-// (in2_full) is staged like `in`.
+// or of in2, which is loaded as one box per stage covering the tile's footprint and upsampled x2
+// (nearest) into the planes by the loader warp.
 //
 // Weights are resident (one TMA box of all taps and channel groups) when they fit, else loaded
 // per stage. Every wait is bounded; a wait that gives up raises the CTA's abort flag, which ends
@@ -217,7 +216,7 @@ struct WsGeom {
   int32_t abuf;      // bytes of one stage's A region: copies x 2G planes (multiple of 128)
   int32_t s2w, s2h;  // in2 box: pixels, rows
   int32_t s2plane;   // bytes of one in2 group plane
-  int32_t s2buf;     // bytes of one stage's in2 boxes (multiple of 128); 0 without in2
+  int32_t s2buf;     // bytes of one stage's in2 boxes (multiple of 128)
   int32_t bstage;    // bytes of one stage's weights; 0 when resident
   int32_t resident;  // weights resident: 9 x (cin / 8) x c_out x 16 bytes at b_off
   int32_t s2_off, b_off;
@@ -362,27 +361,22 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
         if (!ok) break;
         if (lane == 0) {
           const uint32_t abase = s0 + buf * wg.abuf;
-          const bool half = st.in2 && !p.in2_full;  // in2 box, upsampled below
-          uint32_t bytes = half ? in2_box : copies * in_box;
+          uint32_t bytes = st.in2 ? in2_box : copies * in_box;
           if (!wg.resident) bytes += (uint32_t)wg.bstage;
           umma::mbar_arrive_expect_tx(&full[buf], bytes);
-          // a full-resolution in2 is staged like `in`, from its own tensor map
-          const CUtensorMap* src = st.in2 ? &tm_in2 : &tm_in;
-          const int32_t grp0 = 2 * (st.in2 ? st.cs - nci : st.cs);
-          if (half) {
-            umma::tma_load_5d(s0 + wg.s2_off + buf * wg.s2buf, &tm_in2, &full[buf], 0, x0 / 2 - 1, (y0 - 1) >> 1, grp0, img);
+          if (st.in2) {  // upsampled below
+            umma::tma_load_5d(s0 + wg.s2_off + buf * wg.s2buf, &tm_in2, &full[buf], 0, x0 / 2 - 1, (y0 - 1) >> 1, 2 * (st.cs - nci), img);
           } else if (wg.single) {
-            umma::tma_load_5d(abase, src, &full[buf], 0, x0 - 1, y0 - 1, grp0, img);
+            umma::tma_load_5d(abase, &tm_in, &full[buf], 0, x0 - 1, y0 - 1, 2 * st.cs, img);
           } else {
-            for (int32_t dx = 0; dx < 3; ++dx) umma::tma_load_5d(abase + dx * 2 * G * wg.plane, src, &full[buf], 0, x0 - 1 + dx, y0 - 1, grp0, img);
+            for (int32_t dx = 0; dx < 3; ++dx) umma::tma_load_5d(abase + dx * 2 * G * wg.plane, &tm_in, &full[buf], 0, x0 - 1 + dx, y0 - 1, 2 * st.cs, img);
           }
           if (!wg.resident) umma::tma_load_4d(s0 + wg.b_off + buf * wg.bstage, &tm_w, &full[buf], 0, 0, 2 * st.cs, 0);
         }
         issued = k + 1;
-        const bool half = st.in2 && !p.in2_full;
-        // stage k is ready once its loads land (the MMA warp waits on full[] too), unless its
-        // half-resolution in2 must be upsampled first
-        if (!half && lane == 0) umma::mbar_arrive(&ready[buf]);
+        // stage k is ready once its loads land (the MMA warp waits on full[] too), unless its in2
+        // must be upsampled first
+        if (!st.in2 && lane == 0) umma::mbar_arrive(&ready[buf]);
         if (k >= 1 && prev_in2) {
           // stage k - 1: upsample its in2 once it landed
           const int32_t pb = (k - 1) % nst;
@@ -393,7 +387,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
           __syncwarp();
           if (lane == 0) umma::mbar_arrive(&ready[pb]);
         }
-        prev_in2 = half;
+        prev_in2 = st.in2;
         prev_nc = st.nc;
         prev_y0 = y0;
       }
@@ -523,8 +517,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
   if (warp == 0) umma::tmem_free(tmem, ncols);
 }
 
-// ---- blocks of padded rows: the kernel of every layer whose operands fit (conv3x3_ws_kernel takes the
-// rest: half-resolution skips and very wide layers).
+// ---- blocks of padded rows: the kernel of every layer but those with half-resolution skips.
 //
 // A block is T x 128 consecutive positions of an image strip's rows laid end to end, each row with its
 // two halo columns (pitch + 2 positions): in that order the input of tap (dy, dx) lies dy rows and dx
@@ -532,7 +525,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) conv3x3_ws_kernel(const __grid_
 // The two positions per row that are halo columns compute garbage that is not stored (1.5 % of the
 // work at 128 pixels a row, 3 % at 64, 6 % at 32, 11 % at 16), where tiles of whole short rows needed
 // three shifted copies of every row. A block stages its rows and two halo rows once for T
-// accumulators: 11 rows for 7.9 at 128 pixels and T = 8, where single tiles staged 3 rows for 1.
+// accumulators: 9 rows for 5.9 at 128 pixels and T = 6, where single tiles staged 3 rows for 1.
 //
 // One CTA per SM. Warp 8 loads stages (all channels of a block, or G 16-channel chunks at a time); warps
 // 9 and 10 issue the MMAs of the even and odd accumulators of a block (one thread issues an MMA every
@@ -659,7 +652,7 @@ __global__ void __launch_bounds__(kFlatThreads, 1) conv3x3_flat_kernel(const __g
       for (int32_t b = blockIdx.x; b < fg.nblock && ok; b += gridDim.x) {
         int32_t img, x0, t0;
         flat_block(fg, b, img, x0, t0);
-        const int32_t y = t0 * 128 / fg.prow - 1;
+        const int32_t y = (int32_t)((uint32_t)t0 * 128u / (uint32_t)fg.prow) - 1;
         for (int32_t sidx = 0; sidx < nsp && ok; ++sidx, ++k) {
           const int32_t buf = k % nst;
           if (k >= nst) ok = ws_wait(&empty[buf], ((k / nst) + 1) & 1, abort_v, 64);
@@ -701,7 +694,7 @@ __global__ void __launch_bounds__(kFlatThreads, 1) conv3x3_flat_kernel(const __g
       int32_t img, x0, t0;
       flat_block(fg, b, img, x0, t0);
       const int32_t nt = min(fg.T, fg.tiles - t0);
-      const int32_t off = t0 * 128 - t0 * 128 / fg.prow * fg.prow;
+      const int32_t off = (int32_t)((uint32_t)t0 * 128u % (uint32_t)fg.prow);
       const int32_t half = i & 1;
       if (i >= 2) ok = wait(&acc_empty[half], ((i >> 1) + 1) & 1);
       for (int32_t sidx = 0; sidx < nsp && ok; ++sidx, ++k) {
@@ -770,8 +763,8 @@ __global__ void __launch_bounds__(kFlatThreads, 1) conv3x3_flat_kernel(const __g
       }
       umma::fence_after_sync();
       for (int32_t t = parity; t < nt; t += 2) {
-        const int32_t f = (t0 + t) * 128 + m;
-        const int32_t row = fg.row_magic ? (int32_t)__umulhi((uint32_t)f, fg.row_magic) : f / fg.prow, col = f - row * fg.prow;
+        const uint32_t f = (uint32_t)(t0 + t) * 128u + (uint32_t)m;
+        const int32_t row = (int32_t)(fg.row_magic ? __umulhi(f, fg.row_magic) : f / (uint32_t)fg.prow), col = (int32_t)(f - (uint32_t)row * (uint32_t)fg.prow);
         const bool inside = col < fg.pitch && row < p.height;
         const int64_t pix = ((int64_t)img * p.height + row) * p.width + x0 + col;
         const uint32_t acc = tmem + (uint32_t)((half * fg.T + t) * cout) + ((uint32_t)((warp & 3) * 32) << 16);
@@ -839,19 +832,22 @@ bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) ==
 
 namespace {
 
-// shared memory of one CTA of the pipelined kernel: two CTAs per SM
+// shared memory of one CTA of conv3x3_ws_kernel: two CTAs per SM
 #ifndef MJPBR_CONV_SMEM_BUDGET
 #define MJPBR_CONV_SMEM_BUDGET (110 * 1024)
 #endif
 constexpr size_t kPipeSmemBudget = MJPBR_CONV_SMEM_BUDGET;
 // One CTA per SM with most of the shared memory: measured faster for the layers of 16-pixel rows and
 // the 64-pixel-row layers of 96 or more input channels (their staged pipeline then holds bigger
-// stages), slower for every other layer shape of the denoiser.
+// stages), slower for every other layer shape of the denoiser when its skips were at half resolution.
 constexpr size_t kPipeSmemWide = 200 * 1024;
 
 size_t pipe_budget(int32_t width, int32_t cin) {
   return (width <= 16 || (width == 64 && cin >= 96)) ? kPipeSmemWide : kPipeSmemBudget;
 }
+// Layers of rows of 128 pixels sum row by row of taps where their weights fit this beside four staged rows,
+// all others chunk by chunk. The rule has no other use: it keeps the layers' sums in the order they have had.
+constexpr size_t kRowOrderSmem = 110 * 1024;
 constexpr size_t kPipeSmemMax = 220 * 1024;
 int conv_sm_count() { return device_sm_count(); }
 
@@ -911,16 +907,6 @@ int make_weight_map(CUtensorMap* m, const void* base, int32_t cin, int32_t cout,
   return encode(m, base, 4, dims, strides, box);
 }
 
-// MJPBR_CONV_RING=0 sums every layer chunk by chunk (kept for comparison).
-bool conv_ring_enabled() {
-  static int enabled = -1;
-  if (enabled < 0) {
-    const char* v = getenv("MJPBR_CONV_RING");
-    enabled = (v && v[0] == '0') ? 0 : 1;
-  }
-  return enabled == 1;
-}
-
 // MJPBR_CONV_PIPELINE=0 selects the one-tile-per-CTA kernel (kept for comparison).
 bool conv_pipeline_enabled() {
   static int enabled = -1;
@@ -933,8 +919,8 @@ bool conv_pipeline_enabled() {
 
 }  // namespace
 
-// Plans and launches conv3x3_flat_kernel; kFlatUnsuitable when no plan fits. by_row: the accumulation
-// order (the row-ring layers').
+// Plans and launches conv3x3_flat_kernel; kFlatUnsuitable when no plan fits, which no shape that passes
+// conv3x3_launch's checks has given (the plain kernel would take it). by_row: the order of the sum.
 constexpr int kFlatUnsuitable = -1001;
 
 static int flat_launch(const MjpbrConv& c, const ConvGeom& g, bool by_row, cudaStream_t stream) {
@@ -942,9 +928,10 @@ static int flat_launch(const MjpbrConv& c, const ConvGeom& g, bool by_row, cudaS
   fg.pitch = g.pitch;
   fg.prow = g.pitch + 2;
   fg.strips = c.width / g.pitch;
-  if ((int64_t)c.height * fg.prow > INT32_MAX - 1024) return kFlatUnsuitable;
-  fg.tiles = (c.height * fg.prow + 127) / 128;
-  fg.row_magic = c.height * fg.prow < (1 << 24) ? (uint32_t)((((uint64_t)1 << 32) + fg.prow - 1) / fg.prow) : 0u;
+  // positions of a strip: 32 bits without a sign (at most 18 / 16 of its 2^31 pixels)
+  const int64_t positions = (int64_t)c.height * fg.prow;
+  fg.tiles = (int32_t)((positions + 127) / 128);
+  fg.row_magic = positions < (1 << 24) ? (uint32_t)((((uint64_t)1 << 32) + fg.prow - 1) / fg.prow) : 0u;
   fg.by_row = by_row;
   fg.wide = ((reinterpret_cast<uintptr_t>(c.out) | reinterpret_cast<uintptr_t>(c.out_f32)) & 31u) == 0;
   const int32_t nchunk = g.cin / 16, nci = c.c_in / 16, cout = c.c_out;
@@ -1035,8 +1022,18 @@ int conv3x3_launch(const MjpbrConv& c, cudaStream_t stream) {
   g.cin = c.c_in + c.c_in2;
   const int64_t tiles = (int64_t)c.nimg * g.tiles_per_img;
   if (tiles > INT32_MAX) return set_error(MJPBR_ERR_ARG, "conv3x3: too many tiles");
-  if (conv_pipeline_enabled() && (int64_t)c.nimg * c.height * c.width <= INT32_MAX) {
-    // warp-specialised persistent variant (32-bit pixel indices)
+  const bool half_in2 = c.c_in2 > 0 && !c.in2_full;
+  const bool pipelined = conv_pipeline_enabled() && (int64_t)c.nimg * c.height * c.width <= INT32_MAX;  // 32-bit pixel indices
+  const int32_t nchunk = g.cin / 16, nci = c.c_in / 16;
+  const size_t wbytes = (size_t)9 * 2 * nchunk * c.c_out * 16;
+  auto round128 = [](size_t v) { return (v + 127) / 128 * 128; };
+  if (pipelined && !half_in2) {
+    const size_t rowplane = (size_t)(g.pitch + 2) * 16;
+    const size_t slot = round128(round128(2 * nci * rowplane) + 2 * (nchunk - nci) * rowplane);
+    const bool by_row = g.rows == 1 && kRowOrderSmem > wbytes && (kRowOrderSmem - wbytes) / slot >= 4;
+    const int rc = flat_launch(c, g, by_row, stream);
+    if (rc != kFlatUnsuitable) return rc;
+  } else if (pipelined) {
     WsGeom wg;
     wg.g = g;
     wg.ntiles = (int32_t)tiles;
@@ -1049,14 +1046,9 @@ int conv3x3_launch(const MjpbrConv& c, cudaStream_t stream) {
     int acc_cols = 32;
     while (acc_cols < c.c_out) acc_cols <<= 1;
     wg.acc_cols = acc_cols;
-    const int32_t nchunk = g.cin / 16, nci = c.c_in / 16;
     const int32_t copies = wg.single ? 1 : 3;
-    auto round128 = [](size_t v) { return (v + 127) / 128 * 128; };
-    const bool half_in2 = c.c_in2 > 0 && !c.in2_full;
-    const size_t wbytes = (size_t)9 * 2 * nchunk * c.c_out * 16;
     auto stage_bytes = [&](int32_t G, bool resident) {
-      size_t b = round128((size_t)copies * 2 * G * wg.plane);
-      if (half_in2) b += round128((size_t)2 * G * wg.s2plane);
+      size_t b = round128((size_t)copies * 2 * G * wg.plane) + round128((size_t)2 * G * wg.s2plane);
       if (!resident) b += (size_t)9 * 2 * G * c.c_out * 16;
       return b;
     };
@@ -1073,17 +1065,8 @@ int conv3x3_launch(const MjpbrConv& c, cudaStream_t stream) {
     wg.group = G;
     wg.nstage = nst;
     wg.resident = resident;
-    // Layers whose weights and four input rows fit this budget sum row by row of taps, the others chunk by
-    // chunk (results do not depend on which kernel takes a layer).
-    if (!half_in2) {
-      const size_t rowplane = (size_t)(g.pitch + 2) * 16;
-      const size_t slot = round128(round128(2 * nci * rowplane) + 2 * (nchunk - nci) * rowplane);
-      const bool by_row = conv_ring_enabled() && wg.single && budget > wbytes && (budget - wbytes) / slot >= 4;
-      const int rc = flat_launch(c, g, by_row, stream);
-      if (rc != kFlatUnsuitable) return rc;
-    }
     wg.abuf = (int32_t)round128((size_t)copies * 2 * G * wg.plane);
-    wg.s2buf = half_in2 ? (int32_t)round128((size_t)2 * G * wg.s2plane) : 0;
+    wg.s2buf = (int32_t)round128((size_t)2 * G * wg.s2plane);
     wg.bstage = resident ? 0 : 9 * 2 * G * c.c_out * 16;
     wg.s2_off = nst * wg.abuf;
     wg.b_off = wg.s2_off + nst * wg.s2buf;
@@ -1091,10 +1074,8 @@ int conv3x3_launch(const MjpbrConv& c, cudaStream_t stream) {
     if (smem > kPipeSmemMax) return set_error(MJPBR_ERR_ARG, "conv3x3: %zu bytes of shared memory needed", smem);
     if (int rc = ensure_smem(reinterpret_cast<const void*>(conv3x3_ws_kernel), kPipeSmemMax, "conv3x3")) return rc;
     CUtensorMap tm_in, tm_in2, tm_w;
-    memset(&tm_in2, 0, sizeof(tm_in2));
     if (make_act_map(&tm_in, c.in, c.c_in, c.width, c.height, c.nimg, wg.spitch, g.rows + 2, 2 * G) != 0) return MJPBR_ERR_CUDA;
-    if (half_in2 && make_act_map(&tm_in2, c.in2, c.c_in2, c.width / 2, c.height / 2, c.nimg, wg.s2w, wg.s2h, 2 * G) != 0) return MJPBR_ERR_CUDA;
-    if (c.c_in2 > 0 && c.in2_full && make_act_map(&tm_in2, c.in2, c.c_in2, c.width, c.height, c.nimg, wg.spitch, g.rows + 2, 2 * G) != 0) return MJPBR_ERR_CUDA;
+    if (make_act_map(&tm_in2, c.in2, c.c_in2, c.width / 2, c.height / 2, c.nimg, wg.s2w, wg.s2h, 2 * G) != 0) return MJPBR_ERR_CUDA;
     if (make_weight_map(&tm_w, c.weight, g.cin, c.c_out, wg.resident ? 2 * nchunk : 2 * G) != 0) return MJPBR_ERR_CUDA;
     // resident CTAs per SM, limited by shared memory (1 KB of it reserved per CTA), registers
     // and the 512 tensor-memory columns (two accumulators per CTA)
