@@ -376,10 +376,6 @@ __global__ void __launch_bounds__(kThreads) ptw_geometry_kernel(const __grid_con
 #ifndef MJPBR_PTW_REFILL_STEPS
 #define MJPBR_PTW_REFILL_STEPS 32
 #endif
-// Idle lanes before a warp of the scanned stages with meshes fetches again.
-#ifndef MJPBR_SCAN_MIN_IDLE
-#define MJPBR_SCAN_MIN_IDLE 8
-#endif
 
 // Closest hits of `items` rays: start(item, &max_dist) gives a ray (and sets the lane's world block
 // blk), finish(hit) stores its hit. kTogether: where lanes stride over the items, a CTA's warps start each
@@ -405,14 +401,14 @@ MJ_DEV void closest_queue(const MjpbrScene& s, const Stack& st, const BlockLayou
       if (qq.tie) qq.h = trace_ray<true>(s, st, blk, L, qq.m.r, max_dist, cull, false, err);
       finish(qq.h);
     };
-    refill_loop<MJPBR_PTW_REFILL_STEPS, MJPBR_SCAN_MIN_IDLE>(
+    refill_loop<MJPBR_PTW_REFILL_STEPS, kFetchIdle>(
         items, fetched, q,
         [&](int64_t item, ClosestWalk& qq) {
           qq.m.r = start(item, &max_dist);
           qq.m.meshes = scan_closest<true>(qq.h, qq.tie, NodeBoxes{blk, &L}, blk, L, qq.m.r, max_dist, cull);
           qq.m.slot = -1;
           qq.m.sp = 0;
-        qq.m.code = -1;
+          qq.m.code = -1;
           if (qq.m.meshes) return true;
           done(qq);
           return false;
@@ -577,8 +573,8 @@ __global__ void __launch_bounds__(kThreads, kTex ? MJPBR_PTW_TEX_CTAS : MJPBR_PT
       if (features) store_path_features(wm, path, ps);
     }
     // The CTA's warps take each phase together: the stage's code is several times the instruction cache (on
-    // 1024 x 128x128 and, with environments, 128 x 2 x 256x256 paths: 8.7 and 14.5 ms, and 11.8 and 26.4
-    // with no barrier at all, paths appended by warps).
+    // 1024 x 128x128 and, with environments, 128 x 2 x 256x256 paths: 8.7 -> 6.5 and 14.5 -> 10.1 ms with the
+    // queues by hit and miss; 11.8 and 26.4 with no barrier at all, paths appended by warps).
     RecordedNee nee{path, v3(0.0f), &wm, &err};
     __syncthreads();
     if (status == Core::kShade) Core::lights(c, nee, ps, x, pseed, head_dir);
@@ -635,12 +631,12 @@ __global__ void __launch_bounds__(kThreads, kScan ? kScanCtas : 3) ptw_shadow_ke
   } else if constexpr (kScan) {
     const Stack st = wave_stack(s, smem);
     MeshWalk q;
-    refill_loop<MJPBR_PTW_REFILL_STEPS, MJPBR_SCAN_MIN_IDLE>(
+    refill_loop<MJPBR_PTW_REFILL_STEPS, kFetchIdle>(
         items, fetched, q,
         [&](int64_t item, MeshWalk& qq) {
           qq.r = start(item, &qq.cut);
           qq.sp = 0;
-        qq.code = -1;
+          qq.code = -1;
           const bool hit = scan_any<true>(blk, L, qq.r, qq.cut, cull, &qq.meshes);
           if (!hit && qq.meshes) return true;
           if (!hit) visible();

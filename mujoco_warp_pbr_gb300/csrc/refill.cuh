@@ -13,6 +13,11 @@ namespace mjpbr {
 
 constexpr int32_t kAnyAbort = 3;                       // a query stopped by the step bound
 constexpr int32_t kMaxRaySteps = 1 << 20;              // steps of one ray: far above any traversal of a scene
+// Idle lanes before a warp of the scanned stages fetches again, whose fetches trace all primitives of a ray. ms at 1,
+// 4, 8 and 16: shadow rays of 1024 mesh worlds (128 x 128, 2 x 2 samples) 6.30, 6.73, 6.53, 6.31, of 300 terrain
+// worlds 1.38, 1.31, 1.28, 1.26; path-traced frames of 12 and 32 geoms, a third meshes, 6.75, 6.97, 6.80, 6.66 and
+// 5.53, 5.66, 5.54, 5.47. For voted_loop's see there.
+constexpr int32_t kFetchIdle = 16;
 constexpr uint64_t kRefillTimeLimitNs = 4000000000ull; // three orders of magnitude above the largest chunk's stage
 
 MJ_DEV uint64_t global_ns() {

@@ -419,12 +419,6 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_SHADE_CTAS) wave_surface_
 #ifndef MJPBR_WAVE_REFILL_STEPS
 #define MJPBR_WAVE_REFILL_STEPS 32
 #endif
-// Idle lanes before a warp of the scanned stages fetches again.
-// Idle lanes before a warp of the mirror rays' mesh stage fetches again (voted_loop).
-constexpr int32_t kVoteIdle = 16;
-#ifndef MJPBR_SCAN_MIN_IDLE
-#define MJPBR_SCAN_MIN_IDLE 8
-#endif
 
 // Result of mirror entry i: a miss is final (the resolve stage reads nothing else of it); a hit is listed
 // for the surface stage at list position pos (< 0: by one atomic per group of converged lanes), so that
@@ -529,7 +523,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_MIRROR_CTAS) wave_mirror_
   ClosestWalk q;
   const float* blk = nullptr;
   int32_t sample = -1, entry = -1;
-  voted_loop<kVoteIdle>(
+  voted_loop<kFetchIdle>(
       items, reinterpret_cast<unsigned long long*>(wm.counters + 4), q,
       [&](int64_t item, ClosestWalk& qq) {
         entry = wm.mirror[item].index.y;
@@ -668,7 +662,7 @@ __global__ void __launch_bounds__(kThreads, kScanCtas) wave_shadow_scan_kernel(c
   MeshWalk q;
   const float* blk = nullptr;
   int32_t target = -1;
-  refill_loop<MJPBR_WAVE_REFILL_STEPS, MJPBR_SCAN_MIN_IDLE>(
+  refill_loop<MJPBR_WAVE_REFILL_STEPS, kFetchIdle>(
       items, reinterpret_cast<unsigned long long*>(wm.counters + 2), q,
       [&](int64_t item, MeshWalk& qq) {
         const int32_t ei = (int32_t)(item / ns), k = (int32_t)(item - (int64_t)ei * ns);
