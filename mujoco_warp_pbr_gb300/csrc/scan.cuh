@@ -12,14 +12,15 @@
 //
 // What bounds these queries is instruction issue: the per-lane traversal runs 16 (camera rays), 13
 // (shadow) and 7 (mirror) of 32 lanes; the scan 27-30 without meshes. Camera rays of 1024 mesh worlds
-// (128 x 128, 2 x 2 samples) 11.0 -> 7.8 ms, 300 terrain worlds (96 x 96) 3.96 -> 2.92 ms a frame.
+// (128 x 128, 2 x 2 samples) 13.2 -> 8.95 ms, of 300 terrain worlds (96 x 96) 1.34 -> 0.79, the walk's with
+// the primitives' earlier tests.
 //
 // kScanGeoms = 32: one mask word, and the scan is the faster of the two up to there (256 worlds of
-// 128 x 128, ms a frame, scan / BVH): primitives 0.63 / 1.53 at 4 geoms, 1.13 / 1.72 at 17, 1.47 /
-// 2.08 at 32; with a third of them meshes 1.85 / 1.84, 3.02 / 3.71 and 4.17 / 5.19; path-traced 7.48 /
-// 9.37 and with meshes 23.4 / 25.9 at 32. The leaf boxes are read from the scene BVH's nodes (each child
-// of a node with count 1 is a leaf; hidden geoms have none), whose bounds the leaf's ancestors
-// contain, so the boxes that pass are those the traversal reaches.
+// 128 x 128, ms a frame, scan / BVH): primitives 0.71 / 1.62 at 4 geoms, 1.10 / 1.90 at 17, 1.38 / 2.12 at 32;
+// with a third of them meshes 2.11 / 2.50, 3.56 / 4.48 and 4.60 / 5.54; path-traced 2.96 / 3.77, 4.83 /
+// 5.97 and 6.08 / 6.90, with meshes 7.02 / 8.05, 14.4 / 16.3 and 17.7 / 18.8. The leaf boxes are read from the scene
+// BVH's nodes (each child of a node with count 1 is a leaf; hidden geoms have none), whose bounds the leaf's
+// ancestors contain, so the boxes that pass are those the traversal reaches.
 #pragma once
 
 #include "trace.cuh"
