@@ -249,6 +249,29 @@ MJ_DEV void write_geometry(const MjpbrScene& s, int32_t w, const Pixel& p, const
   }
 }
 
+// Column and row of pixel q of a 16 x 16 tile in Z order.
+MJ_DEV int32_t z_x(int32_t q) { return (q & 1) | ((q >> 1) & 2) | ((q >> 2) & 4) | ((q >> 3) & 8); }
+MJ_DEV int32_t z_y(int32_t q) { return ((q >> 1) & 1) | ((q >> 2) & 2) | ((q >> 3) & 4) | ((q >> 4) & 8); }
+
+// A pixel's guides and its resolved image (display RGB, HDR radiance) at its address in the output rows.
+MJ_DEV void write_guides(const MjpbrScene& s, int64_t adr, V3 albedo, V3 normal) {
+  if (!s.settings.render_guides || !s.guide_albedo) return;
+  s.guide_albedo[adr * 3] = albedo.x;
+  s.guide_albedo[adr * 3 + 1] = albedo.y;
+  s.guide_albedo[adr * 3 + 2] = albedo.z;
+  s.guide_normal[adr * 3] = normal.x;
+  s.guide_normal[adr * 3 + 1] = normal.y;
+  s.guide_normal[adr * 3 + 2] = normal.z;
+}
+MJ_DEV void write_image(const MjpbrScene& s, int64_t adr, V3 display, V3 hdr) {
+  if (s.settings.render_hdr && s.hdr_data) {
+    s.hdr_data[adr * 3] = hdr.x;
+    s.hdr_data[adr * 3 + 1] = hdr.y;
+    s.hdr_data[adr * 3 + 2] = hdr.z;
+  }
+  s.rgb_data[adr] = encode_display(display);
+}
+
 // Copies world w's block (written by mjpbr_refit_bvh) into shared memory; the caller synchronises.
 MJ_DEV void stage_world_block(const MjpbrScene& s, int32_t w, float* blk, int32_t nthreads) {
   const float4* src = reinterpret_cast<const float4*>(s.world_blocks + (int64_t)w * s.world_block_floats);

@@ -46,9 +46,6 @@ struct FusedMap {
   int32_t cta_base[MJPBR_MAX_RENDER + 1];
 };
 
-MJ_DEV int32_t z_x(int32_t q) { return (q & 1) | ((q >> 1) & 2) | ((q >> 2) & 4) | ((q >> 3) & 8); }
-MJ_DEV int32_t z_y(int32_t q) { return ((q >> 1) & 1) | ((q >> 2) & 2) | ((q >> 3) & 4) | ((q >> 4) & 8); }
-
 // A surface parked in shared memory: word k of a thread at base[k * kThreads] (conflict-free).
 constexpr int32_t kSurfaceWords = 14;
 template <int kThreads>
@@ -240,26 +237,11 @@ __global__ void __launch_bounds__(kThreads, kThreads == kWide ? 2 : 3) rt_fused_
   }
   if (active) {
     if (rgb) {
-      if (smp == 0 && st.render_guides && s.guide_albedo) {
-        const int64_t a = ((int64_t)w * s.rgb_stride + s.rgb_adr[cam] + p.pixelid) * 3;
-        s.guide_albedo[a] = albedo.x;
-        s.guide_albedo[a + 1] = albedo.y;
-        s.guide_albedo[a + 2] = albedo.z;
-        s.guide_normal[a] = gnormal.x;
-        s.guide_normal[a + 1] = gnormal.y;
-        s.guide_normal[a + 2] = gnormal.z;
-      }
-      V3 display = display_transform(radiance * c.exposure, st.tone_mapper);
       const int64_t adr = (int64_t)w * s.rgb_stride + s.rgb_adr[cam] + p.pixelid;
+      if (smp == 0) write_guides(s, adr, albedo, gnormal);
+      const V3 display = display_transform(radiance * c.exposure, st.tone_mapper);
       if (nn == 1) {
-        // 0 + x as the sums below
-        if (st.render_hdr && s.hdr_data) {
-          const V3 hdr = v3(0.0f) + radiance;
-          s.hdr_data[adr * 3] = hdr.x;
-          s.hdr_data[adr * 3 + 1] = hdr.y;
-          s.hdr_data[adr * 3 + 2] = hdr.z;
-        }
-        s.rgb_data[adr] = encode_display(v3(0.0f) + display);
+        write_image(s, adr, v3(0.0f) + display, v3(0.0f) + radiance);  // 0 + x as the sums below
       } else {
         float* v = sums + threadIdx.x;
         v[0] = display.x, v[kThreads] = display.y, v[2 * kThreads] = display.z;
@@ -279,12 +261,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == kWide ? 2 : 3) rt_fused_
   }
   const int64_t adr = (int64_t)w * s.rgb_stride + s.rgb_adr[cam] + p.pixelid;
   const float inv_nn = inv_n * inv_n;
-  if (st.render_hdr && s.hdr_data) {
-    s.hdr_data[adr * 3] = hdr.x * inv_nn;
-    s.hdr_data[adr * 3 + 1] = hdr.y * inv_nn;
-    s.hdr_data[adr * 3 + 2] = hdr.z * inv_nn;
-  }
-  s.rgb_data[adr] = encode_display(display * inv_nn);
+  write_image(s, adr, display * inv_nn, hdr * inv_nn);
 }
 
 size_t fused_smem(const MjpbrScene& s, int32_t threads) {

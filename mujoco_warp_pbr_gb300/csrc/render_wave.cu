@@ -118,9 +118,6 @@ struct WaveMap {
   int64_t mirror_cap, shadow_cap;
 };
 
-MJ_DEV int32_t z_x(int32_t q) { return (q & 1) | ((q >> 1) & 2) | ((q >> 2) & 4) | ((q >> 3) & 8); }
-MJ_DEV int32_t z_y(int32_t q) { return ((q >> 1) & 1) | ((q >> 2) & 2) | ((q >> 3) & 4) | ((q >> 4) & 8); }
-
 MJ_DEV Stack wave_stack(const MjpbrScene& s, float* base) {
   return shared_stack(base, kThreads, stack_entries(s.settings.stack_depth));
 }
@@ -777,15 +774,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_SHADE_CTAS) wave_resolve_
         }
       }
     }
-    if (smp == 0 && st.render_guides && s.guide_albedo) {
-      const int64_t a = ((int64_t)w * s.rgb_stride + s.rgb_adr[cam] + p.pixelid) * 3;
-      s.guide_albedo[a] = albedo.x;
-      s.guide_albedo[a + 1] = albedo.y;
-      s.guide_albedo[a + 2] = albedo.z;
-      s.guide_normal[a] = gnormal.x;
-      s.guide_normal[a + 1] = gnormal.y;
-      s.guide_normal[a + 2] = gnormal.z;
-    }
+    if (smp == 0) write_guides(s, (int64_t)w * s.rgb_stride + s.rgb_adr[cam] + p.pixelid, albedo, gnormal);
     const V3 display = display_transform(radiance * c.exposure, st.tone_mapper);
     float* slot_sum = sums + threadIdx.x * 6;
     slot_sum[0] = display.x, slot_sum[1] = display.y, slot_sum[2] = display.z;
@@ -801,12 +790,7 @@ __global__ void __launch_bounds__(kThreads, MJPBR_WAVE_SHADE_CTAS) wave_resolve_
   }
   const int64_t adr = (int64_t)w * s.rgb_stride + s.rgb_adr[cam] + p.pixelid;
   const float inv_nn = inv_n * inv_n;
-  if (st.render_hdr && s.hdr_data) {
-    s.hdr_data[adr * 3] = hdr.x * inv_nn;
-    s.hdr_data[adr * 3 + 1] = hdr.y * inv_nn;
-    s.hdr_data[adr * 3 + 2] = hdr.z * inv_nn;
-  }
-  s.rgb_data[adr] = encode_display(display * inv_nn);
+  write_image(s, adr, display * inv_nn, hdr * inv_nn);
 }
 
 // ---------------------------------------------------------------- host side
