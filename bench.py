@@ -15,7 +15,8 @@ environment rotation). A step is refit_bvh + render of one frame of every world.
              has landed.
   roofline   the frame's algorithmic HBM bytes (outputs written once, world blocks and tables
              read once) over its event-timed duration, against the measured copy bandwidth, with
-             the DRAM traffic of the frame's stage kernels from an ncu launch list; the render is
+             the DRAM traffic of the frame's kernels from an ncu launch list (null where these
+             kernels were not measured); the render is
              bound by traversal latency and divergence, not HBM, so this fraction is small by
              construction.
   stages_ms  the wavefront's stage split from CUDA events the library records at every stage
@@ -460,7 +461,7 @@ def run(args) -> None:
 
   # a frame of tens of microseconds (the primitive configuration) is timed as a CUDA graph replay of
   # refit + render (seed fixed), as the reference's benchmark captures its steps in a graph: launched
-  # one by one, its eight launches would be timed at the host's submission rate
+  # one by one, its launches would be timed at the host's submission rate
   graph = None
   if args.workload == "primitives":
     scene_g = mjpbr.scene_descriptor(m, d, rc)

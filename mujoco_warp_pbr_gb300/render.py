@@ -363,8 +363,8 @@ def refit_bvh(m: Any, d: Any, rc: PbrRenderContext) -> None:
 
 
 def render(m: Any, d: Any, rc: PbrRenderContext, seed: int = 0, denoise: bool = True) -> None:
-  """Renders the current frame into the context's output buffers (one kernel for the real-time
-  tier, one persistent kernel for the path-traced tier). The image is a deterministic function of
+  """Renders the current frame into the context's output buffers (by the context's schedule: a
+  wavefront's stages or its fused kernel, or a megakernel). The image is a deterministic function of
   the seed. The per-world blocks come from the last refit_bvh; the first render of a context
   refits once itself. A path-traced context created with denoise=True then runs the a-trous
   filter (the reference's _src/render.py:431-460 dispatch and _src/pathtrace.py:426-438);
