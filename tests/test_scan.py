@@ -147,3 +147,39 @@ def test_far_cameras_match_the_bvh(distance, mesh):
     assert (ref["seg"][..., 0] > 0).mean() > 0.1
     for key in ("rgb", "depth", "seg", "hdr"):
       np.testing.assert_array_equal(got[key], ref[key], err_msg=key)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("mesh", [False, True])
+def test_large_coordinates_match_the_bvh(mesh):
+  """The scene kilometres from the origin, where a coordinate's rounding is as large as the boxes' padding is
+  elsewhere."""
+  sc = scene(17, mesh=mesh, mirror=True, nworld=4)
+  for field in ("geom_xpos", "cam_xpos", "light_xpos"):
+    getattr(sc.mjd, field)[...] += np.array([3000.0, -2000.0, 500.0], np.float32)
+  for options, schedule in (({}, "queue"), ({"tier": 1, "path_samples": 2, "max_depth": 2}, "grid")):
+    ref = images(sc, schedule=schedule, **options)
+    got = images(sc, schedule="wavefront", **options)
+    assert (ref["seg"][..., 0] > 0).mean() > 0.1
+    for key in ("rgb", "depth", "seg", "hdr"):
+      np.testing.assert_array_equal(got[key], ref[key], err_msg=key)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("name", ["hfield", "translucent", "translucent_mesh"])
+def test_path_scan_of_height_fields_and_translucent_geoms(name):
+  if name == "hfield":
+    sc = synthetic.hfield_scene(seed=2, nworld=3, res=36)
+    sc.options.pop("shadow_samples")
+  else:
+    sc = scene(17, mesh=name.endswith("mesh"), nworld=3)
+    sc.per_world["geom_rgba"][:, 2::4, 3] = 0.5
+  got = []
+  for schedule in ("grid", "wavefront"):
+    m, d, rc = helpers.gpu_scene(sc, schedule=schedule, tier=1, path_samples=2, max_depth=3, render_hdr=True)
+    rc.has_transparency = name != "hfield"
+    got.append(helpers.render_gpu(m, d, rc, seed=11))
+  for key in ("rgb", "depth", "seg", "hdr"):
+    np.testing.assert_array_equal(got[1][key], got[0][key], err_msg=key)
